@@ -252,9 +252,20 @@ tr_status tr_profile_nufft(tr_plan* plan, int32_t bin, int32_t reps, double* ms,
  *   forward:     y (N, D, H, W, Cout) f32 = conv(x, w) + bias (bias may be NULL)
  *   weight grad: dw (Cout, 27, Cin) f32 = sum_v gy[v, co] x[v + tap, ci]
  *                (deterministic; needs tr_conv3d_wgrad_workspace bytes of scratch)
- * The data gradient is tr_conv3d_fwd with the flipped, channel-swapped weights. */
+ * The data gradient is the forward convolution with the flipped, channel-swapped weights.
+ * tr_conv3d_pack brings weights (Cout, 27, Cin), bf16 or float (w_f32, rounded to bf16), into the
+ * layout the kernel streams (tr_conv3d_packed_size bytes); with data_grad it reads the layer's own
+ * weights (Cin, 27, Cout) and packs the data gradient's.  tr_conv3d_fwd_packed is the forward
+ * convolution with packed weights; float activations (x_f32) are rounded to bf16 as they are read.
+ * tr_conv3d_fwd packs its weights into stream-ordered scratch on each call.
+ * A kernel whose bounded device wait runs out writes NaN to its outputs. */
 tr_status tr_conv3d_fwd(const void* x, const void* w, const float* bias, float* y, int32_t N, int32_t D,
                         int32_t H, int32_t W, int32_t Cin, int32_t Cout, void* stream);
+tr_status tr_conv3d_packed_size(int32_t Cin, int32_t Cout, size_t* bytes);
+tr_status tr_conv3d_pack(const void* w, int32_t w_f32, int32_t data_grad, void* packed, int32_t Cin, int32_t Cout,
+                         void* stream);
+tr_status tr_conv3d_fwd_packed(const void* x, int32_t x_f32, const void* packed, const float* bias, float* y, int32_t N,
+                               int32_t D, int32_t H, int32_t W, int32_t Cin, int32_t Cout, void* stream);
 tr_status tr_conv3d_wgrad_workspace(int32_t N, int32_t D, int32_t H, int32_t W, int32_t Cin, int32_t Cout,
                                     size_t* bytes);
 tr_status tr_conv3d_wgrad(const void* x, const void* gy, float* dw, int32_t N, int32_t D, int32_t H, int32_t W,

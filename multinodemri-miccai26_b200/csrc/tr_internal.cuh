@@ -1,6 +1,8 @@
 // Internal definitions shared by the toporecon_b200 CUDA sources.
 #pragma once
 
+#include <cuda.h>
+#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -236,6 +238,9 @@ struct tr_plan {
 };
 
 namespace tr {
+
+// cuTensorMapEncodeTiled from the driver, looked up once (no libcuda link); null if it is missing.
+PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder();
 
 tr_status ensure_nufft_buffers(tr_plan* p, size_t ncol);
 tr_status nufft_forward_cols(tr_plan* p, int bin, const float2* images, int64_t img_stride, int n_img,

@@ -1800,8 +1800,7 @@ tr_status ensure_nufft_buffers(tr_plan* p, size_t ncol) {
     return TR_OK;
 }
 
-// cuTensorMapEncodeTiled from the driver, looked up once (no libcuda link).
-static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
+PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
     static std::once_flag once;
     std::call_once(once, [] {

@@ -42,16 +42,34 @@ def _stream(t):
     return ctypes.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
 
 
+def pack_weights(w, cin, cout, data_grad=False):
+    """Weights w, bf16 or float32, contiguous, in the layout the forward kernel streams, as bf16:
+    (cout, 27, cin), or with ``data_grad`` the layer's own (cin, 27, cout) flipped and swapped."""
+    import torch
+    L = _lib.load()
+    nbytes = ctypes.c_size_t(0)
+    _lib.check(L.tr_conv3d_packed_size(cin, cout, ctypes.byref(nbytes)))
+    packed = torch.empty(nbytes.value // 2, dtype=torch.bfloat16, device=w.device)
+    _lib.check(L.tr_conv3d_pack(_ptr(w), int(w.dtype == torch.float32), int(data_grad), _ptr(packed), cin, cout,
+                                _stream(packed)), "tr_conv3d_pack")
+    return packed
+
+
+def conv3d_fwd_packed(x, packed, cout, bias=None):
+    """x (N, D, H, W, Cin), bf16 or float32 (rounded to bf16 as the kernel reads it), packed weights
+    -> (N, D, H, W, cout) f32."""
+    import torch
+    N, D, H, W, Cin = x.shape
+    y = torch.empty((N, D, H, W, cout), dtype=torch.float32, device=x.device)
+    b = _ptr(bias) if bias is not None else None
+    _lib.check(_lib.load().tr_conv3d_fwd_packed(_ptr(x), int(x.dtype == torch.float32), _ptr(packed), b, _ptr(y), N, D, H,
+                                                W, Cin, cout, _stream(y)), "tr_conv3d_fwd")
+    return y
+
+
 def conv3d_fwd_bf16(x_bf, w_bf, bias=None):
     """x (N, D, H, W, Cin) bf16, w (Cout, 27, Cin) bf16 -> (N, D, H, W, Cout) f32."""
-    import torch
-    N, D, H, W, Cin = x_bf.shape
-    Cout = w_bf.shape[0]
-    y = torch.empty((N, D, H, W, Cout), dtype=torch.float32, device=x_bf.device)
-    b = _ptr(bias) if bias is not None else None
-    _lib.check(_lib.load().tr_conv3d_fwd(_ptr(x_bf), _ptr(w_bf), b, _ptr(y), N, D, H, W, Cin, Cout, _stream(y)),
-               "tr_conv3d_fwd")
-    return y
+    return conv3d_fwd_packed(x_bf, pack_weights(w_bf, x_bf.shape[-1], w_bf.shape[0]), w_bf.shape[0], bias)
 
 
 def conv3d_wgrad_bf16(x_bf, gy_bf):
@@ -69,21 +87,15 @@ def conv3d_wgrad_bf16(x_bf, gy_bf):
     return dw
 
 
-def _flip_swap(w):
-    """w (Cout, 27, Cin) -> w' (Cin, 27, Cout) with taps reversed (the data-gradient weights)."""
-    return w.flip(1).permute(2, 1, 0).contiguous()
-
-
 def conv3d_dgrad_bf16(gy_bf, w_bf):
     """Gradient w.r.t. the input: the forward kernel on the flipped, channel-swapped
     weights, with their output channels padded to a multiple of 8."""
-    import torch
-    wt = _flip_swap(w_bf)
-    cin = wt.shape[0]
+    cin, cout = w_bf.shape[2], w_bf.shape[0]
     pad = (-cin) % 8
     if pad:
-        wt = torch.cat([wt, wt.new_zeros((pad,) + tuple(wt.shape[1:]))], dim=0)
-    gx = conv3d_fwd_bf16(gy_bf, wt)
+        import torch
+        w_bf = torch.cat([w_bf, w_bf.new_zeros((cout, 27, pad))], dim=2)
+    gx = conv3d_fwd_packed(gy_bf, pack_weights(w_bf, cout, cin + pad, data_grad=True), cin + pad)
     return gx[..., :cin].contiguous() if pad else gx
 
 
@@ -92,7 +104,11 @@ def _make_conv_fn():
 
     class Conv3dBF16(torch.autograd.Function):
         @staticmethod
-        def forward(ctx, x, w, b):
+        def forward(ctx, x, w, b, grad):
+            if not (grad and any(ctx.needs_input_grad)) and x.dtype == w.dtype == torch.float32:
+                # no backward will read bf16 copies of x and w
+                return conv3d_fwd_packed(x.contiguous(), pack_weights(w.contiguous(), x.shape[-1], w.shape[0]),
+                                         w.shape[0], b)
             xb = x.contiguous().to(torch.bfloat16)
             wb = w.contiguous().to(torch.bfloat16)
             ctx.save_for_backward(xb, wb)
@@ -105,7 +121,7 @@ def _make_conv_fn():
             gx = conv3d_dgrad_bf16(gb, wb) if ctx.needs_input_grad[0] else None
             gw = conv3d_wgrad_bf16(xb, gb) if ctx.needs_input_grad[1] else None
             gbias = gy.sum(dim=(0, 1, 2, 3)) if ctx.needs_input_grad[2] else None
-            return gx, gw, gbias
+            return gx, gw, gbias, None
 
     return Conv3dBF16
 
@@ -117,7 +133,8 @@ def conv3d(x, w, b):
     global _CONV
     if _CONV is None:
         _CONV = _make_conv_fn()
-    return _CONV.apply(x, w, b)
+    import torch
+    return _CONV.apply(x, w, b, torch.is_grad_enabled())
 
 
 # ---------------------------------------------------------------------- network

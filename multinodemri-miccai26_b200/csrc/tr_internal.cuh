@@ -210,10 +210,6 @@ struct tr_plan {
     float2* bufA = nullptr;      // >= OSZ*OSY*OSX*ncol (grid / x-pass output)
     float2* bufB = nullptr;      // >= Z*OSY*OSX*ncol  (y-pass output / z-pass adjoint output)
     size_t buf_cols = 0;         // ncol the buffers are sized for
-    // single-image drop-in scratch
-    float2* one_in = nullptr;
-    float2* one_out = nullptr;
-    size_t one_elems = 0;
     // reductions
     double* partials = nullptr;
     int npartials = 0;
@@ -245,9 +241,10 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder();
 tr_status ensure_nufft_buffers(tr_plan* p, size_t ncol);
 tr_status nufft_forward_cols(tr_plan* p, int bin, const float2* images, int64_t img_stride, int n_img,
                              const float2* maps, int C, int mode, float sigma, const float2* y,
-                             float2* out, cudaStream_t st);
+                             float2* out, cudaStream_t st, const int32_t* perm = nullptr);
 tr_status nufft_adjoint_cols(tr_plan* p, int bin, const float2* ksp, int n_img, const float2* maps, int C,
-                             bool use_dcf, float2* images, int64_t img_stride, cudaStream_t st);
+                             bool use_dcf, float2* images, int64_t img_stride, cudaStream_t st,
+                             const int32_t* perm = nullptr);
 tr_status wavelet_prepare(tr_plan* p);
 tr_status wavelet_dual(tr_plan* p, const float2* u_bar, float2* p_w2, float sigma, float lam, cudaStream_t st);
 tr_status wavelet_adjoint(tr_plan* p, const float2* p_w2, float2* out, cudaStream_t st);

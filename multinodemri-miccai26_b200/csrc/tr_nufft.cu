@@ -31,6 +31,7 @@
 #include <numeric>
 #include <string>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "tr_fft.cuh"
@@ -1321,6 +1322,10 @@ __global__ void __launch_bounds__(kWideNT, 5) k_adj_x_wide(AdjXArgs a, const __g
 }
 
 // ------------------------------------------------------------------ per-sample tap records
+// Column counts of the few-column interpolation and gridding kernels: k_interp and k_spread spread
+// 16 or more columns over their lanes.
+constexpr int kFewCols = 8;
+
 // First tap per axis and the 15 KB weights of every (sorted) sample, computed
 // once at plan creation; interpolation and gridding read them instead of
 // re-evaluating the window.  w[0..4] z taps, w[5..9] y taps, w[10..14] x taps.
@@ -1425,6 +1430,126 @@ __global__ void __launch_bounds__(256) k_interp(const float2* __restrict__ grid,
         const int col = lane + j * G;
         if (col >= ncol) continue;
         const int64_t o = s * ncol + col;
+        if (mode == kInterpDualProx) {
+            const float2 r = csub(acc[j], y[o]);
+            const float2 q = out[o];
+            const float inv = 1.0f / (1.0f + sigma);
+            out[o] = make_float2((q.x + sigma * r.x) * inv, (q.y + sigma * r.y) * inv);
+        } else {
+            out[o] = acc[j];
+        }
+    }
+}
+
+// Few columns (1 to 8): sixteen lanes per sample.  Consecutive lanes take the columns of an x tap
+// (two per 16-byte load; PG lanes at 4 and 8 columns, else one lane takes them all), then the four x
+// taps, then (z, y) tap rows, so that a warp reads whole tap rows; the lanes are summed by shuffles
+// (a step halves the columns that a lane carries while they are even).  With one lane per (sample,
+// column) a small call has too few loads in flight (5,760 samples, one column: 13.0 us, 5.3 us
+// here; 34,000 samples, four columns: 18.2 us, 13.2 us here).  perm (null: none): sample s goes to
+// row perm[s] of out.
+template <int NC>
+__global__ void __launch_bounds__(256) k_interp_rows(const float2* __restrict__ grid, const TapRec* __restrict__ taps,
+                                                     int64_t M, int os0, int os1, int os2, int mode, float sigma,
+                                                     const int32_t* __restrict__ perm, const float2* __restrict__ y,
+                                                     float2* __restrict__ out) {
+    constexpr int PG = NC == 4 ? 2 : (NC == 8 ? 4 : 1), CPL = NC / PG;     // lanes per x tap, columns per lane
+    constexpr int RP = 16 / (4 * PG);                                      // tap rows side by side
+    const int64_t s = ((int64_t)blockIdx.x * 256 + threadIdx.x) >> 4;
+    if (((int64_t)blockIdx.x * 256 + (threadIdx.x & ~31)) >> 4 >= M) return;     // whole warps leave
+    const int l = threadIdx.x & 15, c0 = (l % PG) * CPL, tx = (l / PG) & 3, rr = l / (4 * PG);
+    const TapRec rec = taps[s < M ? s : M - 1];
+    const float wz[5] = {rec.w[0].x, rec.w[0].y, rec.w[0].z, rec.w[0].w, rec.w[1].x};
+    const float wy[5] = {rec.w[1].y, rec.w[1].z, rec.w[1].w, rec.w[2].x, rec.w[2].y};
+    const float wx = tx == 0 ? rec.w[2].z : (tx == 1 ? rec.w[2].w : (tx == 2 ? rec.w[3].x : rec.w[3].y));
+    const int64_t ox = (int64_t)pmod(rec.b.z + tx, os2) * NC + c0;
+    float2 acc[CPL];
+#pragma unroll
+    for (int j = 0; j < CPL; ++j) acc[j] = make_float2(0.f, 0.f);
+    auto add = [&](float w, const float2* g) {
+        if constexpr (CPL % 2 == 0) {
+#pragma unroll
+            for (int j = 0; j < CPL; j += 2) {
+                const float4 v = *reinterpret_cast<const float4*>(g + j);
+                acc[j] = cfma_real(w, make_float2(v.x, v.y), acc[j]);
+                acc[j + 1] = cfma_real(w, make_float2(v.z, v.w), acc[j + 1]);
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < CPL; ++j) acc[j] = cfma_real(w, g[j], acc[j]);
+        }
+    };
+    if (wz[4] == 0.f && wy[4] == 0.f && rec.w[3].z == 0.f) {
+        // common case: four taps per axis
+        int oy[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) oy[t] = pmod(rec.b.y + t, os1);
+#pragma unroll
+        for (int tz = 0; tz < 4; ++tz) {
+            const int64_t oz = (int64_t)pmod(rec.b.x + tz, os0) * os1;
+#pragma unroll
+            for (int t = 0; t < 4 / RP; ++t) {                 // RP <= 4 rows (ty) side by side
+                float wyt = wy[t * RP];
+                int o = oy[t * RP];
+#pragma unroll
+                for (int k = 1; k < RP; ++k) {
+                    wyt = rr == k ? wy[t * RP + k] : wyt;
+                    o = rr == k ? oy[t * RP + k] : o;
+                }
+                add(wz[tz] * wyt * wx, grid + (oz + o) * os2 * NC + ox);
+            }
+        }
+    } else {
+        const int64_t ox4 = (int64_t)pmod(rec.b.z + 4, os2) * NC + c0;
+        for (int r = rr; r < 25; r += RP) {
+            const int tz = r / 5, ty = r - tz * 5;
+            float wzt = 0.f, wyt = 0.f;                        // register arrays: no dynamic index
+#pragma unroll
+            for (int t = 0; t < 5; ++t) {
+                wzt = tz == t ? wz[t] : wzt;
+                wyt = ty == t ? wy[t] : wyt;
+            }
+            const float wzy = wzt * wyt;
+            if (wzy == 0.f) continue;
+            const float2* g = grid + ((int64_t)pmod(rec.b.x + tz, os0) * os1 + pmod(rec.b.y + ty, os1)) * os2 * NC;
+            if (wx != 0.f) add(wzy * wx, g + ox);
+            if (tx == 0 && rec.w[3].z != 0.f) add(wzy * rec.w[3].z, g + ox4);
+        }
+    }
+    __syncwarp();      // the two samples of a warp may have taken different branches
+    // sum over the lanes of a column: a lane bit picks the half of the columns that a lane keeps
+    int col = c0;
+    auto fold = [&](auto nc, int off) {
+        constexpr int n = decltype(nc)::value;
+        const bool up = (threadIdx.x & off) != 0;
+        if constexpr (n % 2 == 0) {
+#pragma unroll
+            for (int j = 0; j < n / 2; ++j) {
+                const float2 give = up ? acc[j] : acc[j + n / 2], keep = up ? acc[j + n / 2] : acc[j];
+                acc[j] = cadd(keep, make_float2(__shfl_xor_sync(0xffffffffu, give.x, off),
+                                                __shfl_xor_sync(0xffffffffu, give.y, off)));
+            }
+            col += up ? n / 2 : 0;
+        } else {
+#pragma unroll
+            for (int j = 0; j < n; ++j)
+                acc[j] = cadd(acc[j], make_float2(__shfl_xor_sync(0xffffffffu, acc[j].x, off),
+                                                  __shfl_xor_sync(0xffffffffu, acc[j].y, off)));
+        }
+    };
+    constexpr auto half = [](int n) { return n % 2 ? n : n / 2; };
+    constexpr int n1 = half(CPL), n2 = half(n1), n3 = PG > 2 ? n2 : half(n2), n4 = PG > 1 ? n3 : half(n3);
+    fold(std::integral_constant<int, CPL>(), 8);
+    fold(std::integral_constant<int, n1>(), 4);
+    if constexpr (PG <= 2) fold(std::integral_constant<int, n2>(), 2);
+    if constexpr (PG <= 1) fold(std::integral_constant<int, n3>(), 1);
+    // lanes that differ only in bits of butterfly steps hold the same sums: the lowest writes
+    constexpr int same = (CPL % 2 ? 8 : 0) | (n1 % 2 ? 4 : 0) | (PG <= 2 && n2 % 2 ? 2 : 0) | (PG <= 1 && n3 % 2 ? 1 : 0);
+    if (s >= M || (threadIdx.x & same)) return;
+    const int64_t so = perm ? perm[s] : s;
+#pragma unroll
+    for (int j = 0; j < n4; ++j) {
+        const int64_t o = so * NC + col + j;
         if (mode == kInterpDualProx) {
             const float2 r = csub(acc[j], y[o]);
             const float2 q = out[o];
@@ -1702,6 +1827,125 @@ __global__ void __launch_bounds__(256, (CG >= 6 ? 3 : (CG >= 4 ? 4 : 5))) k_spre
                 for (int c = lane; c < ncc; c += 32) dst[c] = src[c];
             }
         }
+    }
+}
+
+// Few columns (1 to 8): one warp per work item, two x points of a (z, y) tile row and every column
+// per lane.  k_spread gives a tile 16 column groups of threads, so that one column leaves 15 of 16
+// threads idle (102,000 samples, one column, 105 x 147 x 125 grid: 281 us, 36 us here; 34,000
+// samples, four columns, 60 x 80 x 80 grid: 61 us, 27 us here).  Entries are staged 32 at a time
+// per warp (a lane loads an entry's taps, weights of the 16 rows and 4 columns of the tile), and every
+// point sums its list in order.  perm (null: none): the values of sample m are row perm[m] of vals.
+constexpr int kFewWarps = 8;
+constexpr int kFewZero = 8;              // empty tiles per zero-fill warp
+__host__ __device__ constexpr int few_entry_floats(int nc) { return 20 + 2 * nc + (nc & 1) * 2; }
+template <int NC>
+__global__ void __launch_bounds__(32 * kFewWarps) k_spread_few(SpreadArgs a, const int32_t* __restrict__ perm) {
+    constexpr int kEF = few_entry_floats(NC);            // per entry: 16 row weights, 4 x weights, the values
+    __shared__ __align__(16) float sh[kFewWarps][32 * kEF];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float* e = sh[warp];
+    const long long bb = (long long)blockIdx.x * kFewWarps + warp;
+    const long long nzc = (a.n_empty + kFewZero - 1) / kFewZero, T = a.n_work + nzc;
+    if (bb >= T) return;
+    // zero-fill groups spread evenly among the work items, as in k_spread
+    const long long zlo = bb * nzc / T, zhi = (bb + 1) * nzc / T;
+    int t0z, t0y, t0x, Tz, Ty, Tx;
+    const int row = lane >> 1, xh = (lane & 1) * 2, pz = row >> 2, py = row & 3;
+    auto point = [&](int x) {
+        return a.grid + (((int64_t)(t0z + pz) * a.os1 + (t0y + py)) * a.os2 + t0x + x) * NC;
+    };
+    if (zhi > zlo) {
+        const int z1 = min((int)zhi * kFewZero, a.n_empty);
+        for (int zi = (int)zlo * kFewZero; zi < z1; ++zi) {
+            tile_geometry(a, a.tile_order[a.n_busy + zi], t0z, t0y, t0x, Tz, Ty, Tx);
+            if (pz >= Tz || py >= Ty) continue;
+            for (int x = xh; x < min(xh + 2, Tx); ++x)
+#pragma unroll
+                for (int j = 0; j < NC; ++j) point(x)[j] = make_float2(0.f, 0.f);
+        }
+        return;
+    }
+    const int4 item = a.work[bb - zlo];
+    tile_geometry(a, item.x, t0z, t0y, t0x, Tz, Ty, Tx);
+    float2 acc[2][NC];
+#pragma unroll
+    for (int j = 0; j < NC; ++j) acc[0][j] = acc[1][j] = make_float2(0.f, 0.f);
+    // the list entry is read two batches ahead, the taps and values one batch ahead
+    int2 en = make_int2(0, 0), next = make_int2(0, 0);
+    float4 t0, t1, t2, t3;
+    float2 val[NC];
+    float d = 1.0f;
+    auto fetch_entry = [&](int i) { return i + lane < item.z ? a.list[i + lane] : make_int2(-1, 0); };
+    auto fetch = [&](int2 ent) {
+        if (ent.x < 0) return;
+        const float4* tw = a.taps[ent.x].w;
+        t0 = tw[0], t1 = tw[1], t2 = tw[2], t3 = tw[3];
+        const float2* src = a.vals + (int64_t)(perm ? perm[ent.x] : ent.x) * NC;
+#pragma unroll
+        for (int j = 0; j < NC; ++j) val[j] = src[j];
+        d = a.use_dcf ? a.ks[ent.x].w : 1.0f;
+    };
+    next = fetch_entry(item.y);
+    fetch(next);
+    for (int base = item.y; base < item.z; base += 32) {
+        const int ns = min(32, item.z - base);
+        en = next;
+        next = fetch_entry(base + 32);
+        __syncwarp();
+        if (lane < ns) {
+            const float w[15] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w, t2.x, t2.y, t2.z, t2.w, t3.x, t3.y, t3.z};
+            const int az = (en.y & 0xff) - 128, ay = ((en.y >> 8) & 0xff) - 128, ax = ((en.y >> 16) & 0xff) - 128;
+            float* my = e + lane * kEF;
+            // weight of tap offset o + k (0 outside the five taps), by selects: registers have no dynamic index
+            auto pick = [&](int first, int o, int k) {
+                float v = 0.f;
+#pragma unroll
+                for (int t = 0; t < 5; ++t) v = o + k == t ? w[first + t] : v;
+                return v;
+            };
+            float fy[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) fy[k] = pick(5, ay, k);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float fz = pick(0, az, k);
+                // (wz wy) dcf, the order of k_spread
+                *reinterpret_cast<float4*>(my + 4 * k) = make_float4((fz * fy[0]) * d, (fz * fy[1]) * d, (fz * fy[2]) * d,
+                                                                    (fz * fy[3]) * d);
+            }
+            *reinterpret_cast<float4*>(my + 16) = make_float4(pick(10, ax, 0), pick(10, ax, 1), pick(10, ax, 2), pick(10, ax, 3));
+#pragma unroll
+            for (int j = 0; j < NC; ++j) *reinterpret_cast<float2*>(my + 20 + 2 * j) = val[j];
+        }
+        __syncwarp();
+        fetch(next);
+#pragma unroll 4
+        for (int k = 0; k < ns; ++k) {
+            const float* en = e + k * kEF;
+            const float wzy = en[row];
+            const float2 wx = *reinterpret_cast<const float2*>(en + 16 + xh);
+            // a point outside the support takes nothing from the value, be it infinite
+            const bool in0 = wzy != 0.f && wx.x != 0.f, in1 = wzy != 0.f && wx.y != 0.f;
+            const float w0 = wzy * wx.x, w1 = wzy * wx.y;
+#pragma unroll
+            for (int j = 0; j < NC; ++j) {
+                const float2 v = *reinterpret_cast<const float2*>(en + 20 + 2 * j);
+                if (in0) acc[0][j] = cfma_real(w0, v, acc[0][j]);
+                if (in1) acc[1][j] = cfma_real(w1, v, acc[1][j]);
+            }
+        }
+    }
+    for (int x = 0; x < 2; ++x) {
+        float2* dst;
+        if (item.w >= 0) {
+            dst = a.partials + ((int64_t)item.w * 64 + row * 4 + xh + x) * NC;
+        } else {
+            if (pz >= Tz || py >= Ty || xh + x >= Tx) continue;
+            dst = point(xh + x);
+        }
+#pragma unroll
+        for (int j = 0; j < NC; ++j) dst[j] = x ? acc[1][j] : acc[0][j];
     }
 }
 
@@ -2158,10 +2402,28 @@ static tr_status stage_fwd_z(tr_plan* p, int bin, int ncol, cudaStream_t st) {
                        p->ax[0].pad, 0, false, st, bin_colmask(p, bin, ncol), ncol);
 }
 
+// perm (single-column calls only): sample s goes to out[perm[s]]
 static tr_status stage_interp(tr_plan* p, int bin, int ncol, int mode, float sigma, const float2* y, float2* out,
-                              cudaStream_t st) {
+                              cudaStream_t st, const int32_t* perm = nullptr) {
     const Bin& b = p->bins[bin];
     if (b.count == 0) return TR_OK;
+    if (ncol <= kFewCols) {
+        const TapRec* taps = reinterpret_cast<const TapRec*>(p->taps) + b.offset;
+        const unsigned blocks = (unsigned)((b.count * 16 + 255) / 256);
+#define TR_INTERP_ROWS(NCV)                                                                                       \
+    case NCV:                                                                                                     \
+        k_interp_rows<NCV><<<blocks, 256, 0, st>>>(p->bufA, taps, b.count, p->os[0], p->os[1], p->os[2], mode, sigma, \
+                                                   perm, y, out);                                                 \
+        break;
+        switch (ncol) {
+            TR_INTERP_ROWS(1) TR_INTERP_ROWS(2) TR_INTERP_ROWS(3) TR_INTERP_ROWS(4)
+            TR_INTERP_ROWS(5) TR_INTERP_ROWS(6) TR_INTERP_ROWS(7) TR_INTERP_ROWS(8)
+            default: break;
+        }
+#undef TR_INTERP_ROWS
+        TR_CHECK_LAUNCH();
+        return TR_OK;
+    }
     int G = 1;
     while (G < ncol && G < 32) G <<= 1;
     const int cpl = (ncol + G - 1) / G;
@@ -2196,7 +2458,9 @@ static tr_status launch_spread_t(const SpreadArgs& sa, const CUtensorMap& tgrid,
 }
 
 // gridding: one CTA per (busy 4x4x4 tile, chunk of <= 128 columns), then the zero-fill CTAs
-static tr_status stage_spread(tr_plan* p, int bin, const float2* ksp, int ncol, bool use_dcf, cudaStream_t st) {
+// perm (single-column calls only): the value of sample m is ksp[perm[m]]
+static tr_status stage_spread(tr_plan* p, int bin, const float2* ksp, int ncol, bool use_dcf, cudaStream_t st,
+                              const int32_t* perm = nullptr) {
     const Bin& b = p->bins[bin];
     SpreadArgs sa;
     sa.ks = p->ks + b.offset;
@@ -2224,6 +2488,24 @@ static tr_status stage_spread(tr_plan* p, int bin, const float2* ksp, int ncol, 
     sa.nt2 = p->ntile[2];
     sa.err = p->dev_err;
     sa.poll = p->poll_limit;
+    if (ncol <= kFewCols) {
+        const long long items = sa.n_work + (sa.n_empty + kFewZero - 1) / kFewZero;
+        const unsigned blocks = (unsigned)((items + kFewWarps - 1) / kFewWarps);
+#define TR_SPREAD_FEW(NCV) \
+    case NCV: k_spread_few<NCV><<<blocks, 32 * kFewWarps, 0, st>>>(sa, perm); break;
+        switch (ncol) {
+            TR_SPREAD_FEW(1) TR_SPREAD_FEW(2) TR_SPREAD_FEW(3) TR_SPREAD_FEW(4)
+            TR_SPREAD_FEW(5) TR_SPREAD_FEW(6) TR_SPREAD_FEW(7) TR_SPREAD_FEW(8)
+            default: break;
+        }
+#undef TR_SPREAD_FEW
+        TR_CHECK_LAUNCH();
+        if (b.n_split > 0) {
+            k_spread_reduce<<<(unsigned)b.n_split, 256, 0, st>>>(sa, p->splits + b.split_offset);
+            TR_CHECK_LAUNCH();
+        }
+        return TR_OK;
+    }
     const int cg = (sa.cchunk + 15) / 16;
     // TMA path: even column counts and chunks, 16-byte aligned k-space rows, an encodable grid map
     CUtensorMap tgrid;
@@ -2369,7 +2651,7 @@ static tr_status stage_adj_x(tr_plan* p, int n_img, const float2* maps, int C, f
 
 tr_status nufft_forward_cols(tr_plan* p, int bin, const float2* images, int64_t img_stride, int n_img,
                              const float2* maps, int C, int mode, float sigma, const float2* y, float2* out,
-                             cudaStream_t st) {
+                             cudaStream_t st, const int32_t* perm) {
     const int ncol = n_img * C;
     TR_TRY(ensure_nufft_buffers(p, (size_t)ncol));
     TR_TRY(stage_fwd_x(p, images, img_stride, n_img, maps, C, st));
@@ -2379,7 +2661,7 @@ tr_status nufft_forward_cols(tr_plan* p, int bin, const float2* images, int64_t 
         TR_TRY(stage_fwd_y(p, ncol, st));
         TR_TRY(stage_fwd_z(p, bin, ncol, st));
     }
-    return stage_interp(p, bin, ncol, mode, sigma, y, out, st);
+    return stage_interp(p, bin, ncol, mode, sigma, y, out, st, perm);
 }
 
 // Launch-shape autotuning (TR_PLAN_AUTOTUNE).  The first gridding of a column
@@ -2439,11 +2721,11 @@ static tr_status tune_spread_cols(tr_plan* p, int bin, const float2* ksp, int nc
 }
 
 tr_status nufft_adjoint_cols(tr_plan* p, int bin, const float2* ksp, int n_img, const float2* maps, int C,
-                             bool use_dcf, float2* images, int64_t img_stride, cudaStream_t st) {
+                             bool use_dcf, float2* images, int64_t img_stride, cudaStream_t st, const int32_t* perm) {
     const int ncol = n_img * C;
     TR_TRY(ensure_nufft_buffers(p, (size_t)ncol));
     TR_TRY(tune_spread_cols(p, bin, ksp, ncol, use_dcf, st));
-    TR_TRY(stage_spread(p, bin, ksp, ncol, use_dcf, st));
+    TR_TRY(stage_spread(p, bin, ksp, ncol, use_dcf, st, perm));
     bool fused = false;
     TR_TRY(stage_yz(p, ncol, true, st, &fused));
     if (!fused) {
@@ -2564,8 +2846,6 @@ static void plan_free(tr_plan* p) {
     cudaFree(p->maps);
     cudaFree(p->bufA);
     cudaFree(p->bufB);
-    cudaFree(p->one_in);
-    cudaFree(p->one_out);
     cudaFree(p->partials);
     cudaFree(p->tol_dev);
     cudaFree(p->dev_err);
@@ -3010,40 +3290,23 @@ tr_status tr_plan_unsort_kspace(tr_plan* p, int32_t bin, const void* internal, v
     return TR_OK;
 }
 
-static tr_status ensure_one(tr_plan* p) {
-    size_t need = (size_t)std::max<int64_t>(1, 0);
-    for (auto& b : p->bins) need = std::max(need, (size_t)b.count);
-    if (p->one_in && p->one_elems >= need) return TR_OK;
-    cudaFree(p->one_in);
-    cudaFree(p->one_out);
-    p->one_in = p->one_out = nullptr;
-    TR_CUDA(cudaMalloc(&p->one_in, need * sizeof(float2)));
-    TR_CUDA(cudaMalloc(&p->one_out, need * sizeof(float2)));
-    p->one_elems = need;
-    return TR_OK;
-}
-
+// One image: the interpolation writes, and the gridding reads, the samples in acquisition order.
 tr_status tr_nufft_forward(tr_plan* p, int32_t bin, const void* image, void* ksp, void* stream) {
     TR_TRY(tr_plan_bin_offset(p, bin, nullptr, nullptr));
     if (!image || !ksp) return fail(TR_ERR_INVALID_ARG, "tr_nufft_forward: null pointer");
     DeviceGuard g(p->device);
-    TR_TRY(ensure_one(p));
-    cudaStream_t st = (cudaStream_t)stream;
     const int64_t N = (int64_t)p->n[0] * p->n[1] * p->n[2];
-    TR_TRY(nufft_forward_cols(p, bin, (const float2*)image, N, 1, nullptr, 1, kInterpStore, 0.f, nullptr,
-                              p->one_out, st));
-    return tr_plan_unsort_kspace(p, bin, p->one_out, ksp, 1, stream);
+    return nufft_forward_cols(p, bin, (const float2*)image, N, 1, nullptr, 1, kInterpStore, 0.f, nullptr, (float2*)ksp,
+                              (cudaStream_t)stream, p->perm + p->bins[bin].offset);
 }
 
 tr_status tr_nufft_adjoint(tr_plan* p, int32_t bin, const void* ksp, void* image, void* stream) {
     TR_TRY(tr_plan_bin_offset(p, bin, nullptr, nullptr));
     if (!image || !ksp) return fail(TR_ERR_INVALID_ARG, "tr_nufft_adjoint: null pointer");
     DeviceGuard g(p->device);
-    TR_TRY(ensure_one(p));
-    cudaStream_t st = (cudaStream_t)stream;
-    TR_TRY(tr_plan_sort_kspace(p, bin, ksp, p->one_in, 1, stream));
     const int64_t N = (int64_t)p->n[0] * p->n[1] * p->n[2];
-    return nufft_adjoint_cols(p, bin, p->one_in, 1, nullptr, 1, false, (float2*)image, N, st);
+    return nufft_adjoint_cols(p, bin, (const float2*)ksp, 1, nullptr, 1, false, (float2*)image, N, (cudaStream_t)stream,
+                              p->perm + p->bins[bin].offset);
 }
 
 tr_status tr_nufft_forward_bin(tr_plan* p, int32_t bin, const void* images, void* ksp_internal, void* stream) {

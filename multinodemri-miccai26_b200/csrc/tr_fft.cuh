@@ -366,6 +366,46 @@ struct Dft<10> : DftPfa<2, 5, 1, 3> {};
 template <>
 struct Dft<20> : DftPfa<4, 5, 1, 4> {};
 
+// 9 = 3 x 3 (Cooley-Tukey, as 16): n = 3 n1 + n2, k = k1 + 3 k2, twiddles W9^(n2 k1).
+template <>
+struct Dft<9> {
+    __host__ __device__ __forceinline__ static void run(float2 (&v)[9], bool inv) {
+        float2 a[3][3];
+#pragma unroll
+        for (int n2 = 0; n2 < 3; ++n2) {
+            float2 t[3] = {v[n2], v[3 + n2], v[6 + n2]};
+            Dft<3>::run(t, inv);
+#pragma unroll
+            for (int k1 = 0; k1 < 3; ++k1) a[n2][k1] = t[k1];
+        }
+        // cos / sin of 2 pi m / 9, m = 1, 2, 4
+        a[1][1] = crot(a[1][1], 0.76604444311897804f, 0.64278760968653933f, inv);
+        a[1][2] = crot(a[1][2], 0.17364817766693035f, 0.98480775301220806f, inv);
+        a[2][1] = crot(a[2][1], 0.17364817766693035f, 0.98480775301220806f, inv);
+        a[2][2] = crot(a[2][2], -0.93969262078590838f, 0.34202014332566873f, inv);
+#pragma unroll
+        for (int k1 = 0; k1 < 3; ++k1) {
+            float2 t[3] = {a[0][k1], a[1][k1], a[2][k1]};
+            Dft<3>::run(t, inv);
+#pragma unroll
+            for (int k2 = 0; k2 < 3; ++k2) v[k1 + 3 * k2] = t[k2];
+        }
+    }
+};
+// Further coprime products <N1, N2, N2^-1 mod N1, N1^-1 mod N2>.
+template <>
+struct Dft<6> : DftPfa<2, 3, 1, 2> {};
+template <>
+struct Dft<12> : DftPfa<4, 3, 3, 1> {};
+template <>
+struct Dft<14> : DftPfa<2, 7, 1, 4> {};
+template <>
+struct Dft<15> : DftPfa<3, 5, 2, 2> {};
+template <>
+struct Dft<18> : DftPfa<2, 9, 1, 5> {};
+template <>
+struct Dft<21> : DftPfa<3, 7, 1, 5> {};
+
 // One Stockham stage over every butterfly of every column.
 template <int R, class Src, class Dst>
 __device__ __forceinline__ void fft_stage(const float2* __restrict__ tw, int L, int Ns, int W, bool inv,
@@ -441,9 +481,12 @@ __host__ __device__ constexpr int ct_nstages(int L) {
 // (320 = 20 x 16, 160 = 10 x 16): each pass moves every element through
 // shared memory once each way, and the transforms that are bound by the
 // shared-memory data pipe lose a third of that traffic; other lengths keep P = 0.
+// P = 2: the split that the line pass of tr_lines_part.cuh takes at 120, for the fused y + z kernels
+// (the same bits as the separate passes).
 __host__ __device__ constexpr int ct_radix_p(int P, int L, int s) {
     if (P == 1 && L == 320) return s == 0 ? 20 : (s == 1 ? 16 : 0);
     if (P == 1 && L == 160) return s == 0 ? 10 : (s == 1 ? 16 : 0);
+    if (P == 2 && L == 120) return s == 0 ? 12 : (s == 1 ? 10 : 0);
     return ct_radix(L, s);
 }
 __host__ __device__ constexpr int ct_nstages_p(int P, int L) {

@@ -10,7 +10,7 @@
 //
 // Data layout (device):
 //   images           (n_img, Z, Y, X)                  complex64
-//   coil maps        (Z, Y, X, C)                      complex64, plan-owned copy
+//   coil maps        (Z, Y, X, C)                      complex64, plan-owned copy times apodisation and scale
 //   x-pass buffer    (Z, Y, OSX, ncol)                 ncol = n_img * C columns
 //   y-pass buffer    (Z, OSY, OSX, ncol)
 //   grid             (OSZ, OSY, OSX, ncol)
@@ -35,6 +35,7 @@
 #include <vector>
 
 #include "tr_fft.cuh"
+#include "tr_lines.cuh"
 #include "tr_internal.cuh"
 
 namespace tr {
@@ -97,26 +98,6 @@ __device__ __forceinline__ int axis_taps(float k, float beta, float (&w)[5]) {
 // One CTA: `rows` consecutive (z, y) image rows x `cc` coils of one image.
 // Fuses: image * coil map * separable apodisation * scale, centred zero-pad,
 // x FFT, centred shift; output into the (Z, Y, OSX, ncol) buffer.
-struct FwdXArgs {
-    const float2* img;      // (n_img, Z, Y, X)
-    int64_t img_stride;
-    const float2* maps;     // (Z, Y, X, C) or null
-    int C;                  // coils per image (1 when maps == null)
-    int n_img;
-    int Z, Y, X, OSX, h, pad;
-    int rows, cc;           // rows per CTA, coils per CTA
-    const float* apz;
-    const float* apy;
-    const float* apx;
-    float scale;
-    const float2* tw;
-    FftStages S;
-    float2* out;            // (Z, Y, OSX, ncol)
-    int ncol;
-    int* err;               // device error word (kDevErr* bits)
-    int poll;               // polls before a bounded mbarrier wait gives up
-};
-
 __global__ void __launch_bounds__(256) k_fwd_x(FwdXArgs a) {
     extern __shared__ float2 sm[];
     const int W = a.rows * a.cc;
@@ -145,7 +126,7 @@ __global__ void __launch_bounds__(256) k_fwd_x(FwdXArgs a) {
             const int z = row / a.Y, y = row - z * a.Y;
             v = src[(int64_t)row * a.X + x];
             if (a.maps) v = cmul(v, a.maps[((int64_t)row * a.X + x) * a.C + c]);
-            v = cscale(v, a.apz[z] * a.apy[y] * a.apx[x] * a.scale);
+            else v = cscale(v, a.apz[z] * a.apy[y] * a.apx[x] * a.scale);
         }
         smA[idx] = v;
     }
@@ -167,51 +148,6 @@ __global__ void __launch_bounds__(256) k_fwd_x(FwdXArgs a) {
 // Data viewed as [outer][rows][inner]; transforms along rows for W consecutive
 // inner elements per CTA.  Input rows present: Lin (pad offset p_in inside the
 // length-L line); output rows kept: Lout (crop offset p_out).
-struct LineArgs {
-    const float2* in;
-    float2* out;
-    int64_t inner;
-    int Lin, Lout, p_in, p_out, h;
-    int W;
-    int vec16;              // rows are 16-byte aligned: copy two elements per cp.async
-    bool inv;
-    const float2* tw;
-    FftStages S;
-    int* err;               // device error word (kDevErr* bits)
-    int poll;               // polls before a bounded mbarrier wait gives up
-    int kA, kB;             // TMA variant: first transform row of each output box
-    // z passes: (y, x) tile columns that no sample's kernel reaches; null: none skipped
-    const uint8_t* colmask; // [nt1 * nt2] 1: occupied
-    int skip_zero;          // 0: a CTA whose lines are all unoccupied returns (forward: the output is never
-                            // read); 1: it writes zeros to its output rows (adjoint: the lines are zero)
-    int mcol, mosx, mnt2;   // k-space columns, OSX and tile columns along x of the mask
-};
-
-// Empty-column skip of the z passes.  Inner index q of a z pass is
-// ((y OSX + x) ncol + column); a line is unoccupied when the tile column
-// (y / 4, x / 4) holds no busy tile: gridding wrote no tile there (the line is
-// all zeros) and interpolation reads no tap there.  True when every line
-// q0 .. q0 + W - 1 (< inner) of the CTA is unoccupied (the same for all threads).
-// The host passes a mask only when W divides ncol, so a CTA never mixes lines
-// of occupied and unoccupied columns (it would read unwritten tiles).
-__device__ __forceinline__ bool lines_unoccupied(const LineArgs& a, int64_t q0, int W) {
-    if (!a.colmask) return false;
-    const int64_t q1 = min(q0 + W, a.inner) - 1;
-    for (int64_t yx = q0 / a.mcol; yx <= q1 / a.mcol; ++yx) {
-        const int y = (int)(yx / a.mosx), x = (int)(yx - (int64_t)y * a.mosx);
-        if (a.colmask[(y >> 2) * a.mnt2 + (x >> 2)]) return false;
-    }
-    return true;
-}
-// The zeros of an unoccupied CTA's output rows (adjoint z pass): [Lout][W] at q0.
-__device__ __forceinline__ void lines_write_zeros(const LineArgs& a, int64_t q0, int W, int64_t outer) {
-    float2* out = a.out + outer * a.Lout * a.inner;
-    for (int i = threadIdx.x; i < a.Lout * W; i += blockDim.x) {
-        const int o = i / W, w = i - o * W;
-        if (q0 + w < a.inner) out[(int64_t)o * a.inner + q0 + w] = make_float2(0.f, 0.f);
-    }
-}
-
 // The CTA's [L][W] tile is staged with cp.async (every load in flight at
 // once, zero-filled pad rows and tail columns), then all stages run from
 // shared memory and the last stage stores straight to global memory.
@@ -281,26 +217,6 @@ __global__ void __launch_bounds__(256) k_line(LineArgs a) {
 // One CTA: `rows` rows x all C coils of one image (coils processed in chunks
 // of `cc`).  Fuses: x IFFT, centred shift and crop, apodisation, scale,
 // conj(coil map) and the coil sum; writes (or adds into) the image row.
-struct AdjXArgs {
-    const float2* in;       // (Z, Y, OSX, ncol)
-    int ncol;
-    const float2* maps;     // (Z, Y, X, C) or null
-    int C, cc, rows;
-    int n_img;
-    int Z, Y, X, OSX, h, pad;
-    const float* apz;
-    const float* apy;
-    const float* apx;
-    float scale;
-    const float2* tw;
-    FftStages S;
-    float2* img;            // (n_img, Z, Y, X)
-    int64_t img_stride;
-    int accumulate;
-    int* err;               // device error word (kDevErr* bits)
-    int poll;               // polls before a bounded mbarrier wait gives up
-};
-
 __global__ void __launch_bounds__(256) k_adj_x(AdjXArgs a) {
     extern __shared__ float2 sm[];
     const int W = a.rows * a.cc;
@@ -362,19 +278,25 @@ __global__ void __launch_bounds__(256) k_adj_x(AdjXArgs a) {
         const int row = row0 + rl;
         if (row >= nrows) continue;
         const int z = row / a.Y, y = row - z * a.Y;
-        const float s = a.apz[z] * a.apy[y] * a.apx[x] * a.scale;
-        float2 v = cscale(acc[i], s);
-        float2* dst = a.img + (int64_t)img * a.img_stride + (int64_t)row * a.X + x;
-        if (a.accumulate) v = cadd(*dst, v);
-        *dst = v;
+        const float s = a.maps ? 1.0f : a.apz[z] * a.apy[y] * a.apx[x] * a.scale;
+        a.img[(int64_t)img * a.img_stride + (int64_t)row * a.X + x] = cscale(acc[i], s);
     }
 }
 
-// ------------------------------------------------------------------ compile-time variants
-// The same three FFT kernels with L and W fixed at compile time (fft_ct):
-// used for the transform lengths of the supported workloads.
+// ------------------------------------------------------------------ TMA variants
+// FFT kernels whose tiles travel by TMA, with L and W fixed at compile time (fft_ct), where they are
+// faster than the kernels of tr_lines.cuh:
+// - line passes at L = 160, 200 and 320.  Their two-radix splits (16 x 10, 20 x 10, 20 x 16) fill the
+//   threads of the register passes unevenly or leave two CTAs per SM; in place over TMA tiles: y pass
+//   of 128 x 256 x 256, 96 columns, 2.79 against 3.65 ms, of 112 x 160 x 160, 72 columns, 0.92 against
+//   1.08 ms, z pass at 160, 96 columns, 4.00 against 4.45 ms.  At 60 to 140 and 240 the kernels of
+//   tr_lines.cuh are faster: z pass at 60, 80, 100, 120 (32 columns) 0.15, 0.18, 0.21, 0.26 against
+//   0.19, 0.22, 0.25, 0.29 ms, y pass at 100, 120, 140 0.13, 0.16, 0.19 against 0.14, 0.16, 0.20 ms,
+//   at 240 (24 columns) 0.30 against 0.42 ms.
+// - x passes with whole groups of 8 or 4 coils (below).
 // Lengths up to 200 use 16-column tiles, longer ones 8-column tiles (the
 // shared-memory footprint 2 L W x 8 bytes then allows >= 4 CTAs per SM).
+#define TR_LINE_TMA_LENGTHS(X) X(160) X(200) X(320)
 #define TR_CT_WIDE(X) X(60) X(80) X(100) X(120) X(140) X(160) X(200)
 #define TR_CT_NARROW(X) X(240) X(320)
 #define TR_CT_LENGTHS(X) TR_CT_WIDE(X) TR_CT_NARROW(X)
@@ -420,70 +342,7 @@ __host__ __device__ constexpr int line_min_ctas(int NT, int P) {
     return P == 0 ? (NT == 320 ? 5 : 6) : (NT <= 160 ? 6 : 4);
 }
 
-template <int L, int W, bool INV>
-__global__ void __launch_bounds__(256) k_line_ct(LineArgs a) {
-    extern __shared__ float2 sm[];
-    float2* smA = sm;
-    float2* smB = sm + L * W;
-    float2* tws = sm + 2 * L * W;
-    const int64_t q0 = (int64_t)blockIdx.x * W;
-    if (lines_unoccupied(a, q0, W)) {
-        if (a.skip_zero) lines_write_zeros(a, q0, W, blockIdx.y);
-        return;
-    }
-    const int64_t outer = blockIdx.y;
-    const float2* __restrict__ in = a.in + outer * a.Lin * a.inner;
-    float2* __restrict__ out = a.out + outer * a.Lout * a.inner;
-    for (int i = threadIdx.x; i < L; i += 256) tws[i] = a.tw[i];
-    if (a.vec16) {
-        constexpr int NCH = W / 2;
-#pragma unroll 4
-        for (int idx = threadIdx.x; idx < L * NCH; idx += 256) {
-            const int m = idx / NCH, ch = idx - m * NCH;
-            int j = m + a.h;
-            if (j >= L) j -= L;
-            const int i = j - a.p_in;
-            const int64_t q = q0 + 2 * ch;
-            int bytes = 0;
-            const float2* g = a.in;
-            if (i >= 0 && i < a.Lin && q < a.inner) {
-                bytes = (q + 1 < a.inner) ? 16 : 8;
-                g = in + (int64_t)i * a.inner + q;
-            }
-            cp_async16(smA + m * W + 2 * ch, g, bytes);
-        }
-    } else {
-#pragma unroll 4
-        for (int idx = threadIdx.x; idx < L * W; idx += 256) {
-            const int m = idx / W, w = idx - m * W;
-            int j = m + a.h;
-            if (j >= L) j -= L;
-            const int i = j - a.p_in;
-            const int64_t q = q0 + w;
-            int bytes = 0;
-            const float2* g = a.in;
-            if (i >= 0 && i < a.Lin && q < a.inner) {
-                bytes = 8;
-                g = in + (int64_t)i * a.inner + q;
-            }
-            cp_async8(smA + idx, g, bytes);
-        }
-    }
-    cp_async_wait_all();
-    __syncthreads();
-    const int shift = a.h - a.p_out;
-    const int Lout = a.Lout;
-    const int64_t inner = a.inner;
-    auto store = [&](int k, int w, float2 v) {
-        int o = k + shift;
-        o = o >= L ? o - L : (o < 0 ? o + L : o);
-        const int64_t q = q0 + w;
-        if (q < inner && o < Lout) out[(int64_t)o * inner + q] = v;
-    };
-    fft_ct<L, W, 256, INV>(smA, smB, tws, store);
-}
-
-// TMA variant of k_line_ct: the [L][W] tile arrives as two boxes of L/2 rows
+// Line pass: the [L][W] tile arrives as two boxes of L/2 rows
 // (the centred rotation m -> row (m + L/2) mod L - p_in splits the line in two
 // contiguous runs; rows outside [0, Lin) are zero-filled by the TMA unit), the
 // transform runs in place in that tile (fft_ct_ip), and two boxes of
@@ -648,7 +507,7 @@ __global__ void __launch_bounds__(kYzNT, 2) k_yz_fwd(YzArgs a, const __grid_cons
         }
         __syncthreads();
         auto store = [t](int k, int w, float2 v) { t[k * 8 + w] = v; };
-        fft_ct_ip<LZ, 8, NT, false>(t, twz, store);
+        fft_ct_ip_p<(LZ == 120 ? 2 : 0), LZ, 8, NT, false>(t, twz, store);
         fence_proxy_async_smem();
         __syncthreads();
         if (threadIdx.x == 0 && !bad) {
@@ -715,7 +574,7 @@ __global__ void __launch_bounds__(kYzNT, 2) k_yz_adj(YzArgs a, const __grid_cons
             break;
         }
         auto store = [t](int k, int w, float2 v) { t[k * 8 + w] = v; };
-        fft_ct_ip<LZ, 8, NT, true>(t, twz, store);
+        fft_ct_ip_p<(LZ == 120 ? 2 : 0), LZ, 8, NT, true>(t, twz, store);
         __syncthreads();
         // output row z (cropped) is transform row (z - Z/2) mod LZ; it belongs to CTA z / ZR, whose
         // y-transform row for y' = y_lo + 2 i + yl is (y' + LY/2) mod LY
@@ -752,265 +611,6 @@ __global__ void __launch_bounds__(kYzNT, 2) k_yz_adj(YzArgs a, const __grid_cons
     }
 }
 
-template <int L, int W>
-__global__ void __launch_bounds__(256) k_fwd_x_ct(FwdXArgs a) {
-    extern __shared__ float2 sm[];
-    float2* smA = sm;
-    float2* smB = sm + L * W;
-    float2* tws = sm + 2 * L * W;
-    const int img = (int)(blockIdx.x % (unsigned)a.n_img);      // images of one row block run side by side
-    const int row0 = (int)(blockIdx.x / (unsigned)a.n_img) * a.rows;
-    const int c0 = blockIdx.z * a.cc;
-    const int nrows = a.Z * a.Y;
-    const int cc = a.cc;
-    const float2* __restrict__ src = a.img + (int64_t)img * a.img_stride;
-    for (int i = threadIdx.x; i < L; i += 256) tws[i] = a.tw[i];
-#pragma unroll 4
-    for (int idx = threadIdx.x; idx < L * W; idx += 256) {
-        const int m = idx / W, w = idx - m * W;
-        const int rl = w / cc, cl = w - rl * cc;
-        const int row = row0 + rl, c = c0 + cl;
-        int j = m + a.h;
-        if (j >= L) j -= L;
-        const int x = j - a.pad;
-        float2 v = make_float2(0.f, 0.f);
-        if (x >= 0 && x < a.X && row < nrows && c < a.C) {
-            const int z = row / a.Y, y = row - z * a.Y;
-            v = src[(int64_t)row * a.X + x];
-            if (a.maps) v = cmul(v, a.maps[((int64_t)row * a.X + x) * a.C + c]);
-            v = cscale(v, a.apz[z] * a.apy[y] * a.apx[x] * a.scale);
-        }
-        smA[idx] = v;
-    }
-    __syncthreads();
-    const int h = a.h;
-    auto store = [&](int k, int w, float2 v) {
-        const int rl = w / cc, cl = w - rl * cc;
-        const int row = row0 + rl, c = c0 + cl;
-        if (row >= nrows || c >= a.C) return;
-        int g = k + h;
-        if (g >= L) g -= L;
-        a.out[((int64_t)row * a.OSX + g) * a.ncol + (int64_t)img * a.C + c] = v;
-    };
-    fft_ct<L, W, 256, false>(smA, smB, tws, store);
-}
-
-template <int L, int W>
-__global__ void __launch_bounds__(256) k_adj_x_ct(AdjXArgs a) {
-    extern __shared__ float2 sm[];
-    float2* buf0 = sm;
-    float2* buf1 = sm + L * W;
-    float2* tws = sm + 2 * L * W;
-    float2* acc = tws + L;                  // [rows][X]
-    for (int i = threadIdx.x; i < L; i += 256) tws[i] = a.tw[i];
-    for (int i = threadIdx.x; i < a.rows * a.X; i += 256) acc[i] = make_float2(0.f, 0.f);
-    const int img = (int)(blockIdx.x % (unsigned)a.n_img);      // images of one row block run side by side
-    const int row0 = (int)(blockIdx.x / (unsigned)a.n_img) * a.rows;
-    const int nrows = a.Z * a.Y;
-    const int cc = a.cc;
-    float2* ep = fft_ct_free<L>(buf0, buf1);
-    const int shift = a.h - a.pad;
-    for (int c0 = 0; c0 < a.C; c0 += cc) {
-#pragma unroll 4
-        for (int idx = threadIdx.x; idx < L * W; idx += 256) {
-            const int m = idx / W, w = idx - m * W;
-            const int rl = w / cc, cl = w - rl * cc;
-            const int row = row0 + rl, c = c0 + cl;
-            int j = m + a.h;
-            if (j >= L) j -= L;
-            int bytes = 0;
-            const float2* g = a.in;
-            if (row < nrows && c < a.C) {
-                bytes = 8;
-                g = a.in + ((int64_t)row * a.OSX + j) * a.ncol + (int64_t)img * a.C + c;
-            }
-            cp_async8(buf0 + idx, g, bytes);
-        }
-        cp_async_wait_all();
-        __syncthreads();
-        const int X = a.X;
-        auto store = [&](int k, int w, float2 v) {
-            int o = k + shift;
-            o = o >= L ? o - L : (o < 0 ? o + L : o);
-            if (o < X) ep[o * W + w] = v;
-        };
-        fft_ct<L, W, 256, true>(buf0, buf1, tws, store);
-        __syncthreads();
-        for (int i = threadIdx.x; i < a.rows * X; i += 256) {
-            const int rl = i / X, x = i - rl * X;
-            const int row = row0 + rl;
-            if (row >= nrows) continue;
-            float2 s = acc[i];
-            for (int cl = 0; cl < cc && c0 + cl < a.C; ++cl) {
-                float2 v = ep[x * W + rl * cc + cl];
-                if (a.maps) v = cmulc(v, a.maps[((int64_t)row * X + x) * a.C + c0 + cl]);
-                s = cadd(s, v);
-            }
-            acc[i] = s;
-        }
-        __syncthreads();
-    }
-    for (int i = threadIdx.x; i < a.rows * a.X; i += 256) {
-        const int rl = i / a.X, x = i - rl * a.X;
-        const int row = row0 + rl;
-        if (row >= nrows) continue;
-        const int z = row / a.Y, y = row - z * a.Y;
-        const float sc = a.apz[z] * a.apy[y] * a.apx[x] * a.scale;
-        float2 v = cscale(acc[i], sc);
-        float2* dst = a.img + (int64_t)img * a.img_stride + (int64_t)row * a.X + x;
-        if (a.accumulate) v = cadd(*dst, v);
-        *dst = v;
-    }
-}
-
-// ------------------------------------------------------------------ staged x-pass variants
-// W = 16 columns = ROWS image rows x CC coils (CC in {4, 8, 16}).  Forward:
-// each row's image values and its contiguous coil-map row are staged in shared
-// memory with cp.async, the products formed there.  Adjoint: the coil
-// combination runs with one thread per (x, coil) and a shuffle reduction over
-// the CC lanes of a coil group (no bank conflicts).
-template <int L, int W, int CC>
-__global__ void __launch_bounds__(256) k_fwd_x_st(FwdXArgs a) {
-    constexpr int ROWS = W / CC;
-    extern __shared__ float2 sm[];
-    float2* smA = sm;
-    float2* smB = sm + L * W;
-    float2* tws = sm + 2 * L * W;
-    const int X = a.X;
-    float2* s_img = smB;                 // [ROWS][X]
-    float2* s_map = smB + ROWS * X;      // [ROWS][X][CC]
-    __shared__ float s_apzy[ROWS];
-    const int img = (int)(blockIdx.x % (unsigned)a.n_img);      // images of one row block run side by side
-    const int row0 = (int)(blockIdx.x / (unsigned)a.n_img) * ROWS;
-    const int c0 = blockIdx.z * CC;
-    const int nrows = a.Z * a.Y;
-    const float2* __restrict__ src = a.img + (int64_t)img * a.img_stride;
-    for (int i = threadIdx.x; i < L; i += 256) tws[i] = a.tw[i];
-    if (threadIdx.x < ROWS) {
-        const int row = row0 + threadIdx.x;
-        float v = 0.f;
-        if (row < nrows) {
-            const int z = row / a.Y, y = row - z * a.Y;
-            v = a.apz[z] * a.apy[y] * a.scale;
-        }
-        s_apzy[threadIdx.x] = v;
-    }
-    for (int i = threadIdx.x; i < ROWS * X; i += 256) {
-        const int rl = i / X, x = i - rl * X;
-        const int row = row0 + rl;
-        cp_async8(s_img + i, row < nrows ? src + (int64_t)row * X + x : src, row < nrows ? 8 : 0);
-    }
-    if (a.maps) {
-        for (int i = threadIdx.x; i < ROWS * X * CC; i += 256) {
-            const int rl = i / (X * CC), rem = i - rl * X * CC;
-            const int x = rem / CC, cl = rem - x * CC;
-            const int row = row0 + rl, c = c0 + cl;
-            const bool ok = row < nrows && c < a.C;
-            cp_async8(s_map + i, ok ? a.maps + ((int64_t)row * X + x) * a.C + c : a.maps, ok ? 8 : 0);
-        }
-    }
-    cp_async_wait_all();
-    __syncthreads();
-#pragma unroll 4
-    for (int idx = threadIdx.x; idx < L * W; idx += 256) {
-        const int m = idx / W, w = idx - m * W;
-        const int rl = w / CC, cl = w - rl * CC;
-        int j = m + a.h;
-        if (j >= L) j -= L;
-        const int x = j - a.pad;
-        float2 v = make_float2(0.f, 0.f);
-        if (x >= 0 && x < X) {
-            v = s_img[rl * X + x];
-            if (a.maps) v = cmul(v, s_map[(rl * X + x) * CC + cl]);
-            v = cscale(v, s_apzy[rl] * a.apx[x]);
-        }
-        smA[idx] = v;
-    }
-    __syncthreads();
-    const int h = a.h;
-    auto store = [&](int k, int w, float2 v) {
-        const int rl = w / CC, cl = w - rl * CC;
-        const int row = row0 + rl, c = c0 + cl;
-        if (row >= nrows || c >= a.C) return;
-        int g = k + h;
-        if (g >= L) g -= L;
-        a.out[((int64_t)row * a.OSX + g) * a.ncol + (int64_t)img * a.C + c] = v;
-    };
-    fft_ct<L, W, 256, false>(smA, smB, tws, store);
-}
-
-template <int L, int W, int CC>
-__global__ void __launch_bounds__(256) k_adj_x_st(AdjXArgs a) {
-    constexpr int ROWS = W / CC;
-    extern __shared__ float2 sm[];
-    float2* buf0 = sm;
-    float2* buf1 = sm + L * W;
-    float2* tws = sm + 2 * L * W;
-    float2* acc = tws + L;                  // [ROWS][X]
-    for (int i = threadIdx.x; i < L; i += 256) tws[i] = a.tw[i];
-    for (int i = threadIdx.x; i < ROWS * a.X; i += 256) acc[i] = make_float2(0.f, 0.f);
-    const int img = (int)(blockIdx.x % (unsigned)a.n_img);      // images of one row block run side by side
-    const int row0 = (int)(blockIdx.x / (unsigned)a.n_img) * ROWS;
-    const int nrows = a.Z * a.Y;
-    const int X = a.X;
-    float2* ep = fft_ct_free<L>(buf0, buf1);
-    const int shift = a.h - a.pad;
-    for (int c0 = 0; c0 < a.C; c0 += CC) {
-#pragma unroll 4
-        for (int idx = threadIdx.x; idx < L * W; idx += 256) {
-            const int m = idx / W, w = idx - m * W;
-            const int rl = w / CC, cl = w - rl * CC;
-            const int row = row0 + rl, c = c0 + cl;
-            int j = m + a.h;
-            if (j >= L) j -= L;
-            const bool ok = row < nrows && c < a.C;
-            cp_async8(buf0 + idx, ok ? a.in + ((int64_t)row * a.OSX + j) * a.ncol + (int64_t)img * a.C + c : a.in,
-                      ok ? 8 : 0);
-        }
-        cp_async_wait_all();
-        __syncthreads();
-        auto store = [&](int k, int w, float2 v) {
-            int o = k + shift;
-            o = o >= L ? o - L : (o < 0 ? o + L : o);
-            if (o < X) ep[o * W + w] = v;
-        };
-        fft_ct<L, W, 256, true>(buf0, buf1, tws, store);
-        __syncthreads();
-        // thread (x, w): conj(S) product, then a sum over the CC lanes of one row.
-        // Every lane runs every iteration (the shuffles need the whole warp).
-        for (int base = 0; base < X * W; base += 256) {
-            const int i = base + (int)threadIdx.x;
-            const bool live = i < X * W;
-            const int x = i / W, w = i - x * W;
-            const int rl = w / CC, cl = w - rl * CC;
-            const int row = row0 + rl, c = c0 + cl;
-            float2 v = make_float2(0.f, 0.f);
-            if (live && row < nrows && c < a.C) {
-                v = ep[i];
-                if (a.maps) v = cmulc(v, a.maps[((int64_t)row * X + x) * a.C + c]);
-            }
-#pragma unroll
-            for (int o = CC / 2; o > 0; o >>= 1) {
-                v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-                v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-            }
-            if (live && cl == 0) acc[rl * X + x] = cadd(acc[rl * X + x], v);
-        }
-        __syncthreads();
-    }
-    for (int i = threadIdx.x; i < ROWS * X; i += 256) {
-        const int rl = i / X, x = i - rl * X;
-        const int row = row0 + rl;
-        if (row >= nrows) continue;
-        const int z = row / a.Y, y = row - z * a.Y;
-        const float sc = a.apz[z] * a.apy[y] * a.apx[x] * a.scale;
-        float2 v = cscale(acc[i], sc);
-        float2* dst = a.img + (int64_t)img * a.img_stride + (int64_t)row * X + x;
-        if (a.accumulate) v = cadd(*dst, v);
-        *dst = v;
-    }
-}
-
 // ------------------------------------------------------------------ TMA x-pass variants
 // One image row x W coils per CTA (W = CC).  Forward: the image row and the
 // row's W coil-map columns arrive by TMA in the FFT's second buffer, the
@@ -1019,7 +619,7 @@ __global__ void __launch_bounds__(256) k_adj_x_st(AdjXArgs a) {
 // shift g = (k + L/2) mod L splits it in two).  Adjoint: per coil group the
 // [L][W] tile arrives as two boxes (rows rotated by L/2), the inverse FFT
 // writes the cropped row into shared memory, and the conj(S) product and the
-// coil sum run as in k_adj_x_st.  Loads complete on one mbarrier (phase per
+// coil sum run on the staged tile.  Loads complete on one mbarrier (phase per
 // coil group) with a bounded wait.
 
 template <int L, int W, int NT = 256>
@@ -1028,7 +628,6 @@ __global__ void __launch_bounds__(NT) k_fwd_x_tma(FwdXArgs a, const __grid_const
                                                    const __grid_constant__ CUtensorMap tout) {
     extern __shared__ __align__(128) unsigned char xsm_raw[];
     __shared__ __align__(8) uint64_t bar;
-    __shared__ float s_apzy;
     float2* sm = align128(xsm_raw);
     float2* smA = sm;
     float2* smB = sm + L * W;
@@ -1045,8 +644,6 @@ __global__ void __launch_bounds__(NT) k_fwd_x_tma(FwdXArgs a, const __grid_const
         mbar_expect_tx(&bar, (unsigned)(X * (W + 1) * sizeof(float2)));
         tma_load_3d(s_img, &timg, &bar, 0, row, img);
         tma_load_3d(s_map, &tmap, &bar, c0, 0, row);
-        const int z = row / a.Y, y = row - z * a.Y;
-        s_apzy = a.apz[z] * a.apy[y] * a.scale;
     }
     for (int i = threadIdx.x; i < L; i += NT) tws[i] = a.tw[i];
     const bool ok = mbar_wait_or_drain(&bar, 0, a.poll);
@@ -1054,17 +651,14 @@ __global__ void __launch_bounds__(NT) k_fwd_x_tma(FwdXArgs a, const __grid_const
         if (threadIdx.x == 0) atomicOr(a.err, kDevErrTmaWait);
         return;
     }
-    const float apzy = s_apzy;
     const int h = a.h, pad = a.pad;
-    const float* apx = a.apx;
-    // input element m of column w: u * S * apodisation * scale at x = (m + L/2) mod L - pad, 0 outside the
-    // image (scaling the image row once in shared memory first measured 1 % slower: one more barrier)
+    // input element m of column w: u times the scaled map at x = (m + L/2) mod L - pad, 0 outside the image
     auto load = [=](int m, int w) {
         int j = m + h;
         if (j >= L) j -= L;
         const int x = j - pad;
         float2 v = make_float2(0.f, 0.f);
-        if (x >= 0 && x < X) v = cscale(cmul(s_img[x], s_map[x * W + w]), apzy * apx[x]);
+        if (x >= 0 && x < X) v = cmul(s_img[x], s_map[x * W + w]);
         return v;
     };
     float2* ep = fft_ct_free<L>(smA, smB);
@@ -1154,11 +748,7 @@ __global__ void __launch_bounds__(NT, MINB) k_adj_x_tma(AdjXArgs a, const __grid
         }
     }
     if (x < X) {
-        const int z = row / a.Y, y = row - z * a.Y;
-        float2 v = cscale(s, a.apz[z] * a.apy[y] * a.scale * a.apx[x]);
-        float2* dst = a.img + (int64_t)img * a.img_stride + (int64_t)row * X + x;
-        if (a.accumulate) v = cadd(*dst, v);
-        *dst = v;
+        a.img[(int64_t)img * a.img_stride + (int64_t)row * X + x] = s;
     }
 }
 
@@ -1178,7 +768,6 @@ __global__ void __launch_bounds__(kWideNT, 5) k_fwd_x_wide(FwdXArgs a, const __g
     constexpr int NT = kWideNT;
     extern __shared__ __align__(128) unsigned char xsm_raw[];
     __shared__ __align__(8) uint64_t bar;
-    __shared__ float s_apzy;
     float2* sm = align128(xsm_raw);
     float2* smA = sm;
     float2* smB = sm + L * W;
@@ -1195,8 +784,6 @@ __global__ void __launch_bounds__(kWideNT, 5) k_fwd_x_wide(FwdXArgs a, const __g
         mbar_expect_tx(&bar, (unsigned)(X * (W + 1) * sizeof(float2)));
         tma_load_3d(s_img, &timg, &bar, 0, row, img);
         tma_load_3d(s_map, &tmap, &bar, c0, 0, row);
-        const int z = row / a.Y, y = row - z * a.Y;
-        s_apzy = a.apz[z] * a.apy[y] * a.scale;
     }
     for (int i = threadIdx.x; i < L; i += NT) tws[i] = a.tw[i];
     const bool ok = mbar_wait_or_drain(&bar, 0, a.poll);
@@ -1204,15 +791,13 @@ __global__ void __launch_bounds__(kWideNT, 5) k_fwd_x_wide(FwdXArgs a, const __g
         if (threadIdx.x == 0) atomicOr(a.err, kDevErrTmaWait);
         return;
     }
-    const float apzy = s_apzy;
     const int h = a.h, pad = a.pad;
-    const float* apx = a.apx;
     auto load = [=](int m, int w) {
         int j = m + h;
         if (j >= L) j -= L;
         const int x = j - pad;
         float2 v = make_float2(0.f, 0.f);
-        if (x >= 0 && x < X) v = cscale(cmul(s_img[x], s_map[x * W + w]), apzy * apx[x]);
+        if (x >= 0 && x < X) v = cmul(s_img[x], s_map[x * W + w]);
         return v;
     };
     float2* ep = fft_ct_free<L, 1>(smA, smB);        // smA: the staged row is read by the first pass only
@@ -1266,8 +851,6 @@ __global__ void __launch_bounds__(kWideNT, 5) k_adj_x_wide(AdjXArgs a, const __g
     for (int i = threadIdx.x; i < L; i += NT) tws[i] = a.tw[i];
     const int shift = a.h - a.pad;
     const float4* mrow = reinterpret_cast<const float4*>(a.maps + (int64_t)row * X * a.C);
-    const int z = row / a.Y, y = row - z * a.Y;
-    const float szy = a.apz[z] * a.apy[y] * a.scale;
     auto issue = [&](int c0, float2* dst) {
         mbar_expect_tx(&bar, (unsigned)(L * W * sizeof(float2)));
         const int col = img * a.C + c0;
@@ -1309,9 +892,9 @@ __global__ void __launch_bounds__(kWideNT, 5) k_adj_x_wide(AdjXArgs a, const __g
                 // lane 2i forms t0.x + t1.x, lane 2i + 1 t0.y + t1.y; each adds its
                 // scaled float into the image row (the first group writes it)
                 const float recv = __shfl_xor_sync(0xffffffffu, hf ? t.x : t.y, 1);
-                float v = (hf ? recv + t.y : t.x + recv) * (szy * a.apx[x]);
+                float v = hf ? recv + t.y : t.x + recv;
                 float* dst = reinterpret_cast<float*>(a.img + (int64_t)img * a.img_stride + (int64_t)row * X + x) + hf;
-                if (a.accumulate || c0 > 0) v = *dst + v;
+                if (c0 > 0) v = *dst + v;
                 *dst = v;
             }
         }
@@ -1985,13 +1568,16 @@ __global__ void k_unsort_ksp(const float2* __restrict__ internal, float2* __rest
     ext[(int64_t)col * M + perm[s]] = internal[i];
 }
 
-// (Z, Y, X, C) <- (C, Z, Y, X)
-__global__ void k_interleave_maps(const float2* __restrict__ src, float2* __restrict__ dst, int64_t N, int C) {
+// (Z, Y, X, C) <- (C, Z, Y, X), times the separable apodisation and the NUFFT's scale (the same in
+// both directions), which the x passes then need not apply per column.
+__global__ void k_interleave_maps(const float2* __restrict__ src, float2* __restrict__ dst, int64_t N, int C, int Y, int X,
+                                  const float* __restrict__ apz, const float* __restrict__ apy,
+                                  const float* __restrict__ apx, float scale) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N * C) return;
-    const int64_t v = i / C;
-    const int c = (int)(i - v * C);
-    dst[i] = src[(int64_t)c * N + v];
+    const int64_t v = i / C, zy = v / X;
+    const int c = (int)(i - v * C), x = (int)(v - zy * X), z = (int)(zy / Y), y = (int)(zy - (int64_t)z * Y);
+    dst[i] = cscale(src[(int64_t)c * N + v], apz[z] * apy[y] * apx[x] * scale);
 }
 
 // ------------------------------------------------------------------ host helpers
@@ -2098,6 +1684,23 @@ static bool line_tma_setup(LineArgs& la, int L, int W, int64_t outer, CUtensorMa
     return true;
 }
 
+// Every length's FFT pass kernels (filled once, in the translation units tr_lines_*.cu).
+#define TR_LINE_PARTS(X) X(0) X(1) X(2) X(3) X(4) X(5) X(6) X(7)
+#define TR_LINE_FILL_DECL(K) void lp_fill_##K(LineKernels* table);
+TR_LINE_PARTS(TR_LINE_FILL_DECL)
+#undef TR_LINE_FILL_DECL
+const LineKernels& line_kernels(int L) {
+    static LineKernels table[kMaxLineLen + 1];
+    static const LineKernels none;
+    static std::once_flag once;
+    std::call_once(once, [] {
+#define TR_LINE_FILL(K) lp_fill_##K(table);
+        TR_LINE_PARTS(TR_LINE_FILL)
+#undef TR_LINE_FILL
+    });
+    return L <= kMaxLineLen ? table[L] : none;
+}
+
 // colmask (z passes of bin grids, ncol k-space columns): skip the lines of
 // unoccupied tile columns (inverse: write their zeros), see lines_unoccupied.
 static tr_status launch_line(tr_plan* p, int axis, const float2* in, float2* out, int64_t outer, int64_t inner,
@@ -2134,11 +1737,21 @@ static tr_status launch_line(tr_plan* p, int axis, const float2* in, float2* out
         tma = p->use_tma && line_tma_setup(la, LV, ct_width(LV), outer, &tin, &tout);                     \
         if (tma)                                                                                          \
             fn = inv ? (const void*)k_line_tma<LV, ct_width(LV), true> : (const void*)k_line_tma<LV, ct_width(LV), false>; \
-        else                                                                                              \
-            fn = inv ? (const void*)k_line_ct<LV, ct_width(LV), true> : (const void*)k_line_ct<LV, ct_width(LV), false>; \
         break;
-    switch (A.L) { TR_CT_LENGTHS(TR_LINE_CASE) default: break; }
+    switch (A.L) { TR_LINE_TMA_LENGTHS(TR_LINE_CASE) default: break; }
 #undef TR_LINE_CASE
+    if (!tma) {
+        const LineKernels& lk = line_kernels(A.L);
+        if (lk.fwd) {
+            const void* lfn = inv ? lk.inv : lk.fwd;
+            TR_TRY(set_smem_limit(lfn, lk.smem));
+            void* args[] = {&la};
+            TR_CUDA(cudaLaunchKernel(lfn, dim3((unsigned)((inner + kLineW - 1) / kLineW), (unsigned)outer),
+                                     dim3((unsigned)lk.threads), args, lk.smem, st));
+            return TR_OK;
+        }
+        la.W = p->line_width;
+    }
     unsigned nt = (unsigned)line_threads(A.L, la.W);
     // 320-point lines in two passes (radices 20, 16: measured 15 % faster on the y
     // passes of the 160 x 320 x 320 grid); at 160 the two passes (10, 16: 256 and
@@ -2180,20 +1793,10 @@ static tr_status stage_fwd_x(tr_plan* p, const float2* images, int64_t img_strid
     fa.OSX = OSX;
     fa.h = p->ax[2].h;
     fa.pad = p->ax[2].pad;
-    // launch shape: compile-time kernels for the listed lengths
-    bool ct = false;
+    bool ct = false;          // a length the TMA kernels are compiled for
 #define TR_IS_CT(LV) case LV: ct = true; break;
     switch (OSX) { TR_CT_LENGTHS(TR_IS_CT) default: break; }
 #undef TR_IS_CT
-    const int Wct = ct_width(OSX);
-    const bool pow2C = (C & (C - 1)) == 0;
-    if (ct && (C >= Wct || pow2C)) {
-        fa.cc = C >= Wct ? Wct : C;
-        fa.rows = Wct / fa.cc;
-    } else {
-        fa.cc = coils_per_cta(C);
-        fa.rows = std::max(1, 16 / fa.cc);
-    }
     fa.apz = p->ax[0].apod;
     fa.apy = p->ax[1].apod;
     fa.apx = p->ax[2].apod;
@@ -2251,25 +1854,22 @@ static tr_status stage_fwd_x(tr_plan* p, const float2* images, int64_t img_strid
             return TR_OK;
         }
     }
+    const LineKernels& lk = line_kernels(OSX);
+    if (lk.fwd_x) {
+        const int64_t q = (int64_t)Z * Y * fa.ncol;
+        TR_TRY(set_smem_limit(lk.fwd_x, lk.smem));
+        void* args[] = {&fa};
+        TR_CUDA(cudaLaunchKernel(lk.fwd_x, dim3((unsigned)((q + kLineW - 1) / kLineW)), dim3((unsigned)lk.threads), args,
+                                 lk.smem, st));
+        return TR_OK;
+    }
+    fa.cc = coils_per_cta(C);
+    fa.rows = std::max(1, 16 / fa.cc);
     const int W = fa.rows * fa.cc;
     const size_t smem = fft_smem_bytes(OSX, W);
     // the n_img CTAs of one row block are adjacent, so the coil-map rows they share come from L2
     dim3 grid((unsigned)(((Z * Y + fa.rows - 1) / fa.rows) * n_img), 1u, (unsigned)((C + fa.cc - 1) / fa.cc));
-    const void* fn = nullptr;
-    // staged variant when a row's coil-map slice fits the free FFT buffer
-    const bool staged = ct && W == Wct && fa.cc >= 4 && (size_t)fa.rows * X * (fa.cc + 1) <= (size_t)OSX * W;
-#define TR_FWDX_CASE(LV)                                                                              \
-    case LV: {                                                                                        \
-        constexpr int WV = ct_width(LV);                                                              \
-        if (staged) fn = fa.cc == 16 ? (const void*)k_fwd_x_st<LV, WV, (WV >= 16 ? 16 : WV)>          \
-                       : fa.cc == 8 ? (const void*)k_fwd_x_st<LV, WV, 8> : (const void*)k_fwd_x_st<LV, WV, 4>; \
-        else if (W == WV) fn = (const void*)k_fwd_x_ct<LV, WV>;                                       \
-        else if (W == 12 && WV == 16) fn = (const void*)k_fwd_x_ct<LV, 12>;                          \
-        break;                                                                                        \
-    }
-    switch (OSX) { TR_CT_LENGTHS(TR_FWDX_CASE) default: break; }
-#undef TR_FWDX_CASE
-    if (!fn) fn = (const void*)k_fwd_x;
+    const void* fn = (const void*)k_fwd_x;
     TR_TRY(set_smem_limit(fn, smem));
     void* args[] = {&fa};
     TR_CUDA(cudaLaunchKernel(fn, grid, dim3(256), args, smem, st));
@@ -2374,15 +1974,6 @@ static tr_status stage_fwd_y(tr_plan* p, int ncol, cudaStream_t st) {
                        false, st);
 }
 
-static bool ct_compiled(int L) {
-    switch (L) {
-#define TR_CT_CASE_TRUE(LV) case LV: return true;
-        TR_CT_LENGTHS(TR_CT_CASE_TRUE)
-#undef TR_CT_CASE_TRUE
-        default: return false;
-    }
-}
-
 // Unoccupied-column mask of a bin for its z passes and its gridding (null: no
 // skipping).  Gridding leaves the tiles of unoccupied columns unwritten only
 // when no z-pass CTA mixes lines of occupied and unoccupied columns (a mixed
@@ -2390,8 +1981,7 @@ static bool ct_compiled(int L) {
 // when ncol is a multiple of the z pass's W (16 at the compiled lengths, the
 // runtime-radix width elsewhere).
 static const uint8_t* bin_colmask(const tr_plan* p, int bin, int ncol) {
-    const int zw = ct_compiled(p->os[0]) ? ct_width(p->os[0]) : p->line_width;
-    if (!p->skip_empty_cols || !p->colmask || ncol % zw) return nullptr;
+    if (!p->skip_empty_cols || !p->colmask || ncol % kLineW) return nullptr;
     return p->colmask + (int64_t)bin * p->ntile[1] * p->ntile[2];
 }
 
@@ -2568,15 +2158,6 @@ static tr_status stage_adj_x(tr_plan* p, int n_img, const float2* maps, int C, f
 #define TR_IS_CT(LV) case LV: ct = true; break;
     switch (OSX) { TR_CT_LENGTHS(TR_IS_CT) default: break; }
 #undef TR_IS_CT
-    const int Wct = ct_width(OSX);
-    const bool pow2C = (C & (C - 1)) == 0;
-    if (ct && (C >= Wct || pow2C)) {
-        aa.cc = C >= Wct ? Wct : C;
-        aa.rows = Wct / aa.cc;
-    } else {
-        aa.cc = coils_per_cta(C);
-        aa.rows = std::max(1, 16 / aa.cc);
-    }
     aa.Z = Z;
     aa.Y = Y;
     aa.X = X;
@@ -2591,7 +2172,6 @@ static tr_status stage_adj_x(tr_plan* p, int n_img, const float2* maps, int C, f
     aa.S = stages_of(p->ax[2]);
     aa.img = images;
     aa.img_stride = img_stride;
-    aa.accumulate = 0;
     aa.err = p->dev_err;
     aa.poll = p->poll_limit;
     // TMA variant: one image row per CTA, coil groups of wt (8, or 4 where 8 does not divide C
@@ -2625,24 +2205,22 @@ static tr_status stage_adj_x(tr_plan* p, int n_img, const float2* maps, int C, f
             return TR_OK;
         }
     }
+    const LineKernels& lk = line_kernels(OSX);
+    if (lk.adj_x) {
+        const int64_t rows = (int64_t)Z * Y, per = aa.ncol >= kLineW ? 1 : kLineW / aa.ncol;
+        const size_t smem = maps ? lk.smem_adj_x : lk.smem;
+        TR_TRY(set_smem_limit(lk.adj_x, smem));
+        void* args[] = {&aa};
+        TR_CUDA(cudaLaunchKernel(lk.adj_x, dim3((unsigned)((rows + per - 1) / per)), dim3((unsigned)lk.threads), args, smem,
+                                 st));
+        return TR_OK;
+    }
+    aa.cc = coils_per_cta(C);
+    aa.rows = std::max(1, 16 / aa.cc);
     const int W = aa.rows * aa.cc;
     const size_t smem = fft_smem_bytes(OSX, W) + (size_t)aa.rows * X * sizeof(float2);
     dim3 grid((unsigned)(((Z * Y + aa.rows - 1) / aa.rows) * n_img));
-    const void* fn = nullptr;
-    const bool staged = ct && W == Wct;   // cc is a power of two here
-#define TR_ADJX_CASE(LV)                                                                              \
-    case LV: {                                                                                        \
-        constexpr int WV = ct_width(LV);                                                              \
-        if (staged) fn = aa.cc == 16 ? (const void*)k_adj_x_st<LV, WV, (WV >= 16 ? 16 : WV)>          \
-                       : aa.cc == 8 ? (const void*)k_adj_x_st<LV, WV, 8>                              \
-                       : aa.cc == 4 ? (const void*)k_adj_x_st<LV, WV, 4>                              \
-                       : aa.cc == 2 ? (const void*)k_adj_x_st<LV, WV, 2> : (const void*)k_adj_x_st<LV, WV, 1>; \
-        else if (W == 12 && WV == 16) fn = (const void*)k_adj_x_ct<LV, 12>;                          \
-        break;                                                                                        \
-    }
-    switch (OSX) { TR_CT_LENGTHS(TR_ADJX_CASE) default: break; }
-#undef TR_ADJX_CASE
-    if (!fn) fn = (const void*)k_adj_x;
+    const void* fn = (const void*)k_adj_x;
     TR_TRY(set_smem_limit(fn, smem));
     void* args[] = {&aa};
     TR_CUDA(cudaLaunchKernel(fn, grid, dim3(256), args, smem, st));
@@ -3256,8 +2834,8 @@ tr_status tr_plan_set_maps(tr_plan* p, const void* mps, void* stream) {
         p->workspace_bytes += N * p->C * (int64_t)sizeof(float2);
     }
     const int64_t tot = N * p->C;
-    k_interleave_maps<<<(unsigned)((tot + 255) / 256), 256, 0, (cudaStream_t)stream>>>((const float2*)mps, p->maps,
-                                                                                        N, p->C);
+k_interleave_maps<<<(unsigned)((tot + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+        (const float2*)mps, p->maps, N, p->C, p->n[1], p->n[2], p->ax[0].apod, p->ax[1].apod, p->ax[2].apod, p->fwd_scale);
     TR_CHECK_LAUNCH();
     return TR_OK;
 }

@@ -246,7 +246,8 @@ tr_status nufft_adjoint_cols(tr_plan* p, int bin, const float2* ksp, int n_img, 
                              bool use_dcf, float2* images, int64_t img_stride, cudaStream_t st,
                              const int32_t* perm = nullptr);
 tr_status wavelet_prepare(tr_plan* p);
-tr_status wavelet_dual(tr_plan* p, const float2* u_bar, float2* p_w2, float sigma, float lam, cudaStream_t st);
+tr_status wavelet_dual(tr_plan* p, const float2* u_bar, float2* p_w2, float sigma, float lam, cudaStream_t st,
+                       bool fresh = false);
 tr_status wavelet_adjoint(tr_plan* p, const float2* p_w2, float2* out, cudaStream_t st);
 void wavelet_destroy(tr_plan* p);
 void wavelet_info(const tr_plan* p, int32_t* levels, int64_t* coeffs);

@@ -193,6 +193,7 @@ struct tr_plan {
     float4* ks = nullptr;        // (kz, ky, kx, dcf) in oversampled-grid units, sorted
     void* taps = nullptr;        // per-sample first taps and KB weights (TapRec), sorted
     int32_t* perm = nullptr;     // sorted position -> acquisition index within the bin
+    int32_t* inv_perm = nullptr;     // per bin: place of an acquired sample in the tile order
     int2* glist = nullptr;          // gridding gather lists: (sample in bin, packed tap offsets), all bins
     int32_t* list_start = nullptr;  // per bin [ntiles + 1] (relative to the bin's first entry)
     int32_t* tile_order = nullptr;  // per bin [ntiles]: busy tiles heaviest first, then the empty tiles of

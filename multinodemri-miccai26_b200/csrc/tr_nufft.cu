@@ -1150,9 +1150,13 @@ __global__ void __launch_bounds__(256) k_interp_rows(const float2* __restrict__ 
 // g = column group of CG consecutive columns.  The plan holds, per tile, the
 // list of samples whose KB support meets it (in sorted-sample order) with the
 // tap offsets of the tile origin, so a CTA only stages those samples' weights
-// and dcf-weighted values in shared memory, 64 at a time, and every
-// (point, column) accumulator sums them in list order: no atomics, bitwise
-// reproducible.  The launch runs work items first: a tile's list range
+// (times dcf) and values in shared memory, 32 at a time, the next 32 while it sums
+// the current ones (one CTA barrier per 32), and every (point, column) accumulator
+// sums them in list order: no atomics, bitwise reproducible.  Each half-warp (a tile
+// row) steps through the entries that reach its row, found by a ballot over the row
+// weights.  Bound by instruction issue; with every warp stepping through every entry
+// and three barriers per 32 the gridding of 96 columns (128 x 256 x 256 image) took
+// 3.81 ms and of 72 columns (112 x 160 x 160) 1.33 ms, now 3.32 and 1.18 ms.  The launch runs work items first: a tile's list range
 // (lists longer than kSplitEntries are cut into ranges whose partial tiles go
 // to a scratch buffer, the first range writing the grid), heaviest first; the
 // trailing CTAs write zeros into tiles no sample reaches, kZeroTiles each.
@@ -1206,22 +1210,18 @@ __device__ __forceinline__ void tile_geometry(const SpreadArgs& a, int tile, int
 }
 
 // Tile gather.  TMA = true (even column counts, aligned k-space): each
-// entry's values arrive by one bulk copy (cp.async.bulk) on an mbarrier, the
-// dcf weight folds into the row weights, and finished tiles (and the zero
-// tiles) leave by one 4-D TMA store each, clipped at the grid edge by the TMA
-// unit.  TMA = false: values staged by plain loads, coalesced warp stores.
+// entry's values arrive by one bulk copy (cp.async.bulk) on an mbarrier, and
+// finished tiles (and the zero tiles) leave by one 4-D TMA store each, clipped
+// at the grid edge by the TMA unit.  TMA = false: values staged by plain loads, coalesced warp stores.
 template <int CG, bool TMA>
 __global__ void __launch_bounds__(256, (CG >= 6 ? 3 : (CG >= 4 ? 4 : 5))) k_spread(SpreadArgs a,
                                                                  const __grid_constant__ CUtensorMap tgrid) {
     extern __shared__ __align__(128) unsigned char smraw_[];
-    __shared__ int l_rel[kSpreadSub];
-    __shared__ float s_dcf[kSpreadSub];
-    __shared__ float s_wzy[kSpreadSub * 16];
-    __shared__ __align__(16) float s_wx[kSpreadSub * 4];
+    __shared__ float s_wzy[2][kSpreadSub * 17];          // (z, y) weight times dcf of the 16 tile rows
+    __shared__ __align__(16) float s_wx[2][kSpreadSub * 4];
     __shared__ __align__(8) uint64_t bar;
     unsigned char* smraw = reinterpret_cast<unsigned char*>(align128(smraw_));
-    float* c_w = reinterpret_cast<float*>(smraw);                        // [kSpreadSub][16]
-    float2* dq = reinterpret_cast<float2*>(c_w + 16 * kSpreadSub);       // [kSpreadSub][cchunk]
+    float2* dq = reinterpret_cast<float2*>(smraw);       // [2][kSpreadSub][cchunk]
     const int tid = threadIdx.x;
     const int cst = a.cchunk;                                            // row stride of dq
 
@@ -1290,81 +1290,97 @@ __global__ void __launch_bounds__(256, (CG >= 6 ? 3 : (CG >= 4 ? 4 : 5))) k_spre
 #pragma unroll
         for (int j = 0; j < CG; ++j) acc[x][j] = make_float2(0.f, 0.f);
 
-    unsigned phase = 0;
-    for (int base = beg; base < end; base += kSpreadSub, phase ^= 1u) {
+    // A sub-chunk's values travel (bulk copies, or loads) into one buffer while the other one is summed,
+    // and its weights are fetched then too: eight threads per entry, two tile rows each (and one tile
+    // column by four of them).
+    const int we = tid >> 3, wp = tid & 7, wz = wp >> 1, wy = (wp & 1) * 2;
+    auto copy_vals = [&](int base, int buf) {
         const int ns = min(kSpreadSub, end - base);
+        float2* d = dq + buf * kSpreadSub * cst;
         if constexpr (TMA) {
-            __syncthreads();                       // dq free; the barrier init is visible
             if (tid < 32) {                        // warp 0: one bulk copy per entry
                 if (tid == 0) mbar_expect_tx(&bar, (unsigned)(ns * ncc * sizeof(float2)));
                 __syncwarp();
-                for (int cand = tid; cand < ns; cand += 32) {
-                    const int sm = a.list[base + cand].x;
-                    bulk_g2s(dq + cand * cst, a.vals + (int64_t)sm * a.ncol + col0, (unsigned)(ncc * sizeof(float2)),
-                             &bar);
-                }
+                if (tid < ns)
+                    bulk_g2s(d + tid * cst, a.vals + (int64_t)a.list[base + tid].x * a.ncol + col0,
+                             (unsigned)(ncc * sizeof(float2)), &bar);
             }
-        }
-        if (tid < 4 * ns) {
-            const int cand = tid >> 2, part = tid & 3;
-            const int2 e = a.list[base + cand];
-            reinterpret_cast<float4*>(c_w)[cand * 4 + part] = a.taps[e.x].w[part];
-            if (part == 0) {
-                l_rel[cand] = e.y;
-                s_dcf[cand] = (TMA && a.use_dcf) ? a.ks[e.x].w : 1.0f;
-            }
-        }
-        if constexpr (!TMA) {
+        } else {
             for (int cand = tid >> 5; cand < ns; cand += 8) {     // one warp per entry, lanes over columns
-                const int sm = a.list[base + cand].x;
-                const float2* src = a.vals + (int64_t)sm * a.ncol + col0;
-                const float dw = a.use_dcf ? a.ks[sm].w : 1.0f;
-                for (int col = tid & 31; col < ncc; col += 32) dq[cand * cst + col] = cscale(src[col], dw);
+                const float2* src = a.vals + (int64_t)a.list[base + cand].x * a.ncol + col0;
+                for (int col = tid & 31; col < ncc; col += 32) d[cand * cst + col] = src[col];
             }
         }
-        __syncthreads();
-        // per entry: the (z, y) weight of each of the 16 tile rows (times the dcf
-        // weight on the TMA path) and the x weight of each of the 4 tile columns
-        for (int i = tid; i < ns * 20; i += 256) {
-            const int cand = i / 20, k = i - cand * 20;
-            const int pk = l_rel[cand];
-            const float* w = c_w + 16 * cand;
-            if (k < 16) {
-                const int az = (pk & 0xff) - 128 + (k >> 2);
-                const int ay = ((pk >> 8) & 0xff) - 128 + (k & 3);
-                s_wzy[cand * 16 + k] =
-                    ((unsigned)az <= 4u && (unsigned)ay <= 4u) ? (w[az] * w[5 + ay]) * s_dcf[cand] : 0.f;
-            } else {
-                const int ax = ((pk >> 16) & 0xff) - 128 + (k - 16);
-                s_wx[cand * 4 + (k - 16)] = (unsigned)ax <= 4u ? w[10 + ax] : 0.f;
-            }
-        }
+    };
+    float f0 = 0.f, f1 = 0.f, fx = 0.f;            // this thread's weights of the next sub-chunk
+    auto fetch_weights = [&](int base) {
+        f0 = f1 = fx = 0.f;
+        if (base + we >= end) return;
+        const int2 e = a.list[base + we];
+        const float* w = reinterpret_cast<const float*>(a.taps[e.x].w);
+        const int az = (e.y & 0xff) - 128 + wz, ay = ((e.y >> 8) & 0xff) - 128 + wy, ax = ((e.y >> 16) & 0xff) - 128 + wp;
+        const float d = a.use_dcf ? a.ks[e.x].w : 1.0f;
+        const float vz = (unsigned)az <= 4u ? w[az] : 0.f;
+        f0 = (unsigned)ay <= 4u ? (vz * w[5 + ay]) * d : 0.f;
+        f1 = (unsigned)(ay + 1) <= 4u ? (vz * w[6 + ay]) * d : 0.f;
+        if (wp < 4) fx = (unsigned)ax <= 4u ? w[10 + ax] : 0.f;
+    };
+    auto put_weights = [&](int buf) {
+        s_wzy[buf][we * 17 + 2 * wp] = f0;
+        s_wzy[buf][we * 17 + 2 * wp + 1] = f1;
+        if (wp < 4) s_wx[buf][we * 4 + wp] = fx;
+    };
+    if (TMA) __syncthreads();                      // the barrier is initialised
+    copy_vals(beg, 0);
+    fetch_weights(beg);
+    put_weights(0);
+    int n = 0;
+    for (int base = beg; base < end; base += kSpreadSub, ++n) {
+        const int buf = n & 1;
         if constexpr (TMA) {
-            const bool ok = mbar_wait_or_drain(&bar, phase, a.poll);
-            if (__syncthreads_or(!ok)) {
+            const bool ok = mbar_wait_or_drain(&bar, (unsigned)buf, a.poll);
+            if (__syncthreads_or(!ok)) {           // weights and values of this sub-chunk are there
                 if (tid == 0) atomicOr(a.err, kDevErrTmaWait);
                 return;
             }
         } else {
             __syncthreads();
         }
-        for (int cc = 0; cc < ns; ++cc) {
-            const float wzy = s_wzy[cc * 16 + row];
-            if (wzy == 0.f) continue;
-            const float4 wx4 = reinterpret_cast<const float4*>(s_wx)[cc];
-            const float wx[4] = {wx4.x, wx4.y, wx4.z, wx4.w};
-            float2 v[CG];
+        const bool more = base + kSpreadSub < end;
+        if (more) {
+            copy_vals(base + kSpreadSub, buf ^ 1);
+            fetch_weights(base + kSpreadSub);
+        }
+        // entries that reach this thread's tile row, in list order; a half-warp (one row) takes its own,
+        // so a warp makes as many steps as the fuller of its two rows has entries
+        const float* wzy_s = s_wzy[buf];
+        const int lane = tid & 31, row0 = (tid >> 5) * 2;
+        const float r0 = wzy_s[lane * 17 + row0], r1 = wzy_s[lane * 17 + row0 + 1];
+        const unsigned m0 = __ballot_sync(0xffffffffu, r0 != 0.f), m1 = __ballot_sync(0xffffffffu, r1 != 0.f);
+        unsigned mine = (row & 1) ? m1 : m0;
+        const float2* vals = dq + buf * kSpreadSub * cst;
+        for (int steps = max(__popc(m0), __popc(m1)); steps > 0; --steps) {
+            if (mine) {
+                const int cc = __ffs(mine) - 1;
+                mine &= mine - 1;
+                const float wzy = wzy_s[cc * 17 + row];
+                const float4 wx4 = reinterpret_cast<const float4*>(s_wx[buf])[cc];
+                const float wx[4] = {wx4.x, wx4.y, wx4.z, wx4.w};
+                float2 v[CG];
 #pragma unroll
-            for (int j = 0; j < CG; ++j) v[j] = (g + 16 * j < ncc) ? dq[cc * cst + g + 16 * j] : make_float2(0.f, 0.f);
+                for (int j = 0; j < CG; ++j)
+                    v[j] = (g + 16 * j < ncc) ? vals[cc * cst + g + 16 * j] : make_float2(0.f, 0.f);
 #pragma unroll
-            for (int x = 0; x < 4; ++x) {
-                if (wx[x] == 0.f) continue;
-                const float wt = wzy * wx[x];
+                for (int x = 0; x < 4; ++x) {
+                    const float wt = wzy * wx[x];
+                    if (wx[x] != 0.f) {
 #pragma unroll
-                for (int j = 0; j < CG; ++j) acc[x][j] = cfma_real(wt, v[j], acc[x][j]);
+                        for (int j = 0; j < CG; ++j) acc[x][j] = cfma_real(wt, v[j], acc[x][j]);
+                    }
+                }
             }
         }
-        if constexpr (!TMA) __syncthreads();
+        if (more) put_weights(buf ^ 1);
     }
     // ---- store the tile in pieces of kSlabZ z planes: each piece is staged as
     // [kSpreadSub points][cchunk] in the value buffer, then leaves as one TMA box,
@@ -1532,40 +1548,68 @@ __global__ void __launch_bounds__(32 * kFewWarps) k_spread_few(SpreadArgs a, con
     }
 }
 
-// Split lists: grid tile += its partial tiles, in range order (one CTA per tile).
+// Split lists: grid tile += its partial tiles, in range order; one thread per value (with one CTA per
+// tile the k-space centre's 61 partial tiles of 96 columns took 157 us, now 45).
 __global__ void __launch_bounds__(256) k_spread_reduce(SpreadArgs a, const int4* __restrict__ splits) {
     const int4 sp = splits[blockIdx.x];
     int t0z, t0y, t0x, Tz, Ty, Tx;
     tile_geometry(a, sp.x, t0z, t0y, t0x, Tz, Ty, Tx);
-    const int n = 64 * a.ncol;
-    for (int i = threadIdx.x; i < n; i += 256) {
-        const int pt = i / a.ncol, col = i - pt * a.ncol;
-        const int pz = pt >> 4, py = (pt >> 2) & 3, px = pt & 3;
-        if (pz >= Tz || py >= Ty || px >= Tx) continue;
-        float2* g = a.grid + (((int64_t)(t0z + pz) * a.os1 + (t0y + py)) * a.os2 + (t0x + px)) * a.ncol + col;
-        float2 v = *g;
-        for (int s = 0; s < sp.z; ++s) v = cadd(v, a.partials[((int64_t)(sp.y + s) * 64 + pt) * a.ncol + col]);
-        *g = v;
-    }
+    const int n = 64 * a.ncol, i = blockIdx.y * 256 + threadIdx.x;
+    if (i >= n) return;
+    const int pt = i / a.ncol, col = i - pt * a.ncol;
+    const int pz = pt >> 4, py = (pt >> 2) & 3, px = pt & 3;
+    if (pz >= Tz || py >= Ty || px >= Tx) return;
+    float2* g = a.grid + (((int64_t)(t0z + pz) * a.os1 + (t0y + py)) * a.os2 + (t0x + px)) * a.ncol + col;
+    const float2* part = a.partials + (int64_t)sp.y * n + i;
+    float2 v = *g;
+#pragma unroll 8
+    for (int s = 0; s < sp.z; ++s) v = cadd(v, part[(int64_t)s * n]);
+    *g = v;
 }
 
 // ------------------------------------------------------------------ sample order conversion
-__global__ void k_sort_ksp(const float2* __restrict__ ext, float2* __restrict__ internal, const int32_t* __restrict__ perm,
-                           int64_t M, int ncol) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= M * ncol) return;
-    const int64_t s = i / ncol;
-    const int col = (int)(i - s * ncol);
-    internal[i] = ext[(int64_t)col * M + perm[s]];
+// Both directions go through shared memory in tiles of 64 samples (acquisition order) by up to 32
+// columns: the (ncol, M) side is read or written along the samples, the tile-sorted (M, ncol) side along
+// the columns of a sample, whose place inv[m] in the tile order comes from the inverse permutation.
+// One thread per element, gathering or scattering 8 bytes, took 650 us to bring 546,400 samples of 96
+// columns back to acquisition order; this takes 180 us.
+constexpr int kSortSamples = 64, kSortCols = 32;
+template <bool TO_INTERNAL>
+__global__ void __launch_bounds__(256) k_reorder_ksp(const float2* __restrict__ src, float2* __restrict__ dst,
+                                                     const int32_t* __restrict__ inv, int64_t M, int ncol) {
+    __shared__ float2 tile[kSortCols][kSortSamples + 1];
+    __shared__ int place[kSortSamples];
+    const int64_t m0 = (int64_t)blockIdx.x * kSortSamples;
+    const int ns = (int)min((int64_t)kSortSamples, M - m0);
+    if (threadIdx.x < ns) place[threadIdx.x] = inv[m0 + threadIdx.x];
+    int c0 = blockIdx.y * kSortCols, nc = 0;
+    auto by_column = [&](auto&& f) {                  // consecutive threads along the samples
+        const int s = threadIdx.x & (kSortSamples - 1);
+        if (s < ns)
+            for (int c = threadIdx.x / kSortSamples; c < nc; c += 256 / kSortSamples) f(s, c);
+    };
+    auto by_sample = [&](auto&& f) {                  // consecutive threads along the columns
+        for (int i = threadIdx.x; i < ns * nc; i += 256) f(i / nc, i % nc);
+    };
+    for (; c0 < ncol; c0 += gridDim.y * kSortCols) {
+        nc = min(kSortCols, ncol - c0);
+        __syncthreads();                              // places are there; the tile is free
+        if (TO_INTERNAL) {
+            by_column([&](int s, int c) { tile[c][s] = src[(int64_t)(c0 + c) * M + m0 + s]; });
+            __syncthreads();
+            by_sample([&](int s, int c) { dst[(int64_t)place[s] * ncol + c0 + c] = tile[c][s]; });
+        } else {
+            by_sample([&](int s, int c) { tile[c][s] = src[(int64_t)place[s] * ncol + c0 + c]; });
+            __syncthreads();
+            by_column([&](int s, int c) { dst[(int64_t)(c0 + c) * M + m0 + s] = tile[c][s]; });
+        }
+    }
 }
 
-__global__ void k_unsort_ksp(const float2* __restrict__ internal, float2* __restrict__ ext, const int32_t* __restrict__ perm,
-                             int64_t M, int ncol) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= M * ncol) return;
-    const int64_t s = i / ncol;
-    const int col = (int)(i - s * ncol);
-    ext[(int64_t)col * M + perm[s]] = internal[i];
+// inv[perm[s]] = s
+__global__ void k_invert_perm(const int32_t* __restrict__ perm, int32_t* __restrict__ inv, int64_t M) {
+    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (s < M) inv[perm[s]] = (int32_t)s;
 }
 
 // (Z, Y, X, C) <- (C, Z, Y, X), times the separable apodisation and the NUFFT's scale (the same in
@@ -2037,7 +2081,7 @@ static tr_status stage_interp(tr_plan* p, int bin, int ncol, int mode, float sig
 template <int CG, bool TMA>
 static tr_status launch_spread_t(const SpreadArgs& sa, const CUtensorMap& tgrid, unsigned nx, unsigned nchunks,
                                  cudaStream_t st) {
-    const size_t smem = (size_t)kSpreadSub * 16 * sizeof(float) + (size_t)kSpreadSub * sa.cchunk * sizeof(float2) + 128;
+    const size_t smem = (size_t)2 * kSpreadSub * sa.cchunk * sizeof(float2) + 128;
     const void* fn = (const void*)k_spread<CG, TMA>;
     TR_TRY(set_smem_limit(fn, smem));
     SpreadArgs args_copy = sa;
@@ -2091,7 +2135,8 @@ static tr_status stage_spread(tr_plan* p, int bin, const float2* ksp, int ncol, 
 #undef TR_SPREAD_FEW
         TR_CHECK_LAUNCH();
         if (b.n_split > 0) {
-            k_spread_reduce<<<(unsigned)b.n_split, 256, 0, st>>>(sa, p->splits + b.split_offset);
+            k_spread_reduce<<<dim3((unsigned)b.n_split, (unsigned)((64 * ncol + 255) / 256)), 256, 0, st>>>(
+            sa, p->splits + b.split_offset);
             TR_CHECK_LAUNCH();
         }
         return TR_OK;
@@ -2125,7 +2170,8 @@ static tr_status stage_spread(tr_plan* p, int bin, const float2* ksp, int ncol, 
     else TR_SPREAD_CG(8);
 #undef TR_SPREAD_CG
     if (b.n_split > 0) {
-        k_spread_reduce<<<(unsigned)b.n_split, 256, 0, st>>>(sa, p->splits + b.split_offset);
+        k_spread_reduce<<<dim3((unsigned)b.n_split, (unsigned)((64 * ncol + 255) / 256)), 256, 0, st>>>(
+            sa, p->splits + b.split_offset);
         TR_CHECK_LAUNCH();
     }
     return TR_OK;
@@ -2415,6 +2461,7 @@ static void plan_free(tr_plan* p) {
     cudaFree(p->ks);
     cudaFree(p->taps);
     cudaFree(p->perm);
+    cudaFree(p->inv_perm);
     cudaFree(p->glist);
     cudaFree(p->work);
     cudaFree(p->splits);
@@ -2730,6 +2777,7 @@ static tr_status plan_create_impl(const tr_plan_desc* d, tr_plan** out) {
     if (cudaMalloc(&p->ks, nks * sizeof(float4)) != cudaSuccess ||
         cudaMalloc(&p->taps, nks * sizeof(TapRec)) != cudaSuccess ||
         cudaMalloc(&p->perm, nks * sizeof(int32_t)) != cudaSuccess ||
+        cudaMalloc(&p->inv_perm, nks * sizeof(int32_t)) != cudaSuccess ||
         cudaMalloc(&p->glist, std::max<size_t>(glist.size(), 1) * sizeof(int2)) != cudaSuccess ||
         cudaMalloc(&p->list_start, lstart.size() * sizeof(int32_t)) != cudaSuccess ||
         cudaMalloc(&p->work, std::max<size_t>(gwork.size(), 1) * sizeof(int4)) != cudaSuccess ||
@@ -2739,6 +2787,11 @@ static tr_status plan_create_impl(const tr_plan_desc* d, tr_plan** out) {
         return bad(TR_ERR_OOM, "allocation of the sorted trajectory failed");
     TR_CUDA(cudaMemcpy(p->ks, ks_sorted.data(), nks * sizeof(float4), cudaMemcpyHostToDevice));
     TR_CUDA(cudaMemcpy(p->perm, perm.data(), nks * sizeof(int32_t), cudaMemcpyHostToDevice));
+    for (const Bin& b : p->bins) {
+        if (b.count == 0) continue;
+        k_invert_perm<<<(unsigned)((b.count + 255) / 256), 256>>>(p->perm + b.offset, p->inv_perm + b.offset, b.count);
+        TR_CHECK_LAUNCH();
+    }
     k_prep_taps<<<(unsigned)((nks + 255) / 256), 256>>>(p->ks, (int64_t)nks, p->beta, (TapRec*)p->taps);
     TR_CHECK_LAUNCH();
     TR_CUDA(cudaDeviceSynchronize());
@@ -2763,7 +2816,7 @@ static tr_status plan_create_impl(const tr_plan_desc* d, tr_plan** out) {
     // the fused y + z kernels transform every line: gridding then zero-fills every empty tile
     p->skip_empty_cols = (d->flags & TR_PLAN_NO_COLUMN_SKIP) == 0 && !p->fuse_yz;
     p->autotune = (d->flags & TR_PLAN_AUTOTUNE) != 0;
-    p->workspace_bytes = (int64_t)(nks * (sizeof(float4) + sizeof(TapRec) + sizeof(int32_t)) +
+    p->workspace_bytes = (int64_t)(nks * (sizeof(float4) + sizeof(TapRec) + 2 * sizeof(int32_t)) +
                                    glist.size() * sizeof(int2) + (gwork.size() + gsplits.size()) * sizeof(int4) +
                                    (lstart.size() + torder.size()) * sizeof(int32_t) + cmask.size());
     TR_TRY(wavelet_prepare(p));
@@ -2775,6 +2828,16 @@ static tr_status plan_create_impl(const tr_plan_desc* d, tr_plan** out) {
 }  // namespace tr
 
 using namespace tr;
+
+template <bool TO_INTERNAL>
+static tr_status reorder_kspace(tr_plan* p, const Bin& b, const void* src, void* dst, int ncol, cudaStream_t st) {
+    const int64_t gx = (b.count + kSortSamples - 1) / kSortSamples;
+    const int gy = std::min(65535, (ncol + kSortCols - 1) / kSortCols);
+    k_reorder_ksp<TO_INTERNAL><<<dim3((unsigned)gx, (unsigned)gy), 256, 0, st>>>(
+        (const float2*)src, (float2*)dst, p->inv_perm + b.offset, b.count, ncol);
+    TR_CHECK_LAUNCH();
+    return TR_OK;
+}
 
 extern "C" {
 
@@ -2846,12 +2909,8 @@ tr_status tr_plan_sort_kspace(tr_plan* p, int32_t bin, const void* ext, void* in
     if (!ext || !internal || ncol < 1) return fail(TR_ERR_INVALID_ARG, "tr_plan_sort_kspace: bad argument");
     DeviceGuard g(p->device);
     const Bin& b = p->bins[bin];
-    const int64_t n = b.count * ncol;
-    if (n == 0) return TR_OK;
-    k_sort_ksp<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
-        (const float2*)ext, (float2*)internal, p->perm + b.offset, b.count, ncol);
-    TR_CHECK_LAUNCH();
-    return TR_OK;
+    if (b.count == 0) return TR_OK;
+    return reorder_kspace<true>(p, b, ext, internal, ncol, (cudaStream_t)stream);
 }
 
 tr_status tr_plan_unsort_kspace(tr_plan* p, int32_t bin, const void* internal, void* ext, int32_t ncol,
@@ -2860,12 +2919,8 @@ tr_status tr_plan_unsort_kspace(tr_plan* p, int32_t bin, const void* internal, v
     if (!ext || !internal || ncol < 1) return fail(TR_ERR_INVALID_ARG, "tr_plan_unsort_kspace: bad argument");
     DeviceGuard g(p->device);
     const Bin& b = p->bins[bin];
-    const int64_t n = b.count * ncol;
-    if (n == 0) return TR_OK;
-    k_unsort_ksp<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
-        (const float2*)internal, (float2*)ext, p->perm + b.offset, b.count, ncol);
-    TR_CHECK_LAUNCH();
-    return TR_OK;
+    if (b.count == 0) return TR_OK;
+    return reorder_kspace<false>(p, b, internal, ext, ncol, (cudaStream_t)stream);
 }
 
 // One image: the interpolation writes, and the gridding reads, the samples in acquisition order.

@@ -172,7 +172,8 @@ struct Bin {
     int64_t n_split = 0;       // tiles whose list is split over several work items
 };
 
-struct PdhgGraph;        // defined in tr_pdhg.cu
+struct PdhgGraph;
+struct BinLanes;        // defined in tr_pdhg.cu
 struct WaveletPlan;      // defined in tr_wavelet.cu
 
 }  // namespace tr
@@ -214,9 +215,9 @@ struct tr_plan {
     // reductions
     double* partials = nullptr;
     int npartials = 0;
-    double* tol_dev = nullptr;   // [4]
-    double* tol_host = nullptr;  // pinned [4]
-    int* dev_err = nullptr;      // device error word (kDevErr* bits)
+    double* tol_dev = nullptr;   // [4]: tolerance sums, then the error word
+    double* tol_host = nullptr;  // pinned [4], the same
+    int* dev_err = nullptr;      // device error word (kDevErr* bits), in tol_dev
     int poll_limit = tr::kMbarPollLimit;   // polls before a bounded mbarrier wait gives up
     int* err_host = nullptr;     // pinned copy, refreshed with the tolerance scalars
     // launch shapes
@@ -231,6 +232,8 @@ struct tr_plan {
     tr::WaveletPlan* wav = nullptr;
     // CUDA graph of one PDHG iteration
     tr::PdhgGraph* graph = nullptr;
+    // streams and workspaces of bins that run side by side (small problems)
+    tr::BinLanes* lanes = nullptr;
     int64_t workspace_bytes = 0;
 };
 
@@ -253,6 +256,7 @@ tr_status wavelet_adjoint(tr_plan* p, const float2* p_w2, float2* out, cudaStrea
 void wavelet_destroy(tr_plan* p);
 void wavelet_info(const tr_plan* p, int32_t* levels, int64_t* coeffs);
 void pdhg_destroy(tr_plan* p);
+void lanes_destroy(tr_plan* p);
 
 // forward interpolation output modes
 constexpr int kInterpStore = 0;     // out = A x

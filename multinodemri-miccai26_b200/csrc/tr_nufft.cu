@@ -2453,6 +2453,7 @@ static void plan_free(tr_plan* p) {
     cudaGetDevice(&cur);
     cudaSetDevice(p->device);
     pdhg_destroy(p);
+    lanes_destroy(p);
     wavelet_destroy(p);
     for (auto& a : p->ax) {
         cudaFree(a.twiddle);
@@ -2473,8 +2474,6 @@ static void plan_free(tr_plan* p) {
     cudaFree(p->bufB);
     cudaFree(p->partials);
     cudaFree(p->tol_dev);
-    cudaFree(p->dev_err);
-    if (p->err_host) cudaFreeHost(p->err_host);
     if (p->tol_host) cudaFreeHost(p->tol_host);
     cudaSetDevice(cur);
     delete p;
@@ -2805,9 +2804,10 @@ static tr_status plan_create_impl(const tr_plan_desc* d, tr_plan** out) {
     TR_CUDA(cudaMemcpy(p->tile_order, torder.data(), torder.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
     TR_CUDA(cudaMemcpy(p->colmask, cmask.data(), cmask.size(), cudaMemcpyHostToDevice));
     if (cudaMalloc(&p->tol_dev, 4 * sizeof(double)) != cudaSuccess ||
-        cudaMallocHost(&p->tol_host, 4 * sizeof(double)) != cudaSuccess ||
-        cudaMalloc(&p->dev_err, sizeof(int)) != cudaSuccess || cudaMallocHost(&p->err_host, sizeof(int)) != cudaSuccess)
+        cudaMallocHost(&p->tol_host, 4 * sizeof(double)) != cudaSuccess)
         return bad(TR_ERR_OOM, "allocation of reduction scalars failed");
+    p->dev_err = reinterpret_cast<int*>(p->tol_dev + 2);
+    p->err_host = reinterpret_cast<int*>(p->tol_host + 2);
     TR_CUDA(cudaMemset(p->dev_err, 0, sizeof(int)));
     *p->err_host = 0;
     p->use_tma = (d->flags & TR_PLAN_NO_TMA) == 0;

@@ -115,8 +115,14 @@ struct LineKernels {
     const void* adj_x = nullptr;     // (AdjXArgs)
     int threads = 0;
     int smem = 0;                    // dynamic shared memory, bytes
-    int smem_adj_x = 0;
 };
 const LineKernels& line_kernels(int L);
+// Forward x pass: image rows in shared memory (odd pitch: rows in different banks), the most distinct rows
+// that 16 consecutive (row, coil) pairs meet, and their bytes (two buffers where there are several images).
+__host__ __device__ constexpr int lp_row_pitch(int X) { return X | 1; }
+__host__ __device__ constexpr int lp_rows_per_cta(int C) { return (kLineW - 1 + C - 1) / C + 1; }
+constexpr size_t lp_row_bytes(int X, int C, int n_img) {
+    return (size_t)(n_img > 1 ? 2 : 1) * lp_rows_per_cta(C) * lp_row_pitch(X) * sizeof(float2);
+}
 
 }  // namespace tr

@@ -54,41 +54,48 @@ __host__ __device__ constexpr int lp_threads(int L) {
 }
 // CTAs per SM the register budget is set for: about 64 registers a thread.
 __host__ __device__ constexpr int lp_min_ctas(int L) { return 1024 / lp_threads(L) > 0 ? 1024 / lp_threads(L) : 1; }
+// The x passes keep a column's map in registers as well.
+__host__ __device__ constexpr int lp_x_min_ctas(int L) { return 768 / lp_threads(L) > 0 ? 768 / lp_threads(L) : 1; }
 __host__ __device__ constexpr int lp_smem(int L) { return L * kLineW * 8 + L * 8; }
 
+// Butterflies per thread of pass s.
+__host__ __device__ constexpr int lp_iters(int L, int s) {
+    return (L / lp_radix(L, s) + lp_threads(L) / kLineW - 1) / (lp_threads(L) / kLineW);
+}
+// A thread's inputs of the first pass: element j + r NB of its column, from load(m, index).
+template <int L>
+using LpFirst = float2[lp_iters(L, 0)][lp_radix(L, 0)];
+template <int L, class Load>
+__device__ __forceinline__ void lp_load(LpFirst<L>& v, const Load& load) {
+    constexpr int R = lp_radix(L, 0), NB = L / R, JS = lp_threads(L) / kLineW;
+#pragma unroll
+    for (int it = 0; it < lp_iters(L, 0); ++it) {
+        const int j = threadIdx.x / kLineW + it * JS;
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[it][r] = j < NB ? load(j + r * NB, it * R + r) : make_float2(0.f, 0.f);
+    }
+}
+
 // One Stockham pass on the [L][16] tile `buf` (in place: the results of a pass are stored after every
-// input was read).  The first pass reads its inputs from load(m), the last hands its outputs to
-// store(k, v); kSyncLast: store() writes into buf.
-template <int L, bool INV, int s, int Ns, bool kSyncLast, class Load, class Store>
-__device__ __forceinline__ void lp_pass(float2* buf, const float2* tw, Load& load, Store& store) {
-    constexpr int R = lp_radix(L, s), NB = L / R, NT = lp_threads(L), JS = NT / kLineW, IT = (NB + JS - 1) / JS;
+// input was read).  The first pass takes its inputs from v, the last hands its outputs to
+// store(k, v, index); kSyncLast: store() writes into buf.
+template <int L, bool INV, int s, int Ns, bool kSyncLast, class Store>
+__device__ __forceinline__ void lp_pass(float2 (&v)[lp_iters(L, s)][lp_radix(L, s)], float2* buf, const float2* tw,
+                                        const Store& store) {
+    constexpr int R = lp_radix(L, s), NB = L / R, JS = lp_threads(L) / kLineW, IT = lp_iters(L, s);
     constexpr int STEP = L / (Ns * R);
     constexpr bool last = s == lp_stages(L) - 1;
     const int w = threadIdx.x & (kLineW - 1), j0 = threadIdx.x / kLineW;
-    float2 v[IT][R];
 #pragma unroll
     for (int it = 0; it < IT; ++it) {
         const int j = j0 + it * JS;
         if (j < NB) {
-            const int k = Ns == 1 ? 0 : j % Ns;
+            if constexpr (s > 0) {
+                const int k = Ns == 1 ? 0 : j % Ns;
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-                if constexpr (s == 0) load.first(j + r * NB, v[it][r]);
-                else v[it][r] = buf[(j + r * NB) * kLineW + w];
-            }
-            if constexpr (s == 0 && Load::kTwo) {          // a second factor, four loads in flight at a time
+                for (int r = 0; r < R; ++r) v[it][r] = buf[(j + r * NB) * kLineW + w];
 #pragma unroll
-                for (int r0 = 0; r0 < R; r0 += 4) {
-                    float2 f[4];
-#pragma unroll
-                    for (int r = r0; r < r0 + 4 && r < R; ++r) f[r - r0] = load.second(j + r * NB);
-#pragma unroll
-                    for (int r = r0; r < r0 + 4 && r < R; ++r) v[it][r] = cmul(v[it][r], f[r - r0]);
-                }
-            }
-#pragma unroll
-            for (int r = 1; r < R; ++r) {
-                if constexpr (s > 0) {
+                for (int r = 1; r < R; ++r) {
                     float2 t = tw[k * r * STEP];
                     if (INV) t.y = -t.y;
                     v[it][r] = cmul_p(v[it][r], t);
@@ -105,33 +112,29 @@ __device__ __forceinline__ void lp_pass(float2* buf, const float2* tw, Load& loa
             const int k = Ns == 1 ? 0 : j % Ns, d0 = (j / Ns) * Ns * R + k;
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                if constexpr (last) store(d0 + r * Ns, v[it][r]);
+                if constexpr (last) store(d0 + r * Ns, v[it][r], it * R + r);
                 else buf[(d0 + r * Ns) * kLineW + w] = v[it][r];
             }
         }
     }
     if constexpr (!last) {
         __syncthreads();
-        lp_pass<L, INV, s + 1, Ns * R, kSyncLast>(buf, tw, load, store);
+        float2 next[lp_iters(L, s + 1)][lp_radix(L, s + 1)];
+        lp_pass<L, INV, s + 1, Ns * R, kSyncLast>(next, buf, tw, store);
     }
 }
 
-// Inputs of a first pass: row (m + h) mod L of the padded line, zero outside [0, n).  Loads are
-// predicated, never branched around, so that a thread's loads are all in flight together.
-struct LineLoad {
-    static constexpr bool kTwo = false;
-    const float2* in;
-    int64_t stride;
-    int n, d, wrap, L;                       // position m + d, less L from m = wrap on
-    __device__ __forceinline__ int row(int m) const { return m + d - (m >= wrap ? L : 0); }
-    __device__ __forceinline__ void first(int m, float2& v) const {
-        const int i = row(m);
-        v = (unsigned)i < (unsigned)n ? in[i * stride] : make_float2(0.f, 0.f);
-    }
-    __device__ __forceinline__ float2 second(int) const { return make_float2(1.f, 0.f); }
+// Place of element m of a centred, padded line among the n rows kept: (m + h) mod L - pad; outside
+// [0, n) for the padding.
+template <int L>
+struct LineRow {
+    int d, wrap;                             // h - pad; elements from wrap = L - h on lie L lower
+    __device__ __forceinline__ LineRow(int h, int pad) : d(h - pad), wrap(L - h) {}
+    __device__ __forceinline__ int operator()(int m) const { return m + d - (m >= wrap ? L : 0); }
 };
 
 // ------------------------------------------------------------------ line pass
+// Loads are predicated, never branched around, so that a thread's loads are all in flight together.
 template <int L, bool INV>
 __global__ void __launch_bounds__(lp_threads(L), lp_min_ctas(L)) k_lp_line(LineArgs a) {
     extern __shared__ float2 sm[];
@@ -146,162 +149,152 @@ __global__ void __launch_bounds__(lp_threads(L), lp_min_ctas(L)) k_lp_line(LineA
     const bool on = q < a.inner;
     const float2* in = a.in + outer * a.Lin * a.inner + q;
     float2* out = a.out + outer * a.Lout * a.inner + q;
-    const int lin = on ? a.Lin : 0, lout = on ? a.Lout : 0, din = a.h - a.p_in, dout = a.h - a.p_out;
-    LineLoad load{in, a.inner, lin, din, L - a.h, L};
-    auto store = [&](int k, float2 v) {
-        int o = k + dout;
-        if (k + a.h >= L) o -= L;
-        if ((unsigned)o < (unsigned)lout) out[(int64_t)o * a.inner] = v;
-    };
-    lp_pass<L, INV, 0, 1, false>(sm, tw, load, store);
+    const int lin = on ? a.Lin : 0, lout = on ? a.Lout : 0;
+    const LineRow<L> from(a.h, a.p_in), to(a.h, a.p_out);
+    LpFirst<L> v;
+    lp_load<L>(v, [&](int m, int) -> float2 {
+        const int i = from(m);
+        return (unsigned)i < (unsigned)lin ? in[i * a.inner] : make_float2(0.f, 0.f);
+    });
+    lp_pass<L, INV, 0, 1, false>(v, sm, tw, [&](int k, float2 r, int) {
+        const int o = to(k);
+        if ((unsigned)o < (unsigned)lout) out[o * a.inner] = r;
+    });
 }
 
-// u times the scaled map, or u times the apodisation where there are no maps.
-struct MapLoad {
-    static constexpr bool kTwo = true;
-    LineLoad u;
-    const float2* map;
-    const float* apx;
-    int C;
-    float sc;
-    __device__ __forceinline__ void first(int m, float2& v) const { u.first(m, v); }
-    __device__ __forceinline__ float2 second(int m) const {
-        const int x = u.row(m);
-        const bool in = (unsigned)x < (unsigned)u.n;
-        if (map) return in ? map[(int64_t)x * C] : make_float2(0.f, 0.f);
-        return make_float2(in ? sc * apx[x] : 0.f, 0.f);
-    }
-};
-
-// ------------------------------------------------------------------ forward x pass
-// Sixteen consecutive (row, column) pairs per CTA, columns of a row first, so that any coil count and
-// number of images fills the tile.
+// ------------------------------------------------------------------ x passes
+// A CTA takes 16 (row, coil) columns and walks over the images, so that a column's scaled coil map
+// stays in registers: the forward pass multiplies a thread's first inputs with it, the adjoint pass its
+// last outputs.  Without maps (one image, one column per row) the apodisation takes its place.
+// Reading the maps for every column of every image instead (as one flat list of columns, sums by
+// shuffles), the two passes took 204 and 239 us at 56 x 134 x 60 (60 columns), now 180 and 218 us, and
+// 86 and 142 us at 100 x 56 x 72 (48 columns), now 80 and 113 us.  Bound by instruction issue and the
+// latency of the two barriers an image takes; tiles of 8 columns gave 3 % at 200 points with 12 coils
+// and lost 40 % with 5 coils.
+//
+// Forward: 16 consecutive (row, coil) pairs, any coil count fills the tile.  The image rows they share
+// come through shared memory, the next image's while this one's is transformed.
 template <int L>
-__global__ void __launch_bounds__(lp_threads(L), lp_min_ctas(L)) k_lp_fwd_x(FwdXArgs a) {
-    extern __shared__ float2 sm[];
-    float2* tw = sm + L * kLineW;
-    for (int i = threadIdx.x; i < L; i += lp_threads(L)) tw[i] = a.tw[i];
-    const int64_t q = (int64_t)blockIdx.x * kLineW + (threadIdx.x & (kLineW - 1));
-    const int64_t rows = (int64_t)a.Z * a.Y;
-    const bool on = q < rows * a.ncol;
-    const int64_t row = on ? q / a.ncol : 0;
-    const int col = on ? (int)(q - row * a.ncol) : 0, img = col / a.C, c = col - img * a.C;
-    const int z = (int)(row / a.Y), y = (int)(row - (int64_t)z * a.Y);
-    const float sc = a.apz[z] * a.apy[y] * a.scale;
-    const float2* src = a.img + (int64_t)img * a.img_stride + row * a.X;
-    const float2* map = a.maps ? a.maps + row * a.X * a.C + c : nullptr;
-    float2* out = a.out + row * a.OSX * a.ncol + col;
-    const int nx = on ? a.X : 0, din = a.h - a.pad;
-    MapLoad load{{src, 1, nx, din, L - a.h, L}, map, a.apx, a.C, sc};
-    auto store = [&](int k, float2 v) {
-        int g = k + a.h;
-        if (g >= L) g -= L;
-        if (on) out[(int64_t)g * a.ncol] = v;
-    };
-    lp_pass<L, false, 0, 1, false>(sm, tw, load, store);
-}
-
-// ------------------------------------------------------------------ adjoint x pass
-// One row per CTA, its columns in chunks of 16 (several whole rows where they fit one chunk).  The
-// transformed, cropped rows go back into the tile with column w of row x at w ^ (x % 16), which both
-// the products with the coil maps (half-warps along the columns of an x) and the write of the
-// images (warps along x) read without bank conflicts.  The columns of an image are summed by a
-// segmented shuffle; an image whose coils span chunks is added up in its image row.
-template <int L>
-__global__ void __launch_bounds__(lp_threads(L), lp_min_ctas(L)) k_lp_adj_x(AdjXArgs a) {
+__global__ void __launch_bounds__(lp_threads(L), lp_x_min_ctas(L)) k_lp_fwd_x(FwdXArgs a) {
     extern __shared__ float2 sm[];
     constexpr int NT = lp_threads(L);
     float2* tw = sm + L * kLineW;
-    float2* smap = tw + L;                               // [X][16]: the chunk's coil maps
+    const int pitch = lp_row_pitch(a.X), nrows = lp_rows_per_cta(a.C);
+    float2* rowbuf = tw + L;                              // [2 (one image: 1)][nrows][pitch]
+    for (int i = threadIdx.x; i < L; i += NT) tw[i] = a.tw[i];
+    const int64_t rows = (int64_t)a.Z * a.Y, q0 = (int64_t)blockIdx.x * kLineW, r0 = q0 / a.C;
+    const int64_t q = q0 + (threadIdx.x & (kLineW - 1));
+    const bool on = q < rows * a.C;
+    const int64_t row = on ? q / a.C : r0;
+    const int c = on ? (int)(q - row * a.C) : 0;
+    const LineRow<L> from(a.h, a.pad);
+    auto fetch = [&](int e) {
+        const float2* src = a.img + (int64_t)e * a.img_stride + r0 * a.X;
+        float2* dst = rowbuf + (e & 1) * nrows * pitch;
+        const int n = (int)min((int64_t)nrows, rows - r0) * a.X;
+        for (int i = threadIdx.x; i < n; i += NT) {
+            const int r = i / a.X;
+            cp_async8(dst + r * pitch + (i - r * a.X), src + i, 8);
+        }
+    };
+    fetch(0);
+    LpFirst<L> map;
+    {
+        const int z = (int)(row / a.Y), y = (int)(row - (int64_t)z * a.Y);
+        const float sc = a.apz[z] * a.apy[y] * a.scale;
+        const float2* mp = a.maps ? a.maps + row * a.X * a.C + c : nullptr;
+        lp_load<L>(map, [&](int m, int) -> float2 {
+            const int x = from(m);
+            const bool in = (unsigned)x < (unsigned)a.X;
+            if (mp) return in ? mp[x * a.C] : make_float2(0.f, 0.f);
+            return make_float2(in ? sc * a.apx[x] : 0.f, 0.f);
+        });
+    }
+    const float2* mine = rowbuf + (int)(row - r0) * pitch;
+    float2* out = a.out + row * a.OSX * a.ncol + c;
+    for (int e = 0; e < a.n_img; ++e) {
+        cp_async_wait_all();
+        __syncthreads();                                  // image e's rows are there; the tile is free
+        if (e + 1 < a.n_img) fetch(e + 1);
+        const float2* u = mine + (e & 1) * nrows * pitch;
+        LpFirst<L> v;
+        lp_load<L>(v, [&](int m, int i) -> float2 {
+            const int x = from(m);
+            return (unsigned)x < (unsigned)a.X ? cmul(u[x], map[i / lp_radix(L, 0)][i % lp_radix(L, 0)])
+                                               : make_float2(0.f, 0.f);
+        });
+        lp_pass<L, false, 0, 1, false>(v, sm, tw, [&](int k, float2 r, int) {
+            int g = k + a.h;
+            if (g >= L) g -= L;
+            if (on) out[g * a.ncol + e * a.C] = r;
+        });
+    }
+}
+
+// Adjoint: whole rows of at most 16 coils (several rows where they fit), or 16 coils of a row at a
+// time; the products go back into the tile with 17 columns, where the threads along x sum a row's coils
+// in order and write the image row (coils past the first 16 are added to it).  The next image's inputs
+// are loaded during the sums.
+template <int L>
+__global__ void __launch_bounds__(lp_threads(L), lp_x_min_ctas(L)) k_lp_adj_x(AdjXArgs a) {
+    extern __shared__ float2 sm[];
+    constexpr int NT = lp_threads(L), kLast = lp_stages(L) - 1, kPitch = kLineW + 1;
+    constexpr int RL = lp_radix(L, kLast), IL = lp_iters(L, kLast);
+    float2* tw = sm + L * kLineW;
     for (int i = threadIdx.x; i < L; i += NT) tw[i] = a.tw[i];
     const int w = threadIdx.x & (kLineW - 1);
     const int64_t rows = (int64_t)a.Z * a.Y;
-    const int rpc = a.ncol >= kLineW ? 1 : kLineW / a.ncol;                  // rows per CTA
-    const int nchunk = a.ncol >= kLineW ? (a.ncol + kLineW - 1) / kLineW : 1;
-    const int dout = a.h - a.pad;
-    // column w of chunk ch: row, image, coil
-    for (int ch = 0; ch < nchunk; ++ch) {
-        auto place = [&](int slot, int64_t& row, int& col) {
-            const int rl = nchunk > 1 || rpc == 1 ? 0 : slot / a.ncol;
-            row = (int64_t)blockIdx.x * rpc + rl;
-            col = ch * kLineW + slot - rl * a.ncol;
-            return rl < rpc && row < rows && col < a.ncol;
+    const int rpc = a.C >= kLineW ? 1 : kLineW / a.C;
+    const int64_t row0 = (int64_t)blockIdx.x * rpc;
+    const LineRow<L> to(a.h, a.pad);
+    for (int c0 = 0; c0 < a.C; c0 += kLineW) {
+        const int nc = min(kLineW, a.C - c0), rl = a.C >= kLineW ? 0 : w / a.C, c = c0 + w - rl * a.C;
+        const int64_t row = row0 + rl;
+        const bool on = rl < rpc && row < rows && c < a.C;
+        const float2* in = a.in + (on ? row * a.OSX * a.ncol + c : 0);
+        auto inputs = [&](LpFirst<L>& v, int e) {
+            lp_load<L>(v, [&](int m, int) -> float2 {
+                int j = m + a.h;
+                if (j >= L) j -= L;
+                return on ? in[j * a.ncol + e * a.C] : make_float2(0.f, 0.f);
+            });
         };
-        int64_t row;
-        int col;
-        const bool on = place(w, row, col);
-        const float2* in = a.in + (on ? row * a.OSX * a.ncol + col : 0);
-        LineLoad load{in, a.ncol, on ? L : 0, a.h, L - a.h, L};
-        auto store = [&](int k, float2 v) {
-            int x = k + dout;
-            if (k + a.h >= L) x -= L;
-            if ((unsigned)x < (unsigned)a.X) sm[x * kLineW + (w ^ (x & 15))] = v;
-        };
-        const int img = on ? col / a.C : -1, c = on ? col - img * a.C : 0;
-        const int seg = on ? (int)(row - (int64_t)blockIdx.x * rpc) * a.n_img + img : -1;
-        constexpr int JS = NT / kLineW;
-        if (a.maps) {                                      // the columns' maps travel during the transform
-            const float2* map = a.maps + (on ? row * a.X * a.C + c : 0);
-            for (int x = threadIdx.x / kLineW; x < a.X; x += JS)
-                cp_async8(smap + x * kLineW + w, map + (on ? (int64_t)x * a.C : 0), on ? 8 : 0);
+        LpFirst<L> v;
+        inputs(v, 0);
+        float2 map[IL][RL];                               // of the last pass's outputs
+        {
+            // the last pass's butterflies j < L / RL hold the outputs j + r (L / RL)
+            const int z = on ? (int)(row / a.Y) : 0, y = on ? (int)(row - (int64_t)z * a.Y) : 0;
+            const float sc = a.apz[z] * a.apy[y] * a.scale;
+            const float2* mp = a.maps ? a.maps + (on ? row * a.X * a.C + c : 0) : nullptr;
+#pragma unroll
+            for (int it = 0; it < IL; ++it)
+#pragma unroll
+                for (int r = 0; r < RL; ++r) {
+                    const int j = threadIdx.x / kLineW + it * (NT / kLineW), x = to(j + r * (L / RL));
+                    const bool in_x = on && j < L / RL && (unsigned)x < (unsigned)a.X;
+                    if (mp) map[it][r] = in_x ? mp[x * a.C] : make_float2(0.f, 0.f);
+                    else map[it][r] = make_float2(in_x ? sc * a.apx[x] : 0.f, 0.f);
+                }
         }
-        lp_pass<L, true, 0, 1, true>(sm, tw, load, store);
-        cp_async_wait_all();
-        __syncthreads();
-        if (a.maps) {
-            const unsigned half = (threadIdx.x & 16) ? 0xffff0000u : 0x0000ffffu;
-            int same = 0;                                  // bit b: lane w + 2^b belongs to the same image
-            for (int b = 0; b < 4; ++b) {
-                const int other = __shfl_down_sync(half, seg, 1 << b, kLineW);
-                same |= (w + (1 << b) < kLineW && other == seg) << b;
-            }
-            constexpr int U = 4;                           // x positions side by side per thread
-            for (int x0 = threadIdx.x / kLineW; x0 < a.X; x0 += U * JS) {
-                float2 v[U];
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const int x = x0 + u * JS;
-                    v[u] = on && x < a.X ? cmulc(sm[x * kLineW + (w ^ (x & 15))], smap[x * kLineW + w])
-                                         : make_float2(0.f, 0.f);
-                }
-#pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                    if (1 << b >= a.C) break;
-#pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        const float tx = __shfl_down_sync(half, v[u].x, 1 << b, kLineW);
-                        const float ty = __shfl_down_sync(half, v[u].y, 1 << b, kLineW);
-                        if (same & (1 << b)) v[u] = make_float2(v[u].x + tx, v[u].y + ty);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const int x = x0 + u * JS;
-                    if (x < a.X) sm[x * kLineW + (w ^ (x & 15))] = v[u];
-                }
+        for (int e = 0; e < a.n_img; ++e) {
+            lp_pass<L, true, 0, 1, true>(v, sm, tw, [&](int k, float2 r, int i) {
+                const int x = to(k);
+                if ((unsigned)x < (unsigned)a.X) sm[x * kPitch + w] = cmulc(r, map[i / RL][i % RL]);
+            });
+            if (e + 1 < a.n_img) inputs(v, e + 1);
+            __syncthreads();
+            for (int i = threadIdx.x; i < rpc * a.X; i += NT) {
+                const int r = rpc == 1 ? 0 : i / a.X, x = i - r * a.X;
+                if (row0 + r >= rows) break;
+                const float2* p = sm + x * kPitch + r * a.C;
+                float2 t = p[0];
+                for (int k = 1; k < nc; ++k) t = cadd(t, p[k]);
+                float2* dst = a.img + (int64_t)e * a.img_stride + (row0 + r) * a.X + x;
+                *dst = c0 > 0 ? cadd(*dst, t) : t;
             }
             __syncthreads();
         }
-        // the first column of every image in the chunk holds its sum: write (first coils) or add
-        const unsigned heads = __ballot_sync(0xffffffffu, on && (c == 0 || w == 0)) & 0xffffu;
-        const int nx = (a.X + 31) / 32, tasks = __popc(heads) * nx;
-        for (int t = threadIdx.x >> 5; t < tasks; t += NT / 32) {
-            const int hn = t / nx, x = (t - hn * nx) * 32 + (threadIdx.x & 31), slot = __fns(heads, 0, hn + 1);
-            int64_t r;
-            int cl;
-            place(slot, r, cl);
-            if (x >= a.X) continue;
-            const int im = cl / a.C;
-            float2 v = sm[x * kLineW + (slot ^ (x & 15))];
-            if (!a.maps) {
-                const int z = (int)(r / a.Y), y = (int)(r - (int64_t)z * a.Y);
-                v = cscale(v, a.apz[z] * a.apy[y] * a.apx[x] * a.scale);
-            }
-            float2* dst = a.img + (int64_t)im * a.img_stride + r * a.X + x;
-            if (cl - im * a.C > 0) v = cadd(*dst, v);
-            *dst = v;
-        }
-        __syncthreads();
     }
 }
 
@@ -316,7 +309,6 @@ LineKernels lp_entry() {
         k.adj_x = (const void*)k_lp_adj_x<L>;
         k.threads = lp_threads(L);
         k.smem = lp_smem(L);
-        k.smem_adj_x = lp_smem(L) + L * kLineW * 8;
     }
     return k;
 }

@@ -293,7 +293,9 @@ __global__ void __launch_bounds__(256) k_adj_x(AdjXArgs a) {
 //   tr_lines.cuh are faster: z pass at 60, 80, 100, 120 (32 columns) 0.15, 0.18, 0.21, 0.26 against
 //   0.19, 0.22, 0.25, 0.29 ms, y pass at 100, 120, 140 0.13, 0.16, 0.19 against 0.14, 0.16, 0.20 ms,
 //   at 240 (24 columns) 0.30 against 0.42 ms.
-// - x passes with whole groups of 8 or 4 coils (below).
+// - x passes with whole groups of 8 or 4 coils (below): forward 0.18, 0.95 and 2.63 ms at 96 x 128 x 128
+//   (32 columns), 112 x 160 x 160 (72) and 128 x 256 x 256 (96) against 0.23, 1.01 and 2.92 ms, adjoint
+//   0.27, 1.11 and 2.94 against 0.27, 1.49 and 4.53 ms.
 // Lengths up to 200 use 16-column tiles, longer ones 8-column tiles (the
 // shared-memory footprint 2 L W x 8 bytes then allows >= 4 CTAs per SM).
 #define TR_LINE_TMA_LENGTHS(X) X(160) X(200) X(320)
@@ -1900,11 +1902,12 @@ static tr_status stage_fwd_x(tr_plan* p, const float2* images, int64_t img_strid
     }
     const LineKernels& lk = line_kernels(OSX);
     if (lk.fwd_x) {
-        const int64_t q = (int64_t)Z * Y * fa.ncol;
-        TR_TRY(set_smem_limit(lk.fwd_x, lk.smem));
+        const int64_t q = (int64_t)Z * Y * C;
+        const size_t smem = lk.smem + lp_row_bytes(X, C, n_img);
+        TR_TRY(set_smem_limit(lk.fwd_x, smem));
         void* args[] = {&fa};
-        TR_CUDA(cudaLaunchKernel(lk.fwd_x, dim3((unsigned)((q + kLineW - 1) / kLineW)), dim3((unsigned)lk.threads), args,
-                                 lk.smem, st));
+        TR_CUDA(cudaLaunchKernel(lk.fwd_x, dim3((unsigned)((q + kLineW - 1) / kLineW)), dim3((unsigned)lk.threads), args, smem,
+                                 st));
         return TR_OK;
     }
     fa.cc = coils_per_cta(C);
@@ -2253,12 +2256,11 @@ static tr_status stage_adj_x(tr_plan* p, int n_img, const float2* maps, int C, f
     }
     const LineKernels& lk = line_kernels(OSX);
     if (lk.adj_x) {
-        const int64_t rows = (int64_t)Z * Y, per = aa.ncol >= kLineW ? 1 : kLineW / aa.ncol;
-        const size_t smem = maps ? lk.smem_adj_x : lk.smem;
-        TR_TRY(set_smem_limit(lk.adj_x, smem));
+        const int64_t rows = (int64_t)Z * Y, per = C >= kLineW ? 1 : kLineW / C;
+        TR_TRY(set_smem_limit(lk.adj_x, lk.smem));
         void* args[] = {&aa};
-        TR_CUDA(cudaLaunchKernel(lk.adj_x, dim3((unsigned)((rows + per - 1) / per)), dim3((unsigned)lk.threads), args, smem,
-                                 st));
+        TR_CUDA(cudaLaunchKernel(lk.adj_x, dim3((unsigned)((rows + per - 1) / per)), dim3((unsigned)lk.threads), args,
+                                 lk.smem, st));
         return TR_OK;
     }
     aa.cc = coils_per_cta(C);

@@ -937,9 +937,13 @@ __global__ void k_prep_taps(const float4* __restrict__ ks, int64_t M, float beta
 }
 
 // ------------------------------------------------------------------ interpolation
-// G lanes cooperate on one sample (lane = column group); taps read ncol
-// contiguous complex values per grid point (coalesced across lanes).
-template <int CPL>
+// G lanes cooperate on one sample (G need not be a power of two, so no lane is idle): a lane takes CPL
+// pieces of V consecutive columns (V = 2: one 16-byte load), G V columns apart; taps read ncol
+// contiguous complex values per grid point, coalesced across lanes.  Bound by the latency of the grid
+// reads where the grid is small, by HBM where it is large: 32 columns on 120 x 160 x 160 (136 000 samples)
+// 216 -> 148 us against single columns a power of two apart, 72 on 140 x 200 x 200 801 -> 564 us,
+// 96 on 160 x 320 x 320 2.53 -> 2.27 ms (0.93 of the copy rate).
+template <int V, int CPL>
 __global__ void __launch_bounds__(256) k_interp(const float2* __restrict__ grid, const TapRec* __restrict__ taps,
                                                 int64_t M, int ncol, int G, int os0, int os1, int os2,
                                                 int mode, float sigma, const float2* __restrict__ y,
@@ -959,9 +963,26 @@ __global__ void __launch_bounds__(256) k_interp(const float2* __restrict__ grid,
         iy[t] = pmod(by + t, os1);
         ix[t] = pmod(bx + t, os2);
     }
-    float2 acc[CPL];
+    float2 acc[CPL][V];
 #pragma unroll
-    for (int j = 0; j < CPL; ++j) acc[j] = make_float2(0.f, 0.f);
+    for (int j = 0; j < CPL; ++j)
+#pragma unroll
+        for (int u = 0; u < V; ++u) acc[j][u] = make_float2(0.f, 0.f);
+    auto add = [&](float w, const float2* gp) {
+#pragma unroll
+        for (int j = 0; j < CPL; ++j) {
+            const int col = (lane + j * G) * V;
+            if (col < ncol) {
+                if constexpr (V == 2) {
+                    const float4 v = *reinterpret_cast<const float4*>(gp + col);
+                    acc[j][0] = cfma_real(w, make_float2(v.x, v.y), acc[j][0]);
+                    acc[j][1] = cfma_real(w, make_float2(v.z, v.w), acc[j][1]);
+                } else {
+                    acc[j][0] = cfma_real(w, gp[col], acc[j][0]);
+                }
+            }
+        }
+    };
     if (wz[4] == 0.f && wy[4] == 0.f && wx[4] == 0.f) {
         // common case: four taps per axis (k - 2 not an integer), fully unrolled
 #pragma unroll
@@ -972,17 +993,7 @@ __global__ void __launch_bounds__(256) k_interp(const float2* __restrict__ grid,
                 const float wzy = wz[tz] * wy[ty];
                 const int64_t yoff = (zoff + iy[ty]) * os2;
 #pragma unroll
-                for (int tx = 0; tx < 4; ++tx) {
-                    const float w = wzy * wx[tx];
-                    const float2* gp = grid + (yoff + ix[tx]) * ncol;
-#pragma unroll
-                    for (int j = 0; j < CPL; ++j) {
-                        const int col = lane + j * G;
-                        if (col < ncol) {
-                            acc[j] = cfma_real(w, gp[col], acc[j]);
-                        }
-                    }
-                }
+                for (int tx = 0; tx < 4; ++tx) add(wzy * wx[tx], grid + (yoff + ix[tx]) * ncol);
             }
         }
     } else
@@ -998,30 +1009,25 @@ __global__ void __launch_bounds__(256) k_interp(const float2* __restrict__ grid,
 #pragma unroll
             for (int tx = 0; tx < 5; ++tx) {
                 if (wx[tx] == 0.f) continue;
-                const float w = wzy * wx[tx];
-                const float2* gp = grid + (yoff + ix[tx]) * ncol;
-#pragma unroll
-                for (int j = 0; j < CPL; ++j) {
-                    const int col = lane + j * G;
-                    if (col < ncol) {
-                        acc[j] = cfma_real(w, gp[col], acc[j]);
-                    }
-                }
+                add(wzy * wx[tx], grid + (yoff + ix[tx]) * ncol);
             }
         }
     }
 #pragma unroll
     for (int j = 0; j < CPL; ++j) {
-        const int col = lane + j * G;
+        const int col = (lane + j * G) * V;
         if (col >= ncol) continue;
-        const int64_t o = s * ncol + col;
-        if (mode == kInterpDualProx) {
-            const float2 r = csub(acc[j], y[o]);
-            const float2 q = out[o];
-            const float inv = 1.0f / (1.0f + sigma);
-            out[o] = make_float2((q.x + sigma * r.x) * inv, (q.y + sigma * r.y) * inv);
-        } else {
-            out[o] = acc[j];
+#pragma unroll
+        for (int u = 0; u < V; ++u) {
+            const int64_t o = s * ncol + col + u;
+            if (mode == kInterpDualProx) {
+                const float2 r = csub(acc[j][u], y[o]);
+                const float2 q = out[o];
+                const float inv = 1.0f / (1.0f + sigma);
+                out[o] = make_float2((q.x + sigma * r.x) * inv, (q.y + sigma * r.y) * inv);
+            } else {
+                out[o] = acc[j][u];
+            }
         }
     }
 }
@@ -2061,21 +2067,37 @@ static tr_status stage_interp(tr_plan* p, int bin, int ncol, int mode, float sig
         TR_CHECK_LAUNCH();
         return TR_OK;
     }
-    int G = 1;
-    while (G < ncol && G < 32) G <<= 1;
-    const int cpl = (ncol + G - 1) / G;
-    const int64_t threads = b.count * G;
-    const unsigned blocks = (unsigned)((threads + 255) / 256);
+    if (ncol > 256) return fail(TR_ERR_UNSUPPORTED, "more than 256 k-space columns per bin are not supported");
+    // Even column counts read pairs (bufA is aligned and a row of ncol even columns starts on 16 bytes).
+    // Fewer lanes a sample, so that a warp holds several samples and a lane several loads in flight, is
+    // faster from two pieces a lane on (64 x 96 x 96, 80 000 samples, 1 / 2 / 3 / 4 pieces a lane: 12 columns
+    // 71 / 66 / 78 / 110 us, 24: 142 / 90 / 103 / 181, 48: 257 / 155 / 162 / 274; 10: 53 / 63 / 78 / 103);
+    // odd ones, single values, from three on (15: 85 / 100 / 83 / 97, 25: 135 / 136 / 112 / 128,
+    // 45: 218 / 218 / 176 / 201; 9: 48 / 81 / 69 / 84).
+    const int V = ncol % 2 == 0 ? 2 : 1, pieces = ncol / V;
+    const int cpl = std::max((pieces + 31) / 32, V == 2 ? (pieces >= 6 ? 2 : 1) : (pieces >= 15 ? 3 : 1));
+    const int G = (pieces + cpl - 1) / cpl;
+    const unsigned blocks = (unsigned)((b.count * G + 255) / 256);
     const TapRec* taps = reinterpret_cast<const TapRec*>(p->taps) + b.offset;
-#define TR_INTERP(CPLV)                                                                                      \
-    k_interp<CPLV><<<blocks, 256, 0, st>>>(p->bufA, taps, b.count, ncol, G, p->os[0], p->os[1], p->os[2], mode, \
-                                           sigma, y, out)
-    if (cpl <= 1) TR_INTERP(1);
-    else if (cpl <= 2) TR_INTERP(2);
-    else if (cpl <= 3) TR_INTERP(3);
-    else if (cpl <= 4) TR_INTERP(4);
-    else if (cpl <= 8) TR_INTERP(8);
-    else return fail(TR_ERR_UNSUPPORTED, "more than 256 k-space columns per bin are not supported");
+#define TR_INTERP(VV, CPLV)                                                                                      \
+    k_interp<VV, CPLV><<<blocks, 256, 0, st>>>(p->bufA, taps, b.count, ncol, G, p->os[0], p->os[1], p->os[2], mode, \
+                                               sigma, y, out)
+    if (V == 2) {
+        switch (cpl) {
+            case 1: TR_INTERP(2, 1); break;
+            case 2: TR_INTERP(2, 2); break;
+            case 3: TR_INTERP(2, 3); break;
+            default: TR_INTERP(2, 4); break;
+        }
+    } else {
+        switch (cpl) {
+            case 1: TR_INTERP(1, 1); break;
+            case 2: TR_INTERP(1, 2); break;
+            case 3: TR_INTERP(1, 3); break;
+            case 4: TR_INTERP(1, 4); break;
+            default: TR_INTERP(1, 8); break;
+        }
+    }
 #undef TR_INTERP
     TR_CHECK_LAUNCH();
     return TR_OK;

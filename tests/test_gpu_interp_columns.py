@@ -1,0 +1,32 @@
+"""Interpolation lanes: pairs of columns where the count is even, single ones where it is odd, one to
+eight pieces a lane, last lanes partly past the end; against the oracle."""
+
+import numpy as np
+import pytest
+
+from _fixtures import pkg
+from oracle import nufft as onf
+
+pytestmark = pytest.mark.gpu
+
+
+# pieces a lane: 1, 1, 2 (tail), 2, 3, 3 (tail), 2 (several CTAs' worth), 3, 3 (tail), 4, 4 (tail), 8, 4
+@pytest.mark.parametrize("ncoil,necho", [(3, 3), (5, 2), (7, 2), (6, 2), (5, 3), (19, 1), (11, 6), (13, 10), (11, 9),
+                                         (25, 5), (30, 8), (31, 7)])
+def test_column_counts_match_oracle(ncoil, necho):
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    rng = np.random.default_rng(ncoil * 100 + necho)
+    shape, M = (16, 20, 12), 301
+    k = np.stack([rng.uniform(-n / 2, n / 2, M) for n in shape], -1).astype(np.float32)
+    k[0] = 0.0                                                 # five taps per axis
+    k[1] = [-shape[0] / 2, -shape[1] / 2, -shape[2] / 2]       # wraps
+    cplx = lambda *s: (rng.standard_normal(s) + 1j * rng.standard_normal(s)).astype(np.complex64)
+    maps, img = cplx(ncoil, *shape), cplx(necho, *shape)
+    be = pkg("nufft_backend").B200NufftBackend(shape, [k], 0, n_coils=ncoil, n_echoes=necho)
+    be.set_maps(torch.from_numpy(maps))
+    y = be.unsort_kspace(be.forward_bin(torch.from_numpy(img).cuda(), 0), 0).cpu().numpy()
+    be.close()
+    yo = np.stack([onf.nufft(img[e] * maps[c], k) for e in range(necho) for c in range(ncoil)])
+    assert onf.rel_l2(y, yo) < 1e-5                            # float32 sums; about 1e-6 at other sizes

@@ -910,6 +910,13 @@ __global__ void __launch_bounds__(kWideNT, 5) k_adj_x_wide(AdjXArgs a, const __g
 // Column counts of the few-column interpolation and gridding kernels: k_interp and k_spread spread
 // 16 or more columns over their lanes.
 constexpr int kFewCols = 8;
+// Most samples for which k_interp_rows takes a bin of 1 to 8 columns.  Its sixteen lanes a sample hide
+// latency while samples are few; with many, k_interp reads the same grid lines with fewer instructions
+// (us, rows / k_interp, at 50 000, 100 000 and 213 000 samples: 1 column 12.0 / 15.1, 21.4 / 16.8,
+// 43.2 / 22.9; 2: 12.5 / 21.4, 22.4 / 22.1, 45.2 / 31.2; 4: 15.4 / 21.5, 27.2 / 30.6, 55.2 / 48.6;
+// 6: 23.0 / 28.2, 41.6 / 39.6, 83.6 / 72.3; 7: 32.5 / 26.6, 58.2 / 45.7, 115 / 91; 8: 25.2 / 40.0,
+// 43.8 / 53.6, 84.9 / 82.6).
+constexpr int64_t kFewRowsMax[kFewCols + 1] = {0, 65536, 98304, 65536, 131072, 49152, 81920, 20480, 196608};
 
 // First tap per axis and the 15 KB weights of every (sorted) sample, computed
 // once at plan creation; interpolation and gridding read them instead of
@@ -946,7 +953,8 @@ __global__ void k_prep_taps(const float4* __restrict__ ks, int64_t M, float beta
 template <int V, int CPL>
 __global__ void __launch_bounds__(256) k_interp(const float2* __restrict__ grid, const TapRec* __restrict__ taps,
                                                 int64_t M, int ncol, int G, int os0, int os1, int os2,
-                                                int mode, float sigma, const float2* __restrict__ y,
+                                                int mode, float sigma, const int32_t* __restrict__ perm,
+                                                const float2* __restrict__ y,
                                                 float2* __restrict__ out) {
     const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t s = gt / G;
@@ -1013,13 +1021,14 @@ __global__ void __launch_bounds__(256) k_interp(const float2* __restrict__ grid,
             }
         }
     }
+    const int64_t so = perm ? perm[s] : s;
 #pragma unroll
     for (int j = 0; j < CPL; ++j) {
         const int col = (lane + j * G) * V;
         if (col >= ncol) continue;
 #pragma unroll
         for (int u = 0; u < V; ++u) {
-            const int64_t o = s * ncol + col + u;
+            const int64_t o = so * ncol + col + u;
             if (mode == kInterpDualProx) {
                 const float2 r = csub(acc[j][u], y[o]);
                 const float2 q = out[o];
@@ -2050,7 +2059,7 @@ static tr_status stage_interp(tr_plan* p, int bin, int ncol, int mode, float sig
                               cudaStream_t st, const int32_t* perm = nullptr) {
     const Bin& b = p->bins[bin];
     if (b.count == 0) return TR_OK;
-    if (ncol <= kFewCols) {
+    if (ncol <= kFewCols && b.count <= kFewRowsMax[ncol]) {
         const TapRec* taps = reinterpret_cast<const TapRec*>(p->taps) + b.offset;
         const unsigned blocks = (unsigned)((b.count * 16 + 255) / 256);
 #define TR_INTERP_ROWS(NCV)                                                                                       \
@@ -2071,17 +2080,18 @@ static tr_status stage_interp(tr_plan* p, int bin, int ncol, int mode, float sig
     // Even column counts read pairs (bufA is aligned and a row of ncol even columns starts on 16 bytes).
     // Fewer lanes a sample, so that a warp holds several samples and a lane several loads in flight, is
     // faster from two pieces a lane on (64 x 96 x 96, 80 000 samples, 1 / 2 / 3 / 4 pieces a lane: 12 columns
-    // 71 / 66 / 78 / 110 us, 24: 142 / 90 / 103 / 181, 48: 257 / 155 / 162 / 274; 10: 53 / 63 / 78 / 103);
+    // 71 / 66 / 78 / 110 us, 24: 142 / 90 / 103 / 181, 48: 257 / 155 / 162 / 274; 10: 53 / 63 / 78 / 103;
+    // 8, 960 000 samples on 150^3: 399 / 336 / 353 / 577, 6: 304 / 288 / 259 / 394 but 72 / 73 / 82 / 107 at 213 000);
     // odd ones, single values, from three on (15: 85 / 100 / 83 / 97, 25: 135 / 136 / 112 / 128,
     // 45: 218 / 218 / 176 / 201; 9: 48 / 81 / 69 / 84).
     const int V = ncol % 2 == 0 ? 2 : 1, pieces = ncol / V;
-    const int cpl = std::max((pieces + 31) / 32, V == 2 ? (pieces >= 6 ? 2 : 1) : (pieces >= 15 ? 3 : 1));
+    const int cpl = std::max((pieces + 31) / 32, V == 2 ? (pieces == 4 || pieces >= 6 ? 2 : 1) : (pieces >= 15 ? 3 : 1));
     const int G = (pieces + cpl - 1) / cpl;
     const unsigned blocks = (unsigned)((b.count * G + 255) / 256);
     const TapRec* taps = reinterpret_cast<const TapRec*>(p->taps) + b.offset;
 #define TR_INTERP(VV, CPLV)                                                                                      \
     k_interp<VV, CPLV><<<blocks, 256, 0, st>>>(p->bufA, taps, b.count, ncol, G, p->os[0], p->os[1], p->os[2], mode, \
-                                               sigma, y, out)
+                                               sigma, perm, y, out)
     if (V == 2) {
         switch (cpl) {
             case 1: TR_INTERP(2, 1); break;

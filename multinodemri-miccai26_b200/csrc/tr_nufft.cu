@@ -1173,7 +1173,7 @@ __global__ void __launch_bounds__(256) k_interp_rows(const float2* __restrict__ 
 // row) steps through the entries that reach its row, found by a ballot over the row
 // weights.  Bound by instruction issue; with every warp stepping through every entry
 // and three barriers per 32 the gridding of 96 columns (128 x 256 x 256 image) took
-// 3.81 ms and of 72 columns (112 x 160 x 160) 1.33 ms, now 3.32 and 1.18 ms.  The launch runs work items first: a tile's list range
+// 3.81 ms and of 72 columns (112 x 160 x 160) 1.33 ms, now 3.22 and 0.96 ms.  The launch runs work items first: a tile's list range
 // (lists longer than kSplitEntries are cut into ranges whose partial tiles go
 // to a scratch buffer, the first range writing the grid), heaviest first; the
 // trailing CTAs write zeros into tiles no sample reaches, kZeroTiles each.
@@ -1230,9 +1230,16 @@ __device__ __forceinline__ void tile_geometry(const SpreadArgs& a, int tile, int
 // entry's values arrive by one bulk copy (cp.async.bulk) on an mbarrier, and
 // finished tiles (and the zero tiles) leave by one 4-D TMA store each, clipped
 // at the grid edge by the TMA unit.  TMA = false: values staged by plain loads, coalesced warp stores.
+// CTAs per SM that the register budget is cut for.  72 columns (112 x 160 x 160 image, 186 200 samples):
+// CG 6 and three CTAs 1132 us, CG 5 and three 1091, CG 5 and four 961 (80 registers or 64: the latency of
+// a work item's list and values is what more CTAs hide); 128 columns (64 x 96 x 96, 80 000 samples): CG 8 and
+// three CTAs, which spill, 853 us, two 523; four for CG 6 spill too, three or six for CG 1 to 4 are slower.
+template <int CG>
+constexpr int spread_ctas() { return CG >= 7 ? 2 : (CG >= 6 ? 3 : (CG >= 4 ? 4 : 5)); }
+
 template <int CG, bool TMA>
-__global__ void __launch_bounds__(256, (CG >= 6 ? 3 : (CG >= 4 ? 4 : 5))) k_spread(SpreadArgs a,
-                                                                 const __grid_constant__ CUtensorMap tgrid) {
+__global__ void __launch_bounds__(256, spread_ctas<CG>()) k_spread(SpreadArgs a,
+                                                                             const __grid_constant__ CUtensorMap tgrid) {
     extern __shared__ __align__(128) unsigned char smraw_[];
     __shared__ float s_wzy[2][kSpreadSub * 17];          // (z, y) weight times dcf of the 16 tile rows
     __shared__ __align__(16) float s_wx[2][kSpreadSub * 4];
@@ -2201,7 +2208,9 @@ static tr_status stage_spread(tr_plan* p, int bin, const float2* ksp, int ncol, 
     else if (cg <= 2) TR_SPREAD_CG(2);
     else if (cg <= 3) TR_SPREAD_CG(3);
     else if (cg <= 4) TR_SPREAD_CG(4);
+    else if (cg <= 5) TR_SPREAD_CG(5);
     else if (cg <= 6) TR_SPREAD_CG(6);
+    else if (cg <= 7) TR_SPREAD_CG(7);
     else TR_SPREAD_CG(8);
 #undef TR_SPREAD_CG
     if (b.n_split > 0) {

@@ -328,7 +328,7 @@ def run_b200(args):
     # per iteration: TV duals, primal, tolerance reduction
     launches_per_iter = B * (4 + math.ceil(ncol / 128) + 1 + 3) + 3
     if cfg.algorithm == "tvmw":
-        launches_per_iter += 6 * max(1, solver.backend.wavelet_levels)
+        launches_per_iter += 4 * max(1, solver.backend.wavelet_levels)
 
     clocks = ClockSampler(local)
     # ---- warm-up and K timed steps (one PDHG iteration each)

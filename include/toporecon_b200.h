@@ -69,7 +69,7 @@ typedef struct {
 } tr_plan_desc;
 
 #define TR_PLAN_AUTOTUNE 1       /* time candidate launch shapes at plan creation */
-#define TR_PLAN_NO_TMA 2         /* stage FFT tiles with cp.async instead of TMA (comparison runs) */
+#define TR_PLAN_NO_TMA 2         /* FFT passes without TMA (comparison runs) */
 #define TR_PLAN_YZ_FUSION 4      /* run the y and z FFT passes as one cluster kernel where the geometry
                                     allows (comparison runs: measured slower than the separate passes) */
 #define TR_PLAN_THREE_PASS_320 8 /* run the 320-point FFT passes (x and the line passes) in three

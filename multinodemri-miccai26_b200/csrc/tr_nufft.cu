@@ -950,7 +950,8 @@ __global__ void k_prep_taps(const float4* __restrict__ ks, int64_t M, float beta
 // reads where the grid is small, by HBM where it is large: 32 columns on 120 x 160 x 160 (136 000 samples)
 // 216 -> 148 us against single columns a power of two apart, 72 on 140 x 200 x 200 801 -> 564 us,
 // 96 on 160 x 320 x 320 2.53 -> 2.27 ms (0.93 of the copy rate).
-template <int V, int CPL>
+// PERM: sample s goes to row perm[s] of out (as an argument that is null elsewhere it cost 5 %).
+template <int V, int CPL, bool PERM>
 __global__ void __launch_bounds__(256) k_interp(const float2* __restrict__ grid, const TapRec* __restrict__ taps,
                                                 int64_t M, int ncol, int G, int os0, int os1, int os2,
                                                 int mode, float sigma, const int32_t* __restrict__ perm,
@@ -1021,7 +1022,7 @@ __global__ void __launch_bounds__(256) k_interp(const float2* __restrict__ grid,
             }
         }
     }
-    const int64_t so = perm ? perm[s] : s;
+    const int64_t so = PERM ? perm[s] : s;
 #pragma unroll
     for (int j = 0; j < CPL; ++j) {
         const int col = (lane + j * G) * V;
@@ -2097,7 +2098,7 @@ static tr_status stage_interp(tr_plan* p, int bin, int ncol, int mode, float sig
     const unsigned blocks = (unsigned)((b.count * G + 255) / 256);
     const TapRec* taps = reinterpret_cast<const TapRec*>(p->taps) + b.offset;
 #define TR_INTERP(VV, CPLV)                                                                                      \
-    k_interp<VV, CPLV><<<blocks, 256, 0, st>>>(p->bufA, taps, b.count, ncol, G, p->os[0], p->os[1], p->os[2], mode, \
+    k_interp<VV, CPLV, false><<<blocks, 256, 0, st>>>(p->bufA, taps, b.count, ncol, G, p->os[0], p->os[1], p->os[2], mode, \
                                                sigma, perm, y, out)
     if (V == 2) {
         switch (cpl) {
@@ -2108,7 +2109,12 @@ static tr_status stage_interp(tr_plan* p, int bin, int ncol, int mode, float sig
         }
     } else {
         switch (cpl) {
-            case 1: TR_INTERP(1, 1); break;
+            case 1:
+                if (perm)          // one column
+                    k_interp<1, 1, true><<<blocks, 256, 0, st>>>(p->bufA, taps, b.count, ncol, G, p->os[0], p->os[1],
+                                                                 p->os[2], mode, sigma, perm, y, out);
+                else TR_INTERP(1, 1);
+                break;
             case 2: TR_INTERP(1, 2); break;
             case 3: TR_INTERP(1, 3); break;
             case 4: TR_INTERP(1, 4); break;

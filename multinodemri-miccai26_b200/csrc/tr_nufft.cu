@@ -2086,14 +2086,20 @@ static tr_status stage_interp(tr_plan* p, int bin, int ncol, int mode, float sig
     }
     if (ncol > 256) return fail(TR_ERR_UNSUPPORTED, "more than 256 k-space columns per bin are not supported");
     // Even column counts read pairs (bufA is aligned and a row of ncol even columns starts on 16 bytes).
-    // Fewer lanes a sample, so that a warp holds several samples and a lane several loads in flight, is
-    // faster from two pieces a lane on (64 x 96 x 96, 80 000 samples, 1 / 2 / 3 / 4 pieces a lane: 12 columns
-    // 71 / 66 / 78 / 110 us, 24: 142 / 90 / 103 / 181, 48: 257 / 155 / 162 / 274; 10: 53 / 63 / 78 / 103;
-    // 8, 960 000 samples on 150^3: 399 / 336 / 353 / 577, 6: 304 / 288 / 259 / 394 but 72 / 73 / 82 / 107 at 213 000);
-    // odd ones, single values, from three on (15: 85 / 100 / 83 / 97, 25: 135 / 136 / 112 / 128,
-    // 45: 218 / 218 / 176 / 201; 9: 48 / 81 / 69 / 84).
+    // While the lanes of one piece each are at most a wave of the chip's threads, one piece a lane is faster
+    // (us at 1 / 2 / 3 pieces a lane, 60 x 70 x 80 grid: 12 columns, 18 000 samples 23 / 29 / 38, 48 000 35 / 49 / 64;
+    // 32 columns, 6 000 samples 21 / 26 / 32, 18 000 35 / 44 / 66); beyond it fewer lanes a sample, so that a warp
+    // holds several samples and a lane several loads in flight (80 x 120 x 120 grid, 80 000 samples, 1 / 2 / 3 / 4:
+    // 12 columns 71 / 66 / 78 / 110, 24: 142 / 90 / 103 / 181, 48: 257 / 155 / 162 / 274; 10: 53 / 63 / 78 / 103;
+    // 8 columns, 960 000 samples on 150^3: 399 / 336 / 353 / 577, 6: 304 / 288 / 259 / 394 but 72 / 73 / 82 / 107 at
+    // 213 000).  Odd ones, single values, turn at four waves (15: 85 / 100 / 83 / 97, 25: 135 / 136 / 112 / 128, at
+    // 48 000 samples 85 / 103 / 85; 9: 48 / 81 / 69 / 84), above 32 columns at once (45, 6 000 samples: 64 / 63 / 50).
     const int V = ncol % 2 == 0 ? 2 : 1, pieces = ncol / V;
-    const int cpl = std::max((pieces + 31) / 32, V == 2 ? (pieces == 4 || pieces >= 6 ? 2 : 1) : (pieces >= 15 ? 3 : 1));
+    constexpr int64_t kWave = 148 * 2048;
+    const int64_t lanes = b.count * pieces;
+    const int more = V == 2 ? ((pieces == 4 || pieces >= 6) && lanes > kWave ? 2 : 1)
+                            : (pieces > 32 || (pieces >= 15 && lanes > 4 * kWave) ? 3 : 1);
+    const int cpl = std::max((pieces + 31) / 32, more);
     const int G = (pieces + cpl - 1) / cpl;
     const unsigned blocks = (unsigned)((b.count * G + 255) / 256);
     const TapRec* taps = reinterpret_cast<const TapRec*>(p->taps) + b.offset;

@@ -10,7 +10,7 @@ from oracle import nufft as onf
 pytestmark = pytest.mark.gpu
 
 
-# pieces a lane: 1, 1, 2 (tail), 2, 3, 3 (tail), 2 (several CTAs' worth), 3, 3 (tail), 4, 4 (tail), 8, 4
+# one to eight pieces a lane, as far as few samples reach them
 @pytest.mark.parametrize("ncoil,necho", [(3, 3), (5, 2), (7, 2), (6, 2), (5, 3), (19, 1), (11, 6), (13, 10), (11, 9),
                                          (25, 5), (30, 8), (31, 7)])
 def test_column_counts_match_oracle(ncoil, necho):
@@ -32,10 +32,10 @@ def test_column_counts_match_oracle(ncoil, necho):
     assert onf.rel_l2(y, yo) < 1e-5                            # float32 sums; about 1e-6 at other sizes
 
 
-# 1 to 8 columns: the largest bin of the row kernel and one sample more; a sample's value does not
+# 1 to 8 columns: the largest bin of the row kernel and one sample more; 12 to 26: of one piece a lane; a sample's value does not
 # depend on the others, so that the oracle takes the first 300 and the last 20
 @pytest.mark.parametrize("ncol,limit", [(1, 65536), (2, 98304), (3, 65536), (4, 131072), (5, 49152), (6, 81920),
-                                        (7, 20480), (8, 196608)])
+                                        (7, 20480), (8, 196608), (12, 50517), (15, 80827), (26, 23315)])
 def test_few_columns_with_many_samples(ncol, limit):
     torch = pytest.importorskip("torch")
     if not torch.cuda.is_available():

@@ -254,13 +254,13 @@ __global__ void __launch_bounds__(256) k_conv3d_pack(const TW* __restrict__ w, _
 __host__ __device__ constexpr int conv_npad(int cout) { return (cout + 15) / 16 * 16; }
 int64_t packed_elems(int cin, int cout) { return (int64_t)((cin + 15) / 16) * 27 * 16 * conv_npad(cout); }
 
-// VEC: halo rows are read 16 bytes at a time.
+// VEC: halo rows are read 16 bytes at a time; yvec: y is 16-byte aligned, rows are written so.
 template <int NZ, class TIn, bool VEC>
 __global__ void __launch_bounds__(kFwdThreads, 1) k_conv3d_fwd(const TIn* __restrict__ x,
                                                                const __nv_bfloat16* __restrict__ w,
                                                                const float* __restrict__ bias, float* __restrict__ y,
                                                                ConvDims c, int tiles, int npad, int nacc, uint32_t cols,
-                                                               int poll) {
+                                                               int yvec, int poll) {
     extern __shared__ __align__(128) unsigned char smraw_[];
     __shared__ __align__(8) uint64_t hfull[kHaloStages], hempty[kHaloStages], wfull[kMaxWStages],
         wempty[kMaxWStages], afull[2], aempty[2], drained[2];
@@ -451,7 +451,12 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_conv3d_fwd(const TIn* __rest
                         float4 v = *reinterpret_cast<const float4*>(stage + row * kEpPitch + c4);
                         if (bias) v = make_float4(v.x + bv.x, v.y + bv.y, v.z + bv.z, v.w + bv.w);
                         if (bad) v.x = v.y = v.z = v.w = __int_as_float(0x7fffffff);
-                        *reinterpret_cast<float4*>(out + ((int64_t)yy * c.W + xx) * c.Cout + c0 + c4) = v;
+                        float* dst = out + ((int64_t)yy * c.W + xx) * c.Cout + c0 + c4;
+                        if (yvec) {
+                            *reinterpret_cast<float4*>(dst) = v;
+                        } else {
+                            dst[0] = v.x, dst[1] = v.y, dst[2] = v.z, dst[3] = v.w;
+                        }
                     }
                     __syncwarp();
                 }
@@ -729,7 +734,7 @@ tr_status launch_fwd(const TIn* x, const __nv_bfloat16* w, const float* bias, fl
     const int nacc = 2 * NZ * npad <= 512 ? 2 : 1;
     TR_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     fn<<<(unsigned)std::min<int64_t>(tiles, sm_count()), kFwdThreads, smem, st>>>(
-        x, w, bias, y, c, (int)tiles, npad, nacc, tmem_cols(nacc * NZ * npad), kMbarPollLimit);
+        x, w, bias, y, c, (int)tiles, npad, nacc, tmem_cols(nacc * NZ * npad), ((uintptr_t)y % 16) == 0, kMbarPollLimit);
     TR_CHECK_LAUNCH();
     return TR_OK;
 }

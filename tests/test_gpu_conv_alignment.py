@@ -1,0 +1,50 @@
+"""Warm-start convolutions on buffers that are only aligned to their element type: views at odd offsets
+of a caller's allocation give the same bits as aligned ones."""
+
+import ctypes
+
+import pytest
+
+from _fixtures import pkg
+
+pytestmark = pytest.mark.gpu
+
+SHAPE, CIN, COUT = (1, 5, 17, 9), 24, 40
+
+
+def _torch():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    return torch
+
+
+def _at(torch, t, offset):
+    """A contiguous copy of t that starts `offset` elements into its allocation."""
+    buf = torch.empty(t.numel() + offset + 8, dtype=t.dtype, device=t.device)
+    v = buf[offset:offset + t.numel()].view(t.shape)
+    v.copy_(t)
+    return v
+
+
+def _ptr(t):
+    return ctypes.c_void_p(t.data_ptr())
+
+
+@pytest.mark.parametrize("offset", [1, 2, 3])
+def test_forward_into_unaligned_output(offset):
+    torch = _torch()
+    ws, lib = pkg("warmstart"), pkg("_lib")
+    x = torch.randn(SHAPE + (CIN,), device="cuda").bfloat16()
+    w = torch.randn(COUT, 27, CIN, device="cuda").bfloat16()
+    ref = ws.conv3d_fwd_bf16(x, w)
+    packed = ws.pack_weights(w, CIN, COUT)
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    for call, weights in (("tr_conv3d_fwd", w), ("tr_conv3d_fwd_packed", packed)):
+        buf = torch.full((ref.numel() + 8,), -7.0, device="cuda")
+        y = buf[offset:offset + ref.numel()]
+        assert y.data_ptr() % 16 == 4 * offset
+        head = (_ptr(x),) if call == "tr_conv3d_fwd" else (_ptr(x), 0)
+        lib.check(getattr(lib.load(), call)(*head, _ptr(weights), None, _ptr(y), *SHAPE, CIN, COUT, stream))
+        assert torch.equal(y.view(ref.shape), ref)
+        assert torch.all(buf[:offset] == -7.0) and torch.all(buf[offset + ref.numel():] == -7.0)

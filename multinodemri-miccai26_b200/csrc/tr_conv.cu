@@ -140,19 +140,28 @@ __host__ __device__ constexpr int plane_pitch(int voxels) { return voxels + ((2 
 
 // ------------------------------------------------------------------ 8 channels of one voxel
 // Channels [c, c + 8) at p (the voxel's channel 0), zero past C; VEC: C % 8 == 0 and 16-byte
-// aligned rows.
+// aligned rows; else pairs: 4-byte aligned rows.
 template <bool VEC>
-__device__ __forceinline__ uint4 load8(const __nv_bfloat16* p, int c, int C) {
+__device__ __forceinline__ uint4 load8(const __nv_bfloat16* p, int c, int C, bool pairs) {
     if constexpr (VEC) {
         return c < C ? *reinterpret_cast<const uint4*>(p + c) : make_uint4(0, 0, 0, 0);
     } else {
-        uint32_t r[4];
+        uint32_t r[4] = {0u, 0u, 0u, 0u};
+        if (pairs) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)                   // C is even: pairs never straddle the end
-            r[i] = c + 2 * i < C ? *reinterpret_cast<const uint32_t*>(p + c + 2 * i) : 0u;
+            for (int i = 0; i < 4; ++i)               // C is even: pairs never straddle the end
+                if (c + 2 * i < C) r[i] = *reinterpret_cast<const uint32_t*>(p + c + 2 * i);
+        } else {
+            const auto* h = reinterpret_cast<const unsigned short*>(p + c);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (c + 2 * i < C) r[i] = h[2 * i] | ((uint32_t)h[2 * i + 1] << 16);
+        }
         return make_uint4(r[0], r[1], r[2], r[3]);
     }
 }
+__host__ __device__ __forceinline__ bool at16(const void* p) { return (uintptr_t)p % 16 == 0; }
+__host__ __device__ __forceinline__ bool at4(const void* p) { return (uintptr_t)p % 4 == 0; }
 __device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t*>(&h);
@@ -163,7 +172,7 @@ template <class TIn, bool VEC>
 struct Piece {
     uint4 v;
     __device__ __forceinline__ void zero() { v = make_uint4(0, 0, 0, 0); }
-    __device__ __forceinline__ void load(const __nv_bfloat16* p, int c, int C) { v = load8<VEC>(p, c, C); }
+    __device__ __forceinline__ void load(const __nv_bfloat16* p, int c, int C, bool pairs) { v = load8<VEC>(p, c, C, pairs); }
     __device__ __forceinline__ uint4 bf16() const { return v; }
 };
 template <bool VEC>
@@ -173,7 +182,7 @@ struct Piece<float, VEC> {
 #pragma unroll
         for (int i = 0; i < 8; ++i) f[i] = 0.f;
     }
-    __device__ __forceinline__ void load(const float* p, int c, int C) {
+    __device__ __forceinline__ void load(const float* p, int c, int C, bool) {
         if constexpr (VEC) {
             if (c >= C) return zero();
             const float4 a = *reinterpret_cast<const float4*>(p + c), b = *reinterpret_cast<const float4*>(p + c + 4);
@@ -375,6 +384,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_conv3d_fwd(const TIn* __rest
         constexpr int kUnits = 2 * kSlice * (NZ + 2), kPer = (kUnits + kLoaders - 1) / kLoaders;
         constexpr int kBatch = 5;                            // pieces in flight per thread
         const int lt = tid - (kFwdThreads - kLoaders), pl = lt & 1;
+        const bool pairs = at4(x);
         int hs = 0, hu = 0;
         for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
             int b = t;
@@ -402,7 +412,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_conv3d_fwd(const TIn* __rest
                     Piece<TIn, VEC> v[kBatch];
 #pragma unroll
                     for (int k = 0; k < kBatch; ++k)
-                        if (k0 + k < kPer && off[k0 + k] >= 0) v[k].load(corner + (int64_t)off[k0 + k] * c.Cin, c0, c.Cin);
+                        if (k0 + k < kPer && off[k0 + k] >= 0) v[k].load(corner + (int64_t)off[k0 + k] * c.Cin, c0, c.Cin, pairs);
                         else v[k].zero();
 #pragma unroll
                     for (int k = 0; k < kBatch; ++k) {
@@ -525,7 +535,7 @@ template <int NPAD, bool XVEC, bool MX>
 __global__ void __launch_bounds__(kWgThreads) k_conv3d_wgrad(const __nv_bfloat16* __restrict__ x,
                                                              const __nv_bfloat16* __restrict__ gy,
                                                              float* __restrict__ part, ConvDims c, WgradShape s,
-                                                             int gvec, int poll) {
+                                                             int poll) {
     extern __shared__ __align__(128) unsigned char smraw_[];
     __shared__ __align__(8) uint64_t full[kWgRing], empty[kWgRing], done;
     __shared__ uint32_t tmem_slot;
@@ -631,8 +641,9 @@ __global__ void __launch_bounds__(kWgThreads) k_conv3d_wgrad(const __nv_bfloat16
 #pragma unroll
                 for (int k = 0; k < kPerX; ++k) {
                     const int ch = cx0 + (dx[k] / (kXPitch * 16)) * 8;
-                    bx[k] = vx[k] >= 0 && (unsigned)zx < (unsigned)c.D ? load8<XVEC>(xs + (int64_t)vx[k] * c.Cin, ch, c.Cin)
-                                                                       : make_uint4(0, 0, 0, 0);
+                    bx[k] = make_uint4(0, 0, 0, 0);
+                    if (vx[k] >= 0 && (unsigned)zx < (unsigned)c.D)
+                        bx[k] = load8<XVEC>(xs + (int64_t)vx[k] * c.Cin, ch, c.Cin, at4(x));
                 }
                 if (i >= 2) {
 #pragma unroll
@@ -640,8 +651,8 @@ __global__ void __launch_bounds__(kWgThreads) k_conv3d_wgrad(const __nv_bfloat16
                         const int ch = cg0 + (dg[k] / (kGPitch * 16)) * 8;
                         bg[k] = make_uint4(0, 0, 0, 0);
                         if (vg[k] >= 0)
-                            bg[k] = gvec ? load8<true>(gs + (int64_t)vg[k] * c.Cout, ch, c.Cout)
-                                         : load8<false>(gs + (int64_t)vg[k] * c.Cout, ch, c.Cout);
+                            bg[k] = at16(gy) ? load8<true>(gs + (int64_t)vg[k] * c.Cout, ch, c.Cout, true)
+                                             : load8<false>(gs + (int64_t)vg[k] * c.Cout, ch, c.Cout, at4(gy));
                     }
                 }
 #pragma unroll
@@ -734,7 +745,7 @@ tr_status launch_fwd(const TIn* x, const __nv_bfloat16* w, const float* bias, fl
     const int nacc = 2 * NZ * npad <= 512 ? 2 : 1;
     TR_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     fn<<<(unsigned)std::min<int64_t>(tiles, sm_count()), kFwdThreads, smem, st>>>(
-        x, w, bias, y, c, (int)tiles, npad, nacc, tmem_cols(nacc * NZ * npad), ((uintptr_t)y % 16) == 0, kMbarPollLimit);
+        x, w, bias, y, c, (int)tiles, npad, nacc, tmem_cols(nacc * NZ * npad), at16(y), kMbarPollLimit);
     TR_CHECK_LAUNCH();
     return TR_OK;
 }
@@ -759,7 +770,7 @@ tr_status conv_fwd(const TIn* x, const __nv_bfloat16* packed, const float* bias,
     }
     if (tiles > INT32_MAX - sms || (int64_t)c.H * c.W > INT32_MAX / 8)
         return tr::fail(TR_ERR_UNSUPPORTED, "conv3d: volume too large");
-    const bool vec = c.Cin % 8 == 0 && ((uintptr_t)x % 16) == 0;
+    const bool vec = c.Cin % 8 == 0 && at16(x);
 #define TR_FWD_NZ(NZV) \
     return vec ? launch_fwd<NZV, TIn, true>(x, packed, bias, y, c, tiles, st) \
                : launch_fwd<NZV, TIn, false>(x, packed, bias, y, c, tiles, st)
@@ -816,7 +827,7 @@ WgradShape wgrad_shape(const ConvDims& c, int64_t max_splits) {
     return s;
 }
 
-using WgradKernel = void (*)(const __nv_bfloat16*, const __nv_bfloat16*, float*, ConvDims, WgradShape, int, int);
+using WgradKernel = void (*)(const __nv_bfloat16*, const __nv_bfloat16*, float*, ConvDims, WgradShape, int);
 template <int NPAD>
 WgradKernel wgrad_kernel(bool vec, bool mx) {
     return vec ? (mx ? k_conv3d_wgrad<NPAD, true, true> : k_conv3d_wgrad<NPAD, true, false>)
@@ -894,15 +905,14 @@ extern "C" tr_status tr_conv3d_wgrad(const void* x, const void* gy, float* dw, i
     const auto* gb = (const __nv_bfloat16*)gy;
     float* part = (float*)workspace;
     const size_t smem = (size_t)kWgRing * 16 * (s.px * kXPitch + s.pg * kGPitch) + 128;
-    const bool vec = c.Cin % 8 == 0 && ((uintptr_t)x % 16) == 0;
-    const int gvec = ((uintptr_t)gy % 16) == 0;
+    const bool vec = c.Cin % 8 == 0 && at16(x);
     auto fn = wgrad_kernel<16>(vec, s.mx);
     if (s.npad == 32) fn = wgrad_kernel<32>(vec, s.mx);
     else if (s.npad == 48) fn = wgrad_kernel<48>(vec, s.mx);
     else if (s.npad == 64) fn = wgrad_kernel<64>(vec, s.mx);
     TR_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const dim3 grid((unsigned)s.splits, (unsigned)s.groups, (unsigned)(s.cx * s.cg));
-    fn<<<grid, kWgThreads, smem, st>>>(xb, gb, part, c, s, gvec, kMbarPollLimit);
+    fn<<<grid, kWgThreads, smem, st>>>(xb, gb, part, c, s, kMbarPollLimit);
     TR_CHECK_LAUNCH();
     const int64_t total = partial_floats(c);
     k_wgrad_reduce<<<(unsigned)((total + 127) / 128), 128, 0, st>>>(part, dw, s.splits, Cin, Cout);

@@ -48,3 +48,19 @@ def test_forward_into_unaligned_output(offset):
         lib.check(getattr(lib.load(), call)(*head, _ptr(weights), None, _ptr(y), *SHAPE, CIN, COUT, stream))
         assert torch.equal(y.view(ref.shape), ref)
         assert torch.all(buf[:offset] == -7.0) and torch.all(buf[offset + ref.numel():] == -7.0)
+
+
+@pytest.mark.parametrize("cin,cout", [(24, 40), (18, 24)])
+@pytest.mark.parametrize("offset", [1, 2, 3])
+def test_inputs_at_odd_offsets(offset, cin, cout):
+    torch = _torch()
+    ws = pkg("warmstart")
+    x = torch.randn(SHAPE + (cin,), device="cuda").bfloat16()
+    gy = torch.randn(SHAPE + (cout,), device="cuda").bfloat16()
+    w = torch.randn(cout, 27, cin, device="cuda").bfloat16()
+    xo, go = _at(torch, x, offset), _at(torch, gy, offset)
+    assert xo.data_ptr() % 16 == 2 * offset and xo.is_contiguous()
+    dw = ws.conv3d_wgrad_bf16(x, gy)
+    for a, b in ((xo, gy), (x, go), (xo, go)):
+        assert torch.equal(ws.conv3d_wgrad_bf16(a, b), dw)
+    assert torch.equal(ws.conv3d_fwd_bf16(xo, w), ws.conv3d_fwd_bf16(x, w))

@@ -43,9 +43,10 @@ def _stream(t):
 
 
 def pack_weights(w, cin, cout, data_grad=False):
-    """Weights w, bf16 or float32, contiguous, in the layout the forward kernel streams, as bf16:
+    """Weights w, bf16 or float32, any strides, in the layout the forward kernel streams, as bf16:
     (cout, 27, cin), or with ``data_grad`` the layer's own (cin, 27, cout) flipped and swapped."""
     import torch
+    w = w.contiguous()
     L = _lib.load()
     nbytes = ctypes.c_size_t(0)
     _lib.check(L.tr_conv3d_packed_size(cin, cout, ctypes.byref(nbytes)))
@@ -107,8 +108,7 @@ def _make_conv_fn():
         def forward(ctx, x, w, b, grad):
             if not (grad and any(ctx.needs_input_grad)) and x.dtype == w.dtype == torch.float32:
                 # no backward will read bf16 copies of x and w
-                return conv3d_fwd_packed(x.contiguous(), pack_weights(w.contiguous(), x.shape[-1], w.shape[0]),
-                                         w.shape[0], b)
+                return conv3d_fwd_packed(x.contiguous(), pack_weights(w, x.shape[-1], w.shape[0]), w.shape[0], b)
             xb = x.contiguous().to(torch.bfloat16)
             wb = w.contiguous().to(torch.bfloat16)
             ctx.save_for_backward(xb, wb)

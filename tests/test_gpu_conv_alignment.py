@@ -64,3 +64,18 @@ def test_inputs_at_odd_offsets(offset, cin, cout):
     for a, b in ((xo, gy), (x, go), (xo, go)):
         assert torch.equal(ws.conv3d_wgrad_bf16(a, b), dw)
     assert torch.equal(ws.conv3d_fwd_bf16(xo, w), ws.conv3d_fwd_bf16(x, w))
+
+
+@pytest.mark.parametrize("cin,cout", [(24, 40), (18, 24)])
+def test_strided_weights(cin, cout):
+    torch = _torch()
+    ws = pkg("warmstart")
+    w = torch.randn(cout, 27, cin, device="cuda").bfloat16()
+    gy = torch.randn(SHAPE + (cout,), device="cuda").bfloat16()
+    x = torch.randn(SHAPE + (cin,), device="cuda").bfloat16()
+    views = [w.permute(2, 1, 0).contiguous().permute(2, 1, 0), w.repeat_interleave(2, dim=2)[:, :, ::2]]
+    assert not any(v.is_contiguous() for v in views)
+    for v in views + [w[:1].expand(cout, 27, cin)]:
+        c = v.contiguous()
+        assert torch.equal(ws.conv3d_dgrad_bf16(gy, v), ws.conv3d_dgrad_bf16(gy, c))
+        assert torch.equal(ws.conv3d_fwd_bf16(x, v), ws.conv3d_fwd_bf16(x, c))

@@ -264,11 +264,12 @@ __host__ __device__ constexpr int conv_npad(int cout) { return (cout + 15) / 16 
 int64_t packed_elems(int cin, int cout) { return (int64_t)((cin + 15) / 16) * 27 * 16 * conv_npad(cout); }
 
 // VEC: halo rows are read 16 bytes at a time; yvec: y is 16-byte aligned, rows are written so.
-template <int NZ, class TIn, bool VEC>
+// Off: offsets of halo voxels from the halo's corner (64 bits where a halo spans 2^31 voxels or more).
+template <int NZ, class TIn, bool VEC, class Off>
 __global__ void __launch_bounds__(kFwdThreads, 1) k_conv3d_fwd(const TIn* __restrict__ x,
                                                                const __nv_bfloat16* __restrict__ w,
                                                                const float* __restrict__ bias, float* __restrict__ y,
-                                                               ConvDims c, int tiles, int npad, int nacc, uint32_t cols,
+                                                               ConvDims c, int64_t tiles, int npad, int nacc, uint32_t cols,
                                                                int yvec, int poll) {
     extern __shared__ __align__(128) unsigned char smraw_[];
     __shared__ __align__(8) uint64_t hfull[kHaloStages], hempty[kHaloStages], wfull[kMaxWStages],
@@ -328,7 +329,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_conv3d_fwd(const TIn* __rest
             const uint32_t ahi = (uint32_t)(ad >> 32), bhi = (uint32_t)(bd >> 32), alo = (uint32_t)ad + m0 * kSlice;
             const uint32_t row16 = w_row_bytes(npad) >> 4;
             int hs = 0, hu = 0, ws = 0, wu = 0, n = 0;       // ring entries and their use counts
-            for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++n) {
+            for (int64_t t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++n) {
                 const int as = nacc == 2 ? n & 1 : 0, au = nacc == 2 ? n >> 1 : n;
                 if (au > 0) wait(&aempty[as], au - 1);
                 const uint32_t acc = tmem + (as * NZ + m0) * npad;
@@ -364,7 +365,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_conv3d_fwd(const TIn* __rest
         if (elect_one()) {
             const uint32_t bytes = rows * w_row_bytes(npad);
             int ws = 0, wu = 0, last = 0;                    // copies issued (the last nst may be in flight)
-            for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+            for (int64_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
                 const unsigned char* src = reinterpret_cast<const unsigned char*>(w);
                 for (int g = 0; g < 9 * nchunk; g += rows, src += bytes) {
                     if (wu > 0) wait(&wempty[ws], wu - 1);
@@ -386,21 +387,21 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_conv3d_fwd(const TIn* __rest
         const int lt = tid - (kFwdThreads - kLoaders), pl = lt & 1;
         const bool pairs = at4(x);
         int hs = 0, hu = 0;
-        for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
-            int b = t;
-            const int x0 = (b % ntx) * kTX - 1;
+        for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+            int64_t b = t;
+            const int x0 = (int)(b % ntx) * kTX - 1;
             b /= ntx;
-            const int y0 = (b % nty) * kTY - 1;
+            const int y0 = (int)(b % nty) * kTY - 1;
             b /= nty;
-            const int z0 = (b % ntz) * NZ - 1, img = b / ntz;
-            int off[kPer];                                   // voxel offset from the halo corner, -1 outside
+            const int z0 = (int)(b % ntz) * NZ - 1, img = (int)(b / ntz);
+            Off off[kPer];                                   // voxel offset from the halo corner, -1 outside
 #pragma unroll
             for (int k = 0; k < kPer; ++k) {
                 const int u = lt + k * kLoaders, vox = u >> 1;
                 const int hz = vox / kSlice, r = vox - hz * kSlice, hy = r / kHX, hx = r - hy * kHX;
                 const bool in = u < kUnits && (unsigned)(z0 + hz) < (unsigned)c.D && (unsigned)(y0 + hy) < (unsigned)c.H &&
                                 (unsigned)(x0 + hx) < (unsigned)c.W;
-                off[k] = in ? (hz * c.H + hy) * c.W + hx : -1;
+                off[k] = in ? ((Off)hz * c.H + hy) * c.W + hx : -1;
             }
             const TIn* corner = x + ((((int64_t)img * c.D + z0) * c.H + y0) * c.W + x0) * c.Cin;
             for (int ch = 0; ch < nchunk; ++ch) {
@@ -431,13 +432,13 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_conv3d_fwd(const TIn* __rest
         float* stage = reinterpret_cast<float*>(eps) + (warp & 3) * 32 * kEpPitch;
         const int q = warp & 3;
         int n = 0;
-        for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++n) {
-            int b = t;
-            const int x0 = (b % ntx) * kTX;
+        for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x, ++n) {
+            int64_t b = t;
+            const int x0 = (int)(b % ntx) * kTX;
             b /= ntx;
-            const int y0 = (b % nty) * kTY + q * 4;
+            const int y0 = (int)(b % nty) * kTY + q * 4;
             b /= nty;
-            const int z0 = (b % ntz) * NZ, img = b / ntz;
+            const int z0 = (int)(b % ntz) * NZ, img = (int)(b / ntz);
             const int as = nacc == 2 ? n & 1 : 0, au = nacc == 2 ? n >> 1 : n;
             wait(&afull[as], au);
             __syncwarp();
@@ -506,7 +507,8 @@ struct WgradShape {
     int groups;          // tap groups (grid y)
     int cx, cg;          // channel chunks of each side
     uint32_t cols;
-    int cols_n, seg_len, units, splits;
+    int64_t cols_n, units;           // (image, y, x) voxel columns; z segments of all of them
+    int seg_len, splits;
 };
 
 // Tap groups: all 27 taps' accumulators fit TMEM (two per column range) up to 32 columns each.
@@ -570,8 +572,8 @@ __global__ void __launch_bounds__(kWgThreads) k_conv3d_wgrad(const __nv_bfloat16
             const uint32_t slot16 = slot >> 4, xhi = (uint32_t)(xd >> 32), ghi = (uint32_t)(gd >> 32);
             int item = 0;                 // ring items consumed so far
             bool first = true;
-            for (int u = split; u < s.units && ok; u += s.splits) {
-                const int z0 = (u / s.cols_n) * s.seg_len, nz = min(s.seg_len, c.D - z0);
+            for (int64_t u = split; u < s.units && ok; u += s.splits) {
+                const int z0 = (int)(u / s.cols_n) * s.seg_len, nz = min(s.seg_len, c.D - z0);
                 for (int k = 0; k < nz && ok; ++k) {
                     for (int i = (k == 0 ? 0 : 2); i < 3 && ok; ++i) {
                         const int j = item + k + i;
@@ -611,24 +613,26 @@ __global__ void __launch_bounds__(kWgThreads) k_conv3d_wgrad(const __nv_bfloat16
         const int ng = min(s.pg, 2 * ((min(kWgChunk, c.Cout - cg0) + 15) / 16));
         const int64_t hw = (int64_t)c.H * c.W;
         int item = 0;
-        for (int u = split; u < s.units; u += s.splits) {
-            const int col = u % s.cols_n;
-            const int x0 = (col % ntx) * kTX, y0 = ((col / ntx) % nty) * kTY, img = col / (ntx * nty);
-            const int z0 = (u / s.cols_n) * s.seg_len, nz = min(s.seg_len, c.D - z0);
-            int vx[kPerX], vg[kPerG], dx[kPerX], dg[kPerG];        // voxel in the slice (-1: none); place in the slot
+        for (int64_t u = split; u < s.units; u += s.splits) {
+            const int64_t col = u % s.cols_n;
+            const int x0 = (int)(col % ntx) * kTX, y0 = (int)((col / ntx) % nty) * kTY;
+            const int img = (int)(col / ((int64_t)ntx * nty));
+            const int z0 = (int)(u / s.cols_n) * s.seg_len, nz = min(s.seg_len, c.D - z0);
+            int64_t vx[kPerX], vg[kPerG];                          // voxel in the slice (-1: none)
+            int dx[kPerX], dg[kPerG];                              // place in the slot
 #pragma unroll
             for (int k = 0; k < kPerX; ++k) {
                 const int v = lt + k * kWgLoaders, vox = v / nx, pl = v - vox * nx;
                 const int hy = vox / kHX, yy = y0 - 1 + hy, xx = x0 - 1 + vox - hy * kHX;
                 dx[k] = v < kSlice * nx ? (pl * kXPitch + vox) * 16 : -1;
-                vx[k] = dx[k] >= 0 && (unsigned)yy < (unsigned)c.H && (unsigned)xx < (unsigned)c.W ? yy * c.W + xx : -1;
+                vx[k] = dx[k] >= 0 && (unsigned)yy < (unsigned)c.H && (unsigned)xx < (unsigned)c.W ? (int64_t)yy * c.W + xx : -1;
             }
 #pragma unroll
             for (int k = 0; k < kPerG; ++k) {
                 const int v = lt + k * kWgLoaders, vox = v / ng, pl = v - vox * ng;
                 const int yy = y0 + (vox >> 3), xx = x0 + (vox & 7);
                 dg[k] = v < kTX * kTY * ng ? (pl * kGPitch + vox) * 16 : -1;
-                vg[k] = dg[k] >= 0 && yy < c.H && xx < c.W ? yy * c.W + xx : -1;
+                vg[k] = dg[k] >= 0 && yy < c.H && xx < c.W ? (int64_t)yy * c.W + xx : -1;
             }
             for (int i = 0; i < nz + 2; ++i, ++item) {
                 if (item >= kWgRing)
@@ -643,7 +647,7 @@ __global__ void __launch_bounds__(kWgThreads) k_conv3d_wgrad(const __nv_bfloat16
                     const int ch = cx0 + (dx[k] / (kXPitch * 16)) * 8;
                     bx[k] = make_uint4(0, 0, 0, 0);
                     if (vx[k] >= 0 && (unsigned)zx < (unsigned)c.D)
-                        bx[k] = load8<XVEC>(xs + (int64_t)vx[k] * c.Cin, ch, c.Cin, at4(x));
+                        bx[k] = load8<XVEC>(xs + vx[k] * c.Cin, ch, c.Cin, at4(x));
                 }
                 if (i >= 2) {
 #pragma unroll
@@ -651,8 +655,8 @@ __global__ void __launch_bounds__(kWgThreads) k_conv3d_wgrad(const __nv_bfloat16
                         const int ch = cg0 + (dg[k] / (kGPitch * 16)) * 8;
                         bg[k] = make_uint4(0, 0, 0, 0);
                         if (vg[k] >= 0)
-                            bg[k] = at16(gy) ? load8<true>(gs + (int64_t)vg[k] * c.Cout, ch, c.Cout, true)
-                                             : load8<false>(gs + (int64_t)vg[k] * c.Cout, ch, c.Cout, at4(gy));
+                            bg[k] = at16(gy) ? load8<true>(gs + vg[k] * c.Cout, ch, c.Cout, true)
+                                             : load8<false>(gs + vg[k] * c.Cout, ch, c.Cout, at4(gy));
                     }
                 }
 #pragma unroll
@@ -736,16 +740,16 @@ uint32_t tmem_cols(int need) {
     return n;
 }
 
-template <int NZ, class TIn, bool VEC>
+template <int NZ, class TIn, bool VEC, class Off = int>
 tr_status launch_fwd(const TIn* x, const __nv_bfloat16* w, const float* bias, float* y, const ConvDims& c, int64_t tiles,
                      cudaStream_t st) {
-    auto fn = k_conv3d_fwd<NZ, TIn, VEC>;
+    auto fn = k_conv3d_fwd<NZ, TIn, VEC, Off>;
     const int npad = conv_npad(c.Cout);
     const size_t smem = fwd_smem_bytes(NZ, npad);
     const int nacc = 2 * NZ * npad <= 512 ? 2 : 1;
     TR_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     fn<<<(unsigned)std::min<int64_t>(tiles, sm_count()), kFwdThreads, smem, st>>>(
-        x, w, bias, y, c, (int)tiles, npad, nacc, tmem_cols(nacc * NZ * npad), at16(y), kMbarPollLimit);
+        x, w, bias, y, c, tiles, npad, nacc, tmem_cols(nacc * NZ * npad), at16(y), kMbarPollLimit);
     TR_CHECK_LAUNCH();
     return TR_OK;
 }
@@ -768,9 +772,9 @@ tr_status conv_fwd(const TIn* x, const __nv_bfloat16* packed, const float* bias,
             tiles = n;
         }
     }
-    if (tiles > INT32_MAX - sms || (int64_t)c.H * c.W > INT32_MAX / 8)
-        return tr::fail(TR_ERR_UNSUPPORTED, "conv3d: volume too large");
     const bool vec = c.Cin % 8 == 0 && at16(x);
+    if ((int64_t)c.H * c.W > INT32_MAX / 8)              // slices of more than 268 million voxels
+        return launch_fwd<1, TIn, false, int64_t>(x, packed, bias, y, c, cols * c.D, st);
 #define TR_FWD_NZ(NZV) \
     return vec ? launch_fwd<NZV, TIn, true>(x, packed, bias, y, c, tiles, st) \
                : launch_fwd<NZV, TIn, false>(x, packed, bias, y, c, tiles, st)
@@ -809,18 +813,18 @@ WgradShape wgrad_shape(const ConvDims& c, int64_t max_splits) {
     s.cx = (c.Cin + kWgChunk - 1) / kWgChunk;
     s.cg = (c.Cout + kWgChunk - 1) / kWgChunk;
     s.cols = tmem_cols(14 / s.groups * s.npad);       // two M = 64 accumulators per column range
-    s.cols_n = c.N * ((c.W + kTX - 1) / kTX) * ((c.H + kTY - 1) / kTY);
+    s.cols_n = (int64_t)c.N * ((c.W + kTX - 1) / kTX) * ((c.H + kTY - 1) / kTY);
     // one CTA per SM over all groups and chunks; z segments and splits by the slices that the busiest
     // CTA loads (two halo slices a segment)
     const int64_t want = std::max<int64_t>(1, std::min<int64_t>(max_splits, sm_count() / (s.groups * s.cx * s.cg)));
     int64_t best = INT64_MAX;
     for (int segs = 1; segs <= std::min(c.D, 64); ++segs) {
         const int len = (c.D + segs - 1) / segs;
-        const int64_t units = (int64_t)s.cols_n * ((c.D + len - 1) / len), rounds = (units + want - 1) / want;
+        const int64_t units = s.cols_n * ((c.D + len - 1) / len), rounds = (units + want - 1) / want;
         if (rounds * (len + 2) < best) {
             best = rounds * (len + 2);
             s.seg_len = len;
-            s.units = (int)units;
+            s.units = units;
             s.splits = (int)((units + rounds - 1) / rounds);
         }
     }

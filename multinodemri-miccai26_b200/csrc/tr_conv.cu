@@ -488,10 +488,14 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_conv3d_fwd(const TIn* __rest
 // a group of taps in TMEM: M = 64 channels of the wider side, N = up to 64 channels of the other;
 // an M = 64 accumulator fills half of the TMEM lanes, so two taps share a column range.
 // Warps 8-15 keep a ring of four items (x slice i, gy slice i - 2) filled, warps 0 and 2 issue
-// the MMAs of half of the taps each.  Grid: (splits of the voxel columns, tap groups, channel chunks); each CTA writes one
-// partial [27][Cin][Cout] slab piece, summed in split order by k_wgrad_reduce.
-// Measured at (4, 32, 32, 32), 64 -> 32 channels: 437 us with mma.sync (16 voxels a step gathered
-// element by element, 27 passes over the voxels) + 22 us of reduction, 52 + 9 us with these kernels.
+// the MMAs of half of the taps each.  After every run of at most kWgRunSlices slices all warps add the
+// accumulators to the CTA's partial, a [27][Cin][Cout] slab piece (in float32, one add per value and run by
+// the same thread, so in a fixed order).  Grid: (splits of the voxel columns, tap groups, channel chunks); the
+// partials are summed in split order by k_wgrad_reduce.
+// Measured, both kernels: (4, 32, 32, 32), 64 -> 32 channels: 453 us with mma.sync (16 voxels a step
+// gathered element by element, 27 passes over the voxels), 52 us with these.  (8, 32, 32, 32), 128 -> 128:
+// 4.32 ms and a relative error of 1.4e-6 with mma.sync (sums of 2,048 voxels); 290 us and 1.5e-5 with one
+// accumulator over a CTA's whole share (14,600 voxels), 367 us and 1.4e-6 with runs.
 constexpr int kWgThreads = 512;
 constexpr int kWgLoaders = 256;                        // warps 8-15
 constexpr int kWgRing = 4;
@@ -499,6 +503,9 @@ constexpr int kXPitch = plane_pitch(kSlice);          // voxels per plane of an 
 constexpr int kGPitch = plane_pitch(kTX * kTY);       // voxels per plane of a gy slice
 constexpr int kWgChunk = 64;                          // channels per CTA and side
 constexpr int kWgradVox = 2048;                       // voxels per partial that callers' scratch covers at least
+// z slices (128 voxels each) that a TMEM accumulator sums.  The tensor core's float32 sums lose about half
+// a last bit a step, all in one direction, so that the error grows with the length of a sum.
+constexpr int kWgRunSlices = kWgradVox / (kTX * kTY);
 
 struct WgradShape {
     bool mx;             // M side = x (Cin), N side = gy (Cout); else the other way round
@@ -509,6 +516,7 @@ struct WgradShape {
     uint32_t cols;
     int64_t cols_n, units;           // (image, y, x) voxel columns; z segments of all of them
     int seg_len, splits;
+    int run;                         // units whose voxels one accumulator sums
 };
 
 // Tap groups: all 27 taps' accumulators fit TMEM (two per column range) up to 32 columns each.
@@ -562,143 +570,171 @@ __global__ void __launch_bounds__(kWgThreads) k_conv3d_wgrad(const __nv_bfloat16
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
+    const int64_t stride = (int64_t)s.run * s.splits;        // units between two runs
+    float* dst = part + (int64_t)split * 27 * c.Cin * c.Cout;
     bool ok = true;
+    int item0 = 0;                        // ring items before this run
 
-    if (warp == 0 || warp == 2) {
-        if (elect_one()) {
-            const uint32_t idesc = instr_desc(64, NPAD, true);
-            const uint64_t xd = op_desc(smem_u32(sm), kHX * 16, kXPitch * 16);
-            const uint64_t gd = op_desc(smem_u32(sm) + xbytes, kTX * 16, kGPitch * 16);
-            const uint32_t slot16 = slot >> 4, xhi = (uint32_t)(xd >> 32), ghi = (uint32_t)(gd >> 32);
-            int item = 0;                 // ring items consumed so far
-            bool first = true;
-            for (int64_t u = split; u < s.units && ok; u += s.splits) {
-                const int z0 = (int)(u / s.cols_n) * s.seg_len, nz = min(s.seg_len, c.D - z0);
-                for (int k = 0; k < nz && ok; ++k) {
-                    for (int i = (k == 0 ? 0 : 2); i < 3 && ok; ++i) {
-                        const int j = item + k + i;
-                        ok = mbar_wait_bounded(&full[j % kWgRing], (j / kWgRing) & 1, poll);
+    int run = 0;
+    for (int64_t u0 = split; u0 < s.units; u0 += stride, ++run) {
+        const int64_t u1 = min(s.units, u0 + stride);
+        if (warp == 0 || warp == 2) {
+            if (elect_one()) {
+                const uint32_t idesc = instr_desc(64, NPAD, true);
+                const uint64_t xd = op_desc(smem_u32(sm), kHX * 16, kXPitch * 16);
+                const uint64_t gd = op_desc(smem_u32(sm) + xbytes, kTX * 16, kGPitch * 16);
+                const uint32_t slot16 = slot >> 4, xhi = (uint32_t)(xd >> 32), ghi = (uint32_t)(gd >> 32);
+                bool first = true;
+                int item = item0;
+                for (int64_t u = u0; u < u1 && ok; u += s.splits) {
+                    const int z0 = (int)(u / s.cols_n) * s.seg_len, nz = min(s.seg_len, c.D - z0);
+                    for (int k = 0; k < nz && ok; ++k) {
+                        for (int i = (k == 0 ? 0 : 2); i < 3 && ok; ++i) {
+                            const int j = item + k + i;
+                            ok = mbar_wait_bounded(&full[j % kWgRing], (j / kWgRing) & 1, poll);
+                        }
+                        if (!ok) break;
+                        tc_fence_after();
+                        const uint32_t xl[3] = {(uint32_t)xd + (item + k) % kWgRing * slot16,
+                                                (uint32_t)xd + (item + k + 1) % kWgRing * slot16,
+                                                (uint32_t)xd + (item + k + 2) % kWgRing * slot16};
+                        const uint32_t gl = (uint32_t)gd + (item + k + 2) % kWgRing * slot16;
+                        if (G == 1) {
+                            if (warp == 0) wgrad_mmas<NPAD, MX, 0, 0, 14>(xl, xhi, gl, ghi, tmem, idesc, first);
+                            else wgrad_mmas<NPAD, MX, 0, 14, 27>(xl, xhi, gl, ghi, tmem, idesc, first);
+                        } else if (blockIdx.y == 0) {
+                            if (warp == 0) wgrad_mmas<NPAD, MX, 0, 0, 7>(xl, xhi, gl, ghi, tmem, idesc, first);
+                            else wgrad_mmas<NPAD, MX, 0, 7, 14>(xl, xhi, gl, ghi, tmem, idesc, first);
+                        } else {
+                            if (warp == 0) wgrad_mmas<NPAD, MX, 14, 14, 21>(xl, xhi, gl, ghi, tmem, idesc, first);
+                            else wgrad_mmas<NPAD, MX, 14, 21, 27>(xl, xhi, gl, ghi, tmem, idesc, first);
+                        }
+                        first = false;
+                        mma_commit(&empty[(item + k) % kWgRing]);        // x slice k is not read again
                     }
-                    if (!ok) break;
-                    tc_fence_after();
-                    const uint32_t xl[3] = {(uint32_t)xd + (item + k) % kWgRing * slot16,
-                                            (uint32_t)xd + (item + k + 1) % kWgRing * slot16,
-                                            (uint32_t)xd + (item + k + 2) % kWgRing * slot16};
-                    const uint32_t gl = (uint32_t)gd + (item + k + 2) % kWgRing * slot16;
-                    if (G == 1) {
-                        if (warp == 0) wgrad_mmas<NPAD, MX, 0, 0, 14>(xl, xhi, gl, ghi, tmem, idesc, first);
-                        else wgrad_mmas<NPAD, MX, 0, 14, 27>(xl, xhi, gl, ghi, tmem, idesc, first);
-                    } else if (blockIdx.y == 0) {
-                        if (warp == 0) wgrad_mmas<NPAD, MX, 0, 0, 7>(xl, xhi, gl, ghi, tmem, idesc, first);
-                        else wgrad_mmas<NPAD, MX, 0, 7, 14>(xl, xhi, gl, ghi, tmem, idesc, first);
-                    } else {
-                        if (warp == 0) wgrad_mmas<NPAD, MX, 14, 14, 21>(xl, xhi, gl, ghi, tmem, idesc, first);
-                        else wgrad_mmas<NPAD, MX, 14, 21, 27>(xl, xhi, gl, ghi, tmem, idesc, first);
-                    }
-                    first = false;
-                    mma_commit(&empty[(item + k) % kWgRing]);        // x slice k is not read again
+                    for (int i = 0; i < 2; ++i) mma_commit(&empty[(item + nz + i) % kWgRing]);
+                    item += nz + 2;
                 }
-                for (int i = 0; i < 2; ++i) mma_commit(&empty[(item + nz + i) % kWgRing]);
-                item += nz + 2;
+                mma_commit(&done);
             }
-            mma_commit(&done);
-        }
-        __syncwarp();
-    } else if (warp >= 8) {
-        // ---- 16-byte pieces, consecutive lanes along a voxel's channels; a thread's pieces keep their
-        // places while the CTA marches along z
-        constexpr int kPerX = (kSlice * 8 + kWgLoaders - 1) / kWgLoaders, kPerG = kTX * kTY * 8 / kWgLoaders;
-        const int lt = tid - (kWgThreads - kWgLoaders);
-        const int nx = min(s.px, 2 * ((min(kWgChunk, c.Cin - cx0) + 15) / 16));     // planes with channels
-        const int ng = min(s.pg, 2 * ((min(kWgChunk, c.Cout - cg0) + 15) / 16));
-        const int64_t hw = (int64_t)c.H * c.W;
-        int item = 0;
-        for (int64_t u = split; u < s.units; u += s.splits) {
-            const int64_t col = u % s.cols_n;
-            const int x0 = (int)(col % ntx) * kTX, y0 = (int)((col / ntx) % nty) * kTY;
-            const int img = (int)(col / ((int64_t)ntx * nty));
-            const int z0 = (int)(u / s.cols_n) * s.seg_len, nz = min(s.seg_len, c.D - z0);
-            int64_t vx[kPerX], vg[kPerG];                          // voxel in the slice (-1: none)
-            int dx[kPerX], dg[kPerG];                              // place in the slot
-#pragma unroll
-            for (int k = 0; k < kPerX; ++k) {
-                const int v = lt + k * kWgLoaders, vox = v / nx, pl = v - vox * nx;
-                const int hy = vox / kHX, yy = y0 - 1 + hy, xx = x0 - 1 + vox - hy * kHX;
-                dx[k] = v < kSlice * nx ? (pl * kXPitch + vox) * 16 : -1;
-                vx[k] = dx[k] >= 0 && (unsigned)yy < (unsigned)c.H && (unsigned)xx < (unsigned)c.W ? (int64_t)yy * c.W + xx : -1;
-            }
-#pragma unroll
-            for (int k = 0; k < kPerG; ++k) {
-                const int v = lt + k * kWgLoaders, vox = v / ng, pl = v - vox * ng;
-                const int yy = y0 + (vox >> 3), xx = x0 + (vox & 7);
-                dg[k] = v < kTX * kTY * ng ? (pl * kGPitch + vox) * 16 : -1;
-                vg[k] = dg[k] >= 0 && yy < c.H && xx < c.W ? (int64_t)yy * c.W + xx : -1;
-            }
-            for (int i = 0; i < nz + 2; ++i, ++item) {
-                if (item >= kWgRing)
-                    ok = ok && mbar_wait_bounded(&empty[item % kWgRing], (item / kWgRing - 1) & 1, poll);
-                unsigned char* base = sm + (size_t)(item % kWgRing) * slot;
-                const int zx = z0 - 1 + i;
-                const __nv_bfloat16* xs = x + ((int64_t)img * c.D + zx) * hw * c.Cin;
-                const __nv_bfloat16* gs = gy + ((int64_t)img * c.D + zx - 1) * hw * c.Cout;
-                uint4 bx[kPerX], bg[kPerG];
+            __syncwarp();
+        } else if (warp >= 8) {
+            // ---- 16-byte pieces, consecutive lanes along a voxel's channels; a thread's pieces keep their
+            // places while the CTA marches along z
+            constexpr int kPerX = (kSlice * 8 + kWgLoaders - 1) / kWgLoaders, kPerG = kTX * kTY * 8 / kWgLoaders;
+            const int lt = tid - (kWgThreads - kWgLoaders);
+            const int nx = min(s.px, 2 * ((min(kWgChunk, c.Cin - cx0) + 15) / 16));     // planes with channels
+            const int ng = min(s.pg, 2 * ((min(kWgChunk, c.Cout - cg0) + 15) / 16));
+            const int64_t hw = (int64_t)c.H * c.W;
+            int item = item0;
+            for (int64_t u = u0; u < u1; u += s.splits) {
+                const int64_t col = u % s.cols_n;
+                const int x0 = (int)(col % ntx) * kTX, y0 = (int)((col / ntx) % nty) * kTY;
+                const int img = (int)(col / ((int64_t)ntx * nty));
+                const int64_t corner = (int64_t)y0 * c.W + x0;     // of the tile in its slice
+                const int z0 = (int)(u / s.cols_n) * s.seg_len, nz = min(s.seg_len, c.D - z0);
+                int vx[kPerX], vg[kPerG], dx[kPerX], dg[kPerG];    // row, column in the tile (-1: none); place in the slot
 #pragma unroll
                 for (int k = 0; k < kPerX; ++k) {
-                    const int ch = cx0 + (dx[k] / (kXPitch * 16)) * 8;
-                    bx[k] = make_uint4(0, 0, 0, 0);
-                    if (vx[k] >= 0 && (unsigned)zx < (unsigned)c.D)
-                        bx[k] = load8<XVEC>(xs + vx[k] * c.Cin, ch, c.Cin, at4(x));
+                    const int v = lt + k * kWgLoaders, vox = v / nx, pl = v - vox * nx;
+                    const int hy = vox / kHX, hx = vox - hy * kHX, yy = y0 - 1 + hy, xx = x0 - 1 + hx;
+                    dx[k] = v < kSlice * nx ? (pl * kXPitch + vox) * 16 : -1;
+                    vx[k] = dx[k] >= 0 && (unsigned)yy < (unsigned)c.H && (unsigned)xx < (unsigned)c.W ? hy * 16 + hx : -1;
                 }
-                if (i >= 2) {
 #pragma unroll
-                    for (int k = 0; k < kPerG; ++k) {
-                        const int ch = cg0 + (dg[k] / (kGPitch * 16)) * 8;
-                        bg[k] = make_uint4(0, 0, 0, 0);
-                        if (vg[k] >= 0)
-                            bg[k] = at16(gy) ? load8<true>(gs + vg[k] * c.Cout, ch, c.Cout, true)
-                                             : load8<false>(gs + vg[k] * c.Cout, ch, c.Cout, at4(gy));
+                for (int k = 0; k < kPerG; ++k) {
+                    const int v = lt + k * kWgLoaders, vox = v / ng, pl = v - vox * ng;
+                    dg[k] = v < kTX * kTY * ng ? (pl * kGPitch + vox) * 16 : -1;
+                    vg[k] = dg[k] >= 0 && y0 + (vox >> 3) < c.H && x0 + (vox & 7) < c.W ? vox : -1;
+                }
+                for (int i = 0; i < nz + 2; ++i, ++item) {
+                    if (item >= kWgRing)
+                        ok = ok && mbar_wait_bounded(&empty[item % kWgRing], (item / kWgRing - 1) & 1, poll);
+                    unsigned char* base = sm + (size_t)(item % kWgRing) * slot;
+                    const int zx = z0 - 1 + i;
+                    const __nv_bfloat16* xs = x + (((int64_t)img * c.D + zx) * hw + corner - c.W - 1) * c.Cin;
+                    const __nv_bfloat16* gs = gy + (((int64_t)img * c.D + zx - 1) * hw + corner) * c.Cout;
+                    uint4 bx[kPerX], bg[kPerG];
+#pragma unroll
+                    for (int k = 0; k < kPerX; ++k) {
+                        const int ch = cx0 + (dx[k] / (kXPitch * 16)) * 8;
+                        bx[k] = make_uint4(0, 0, 0, 0);
+                        if (vx[k] >= 0 && (unsigned)zx < (unsigned)c.D)
+                            bx[k] = load8<XVEC>(xs + ((int64_t)(vx[k] >> 4) * c.W + (vx[k] & 15)) * c.Cin, ch, c.Cin, at4(x));
+                    }
+                    if (i >= 2) {
+#pragma unroll
+                        for (int k = 0; k < kPerG; ++k) {
+                            const int ch = cg0 + (dg[k] / (kGPitch * 16)) * 8;
+                            bg[k] = make_uint4(0, 0, 0, 0);
+                            const __nv_bfloat16* gv = gs + ((int64_t)(vg[k] >> 3) * c.W + (vg[k] & 7)) * c.Cout;
+                            if (vg[k] >= 0)
+                                bg[k] = at16(gy) ? load8<true>(gv, ch, c.Cout, true)
+                                                 : load8<false>(gv, ch, c.Cout, at4(gy));
+                        }
+                    }
+#pragma unroll
+                    for (int k = 0; k < kPerX; ++k)
+                        if (dx[k] >= 0) *reinterpret_cast<uint4*>(base + dx[k]) = bx[k];
+                    if (i >= 2) {
+#pragma unroll
+                        for (int k = 0; k < kPerG; ++k)
+                            if (dg[k] >= 0) *reinterpret_cast<uint4*>(base + xbytes + dg[k]) = bg[k];
+                    }
+                    tr::fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&full[item % kWgRing]);
+                }
+            }
+        }
+        for (int64_t u = u0; u < u1; u += s.splits) item0 += min(s.seg_len, c.D - (int)(u / s.cols_n) * s.seg_len) + 2;
+        if (tid == 0) ok = ok && mbar_wait_bounded(&done, run & 1, poll);
+        const bool bad = __syncthreads_or(!ok) != 0;
+        tc_fence_after();
+        // ---- part[split][t][ci][co]: lanes 0-15 hold an even accumulator's rows, lanes 16-31 the odd one's
+        const int q = warp & 3;
+        const int nN = MX ? min(kWgChunk, c.Cout - cg0) : min(kWgChunk, c.Cin - cx0);
+        const int nM = MX ? min(kWgChunk, c.Cin - cx0) : min(kWgChunk, c.Cout - cg0);
+        float* stage = reinterpret_cast<float*>(sm) + warp * 32 * kEpPitch;      // the ring is idle
+        for (int a2 = warp >> 2; 2 * a2 < t1 - t0; a2 += kWgThreads / 128) {
+            for (int n0 = 0; n0 < nN; n0 += 32) {
+                const int nc = min(32, NPAD - n0);
+                tmem_to_rows(tmem + ((uint32_t)(q * 32) << 16) + a2 * NPAD + n0, nc, stage + lane * kEpPitch);
+                __syncwarp();
+                // four output channels a lane, consecutive lanes along them: the columns (MX) or the rows of a half-warp
+                for (int i = lane; i < 8 * nc; i += 32) {
+                    const int r = MX ? i / (nc / 4) : (i & 7) * 4, k = MX ? i % (nc / 4) * 4 : i >> 3;
+                    const int t = t0 + 2 * a2 + (r >> 4), row = q * 16 + (r & 15);
+                    if (t >= t1 || row >= nM || n0 + k >= nN) continue;
+                    const int ci = MX ? cx0 + row : cx0 + n0 + k, co = MX ? cg0 + n0 + k : cg0 + row;
+                    const float* v = stage + r * kEpPitch + k;
+                    constexpr int step = MX ? 1 : kEpPitch;
+                    float4 f = make_float4(v[0], v[step], v[2 * step], v[3 * step]);
+                    if (bad) f.x = f.y = f.z = f.w = __int_as_float(0x7fffffff);
+                    float* d = dst + ((int64_t)t * c.Cin + ci) * c.Cout + co;
+                    const bool add = run > 0 && !bad;              // to this thread's own values: nothing is read back
+                    if (at16(part)) {
+                        if (add) atomicAdd(reinterpret_cast<float4*>(d), f);
+                        else *reinterpret_cast<float4*>(d) = f;
+                    } else {
+                        const float g[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            if (add) atomicAdd(d + e, g[e]);
+                            else d[e] = g[e];
                     }
                 }
-#pragma unroll
-                for (int k = 0; k < kPerX; ++k)
-                    if (dx[k] >= 0) *reinterpret_cast<uint4*>(base + dx[k]) = bx[k];
-                if (i >= 2) {
-#pragma unroll
-                    for (int k = 0; k < kPerG; ++k)
-                        if (dg[k] >= 0) *reinterpret_cast<uint4*>(base + xbytes + dg[k]) = bg[k];
-                }
-                tr::fence_proxy_async_smem();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&full[item % kWgRing]);
             }
         }
-    }
-    if (tid == 0) ok = ok && mbar_wait_bounded(&done, 0, poll);
-    const bool bad = __syncthreads_or(!ok) != 0;
-    tc_fence_after();
-    // ---- part[split][t][ci][co]: lanes 0-15 hold an even accumulator's rows, lanes 16-31 the odd one's
-    const int q = warp & 3;
-    const int nN = MX ? min(kWgChunk, c.Cout - cg0) : min(kWgChunk, c.Cin - cx0);
-    const int nM = MX ? min(kWgChunk, c.Cin - cx0) : min(kWgChunk, c.Cout - cg0);
-    float* dst = part + (int64_t)split * 27 * c.Cin * c.Cout;
-    float* stage = reinterpret_cast<float*>(sm) + warp * 32 * kEpPitch;      // the ring is idle
-    for (int a2 = warp >> 2; 2 * a2 < t1 - t0; a2 += kWgThreads / 128) {
-        for (int n0 = 0; n0 < nN; n0 += 32) {
-            const int nc = min(32, NPAD - n0);
-            tmem_to_rows(tmem + ((uint32_t)(q * 32) << 16) + a2 * NPAD + n0, nc, stage + lane * kEpPitch);
-            __syncwarp();
-            // consecutive lanes write consecutive output channels: the columns (MX) or the rows of a half-warp
-            for (int i = lane; i < 32 * nc; i += 32) {
-                const int r = MX ? i / nc : i & 31, k = MX ? i % nc : i >> 5;
-                const int t = t0 + 2 * a2 + (r >> 4), row = q * 16 + (r & 15);
-                if (t >= t1 || row >= nM || n0 + k >= nN) continue;
-                const int ci = MX ? cx0 + row : cx0 + n0 + k, co = MX ? cg0 + n0 + k : cg0 + row;
-                dst[((int64_t)t * c.Cin + ci) * c.Cout + co] = bad ? __int_as_float(0x7fffffff) : stage[r * kEpPitch + k];
-            }
-            __syncwarp();
+        if (bad) {
+            if (tid == 0) mbar_wait_bounded(&done, run & 1, poll);
+            break;
         }
+        tc_fence_before();
+        __syncthreads();                      // accumulators and ring are free for the next run
+        tc_fence_after();
     }
-    if (bad && tid == 0) mbar_wait_bounded(&done, 0, poll);
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_free(tmem, s.cols);
@@ -815,15 +851,18 @@ WgradShape wgrad_shape(const ConvDims& c, int64_t max_splits) {
     s.cols = tmem_cols(14 / s.groups * s.npad);       // two M = 64 accumulators per column range
     s.cols_n = (int64_t)c.N * ((c.W + kTX - 1) / kTX) * ((c.H + kTY - 1) / kTY);
     // one CTA per SM over all groups and chunks; z segments and splits by the slices that the busiest
-    // CTA loads (two halo slices a segment)
+    // CTA loads (two halo slices a segment; adding a run's accumulators to the partial takes about four)
     const int64_t want = std::max<int64_t>(1, std::min<int64_t>(max_splits, sm_count() / (s.groups * s.cx * s.cg)));
     int64_t best = INT64_MAX;
-    for (int segs = 1; segs <= std::min(c.D, 64); ++segs) {
-        const int len = (c.D + segs - 1) / segs;
+    const int fewest = (c.D + kWgRunSlices - 1) / kWgRunSlices;
+    for (int segs = fewest; segs <= std::max(fewest, std::min(c.D, 64)); ++segs) {
+        const int len = (c.D + segs - 1) / segs, run = kWgRunSlices / len;
         const int64_t units = s.cols_n * ((c.D + len - 1) / len), rounds = (units + want - 1) / want;
-        if (rounds * (len + 2) < best) {
-            best = rounds * (len + 2);
+        const int64_t cost = rounds * (len + 2) + (rounds + run - 1) / run * 4;
+        if (cost < best) {
+            best = cost;
             s.seg_len = len;
+            s.run = run;
             s.units = units;
             s.splits = (int)((units + rounds - 1) / rounds);
         }

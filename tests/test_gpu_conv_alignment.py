@@ -79,3 +79,22 @@ def test_strided_weights(cin, cout):
         c = v.contiguous()
         assert torch.equal(ws.conv3d_dgrad_bf16(gy, v), ws.conv3d_dgrad_bf16(gy, c))
         assert torch.equal(ws.conv3d_fwd_bf16(x, v), ws.conv3d_fwd_bf16(x, c))
+
+
+def test_weight_gradient_with_unaligned_scratch():
+    torch = _torch()
+    ws, lib = pkg("warmstart"), pkg("_lib")
+    shape, cin, cout = (1, 300, 32, 32), 64, 64                 # several runs a thread block
+    x = torch.randn(shape + (cin,), device="cuda").bfloat16()
+    gy = torch.randn(shape + (cout,), device="cuda").bfloat16()
+    ref = ws.conv3d_wgrad_bf16(x, gy)
+    nbytes = ctypes.c_size_t(0)
+    lib.check(lib.load().tr_conv3d_wgrad_workspace(*shape, cin, cout, ctypes.byref(nbytes)))
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    for offset in (0, 1, 2):
+        scratch = torch.empty(nbytes.value // 4 + 8, device="cuda")[offset:]
+        buf = torch.zeros(ref.numel() + 4, device="cuda")
+        dw = buf[offset:offset + ref.numel()]
+        lib.check(lib.load().tr_conv3d_wgrad(_ptr(x), _ptr(gy), _ptr(dw), *shape, cin, cout, _ptr(scratch),
+                                             nbytes, stream))
+        assert torch.equal(dw.view(ref.shape), ref)

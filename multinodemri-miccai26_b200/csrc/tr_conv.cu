@@ -540,8 +540,55 @@ __device__ __forceinline__ void wgrad_mmas(const uint32_t (&xl)[3], uint32_t xhi
     }
 }
 
-// XVEC: x is copied 16 bytes at a time; MX: the M side is x (else gy); NPAD: columns per tap.
-template <int NPAD, bool XVEC, bool MX>
+// Infinite and NaN values in the last x or y of the volume, where a tile reaches past it: the tile's voxels
+// outside the volume have gy = 0, and for taps towards smaller x or y the MMAs multiply that zero with the
+// last voxels' x, which must not turn a finite sum into NaN.  The loaders put zeros for such values (finite8),
+// and a CTA that met some adds their products with the tile's own voxels here.
+__device__ __forceinline__ uint4 finite8(uint4 v, int* seen) {
+    uint32_t* r = &v.x;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t m = __vcmpeq2(r[i] & 0x7f807f80u, 0x7f807f80u);
+        r[i] &= ~m;
+        if (m) *seen = 1;
+    }
+    return v;
+}
+__device__ __forceinline__ void wgrad_add_nonfinite(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gy,
+                                                 float* __restrict__ dst, const ConvDims& c, const WgradShape& s, int t0,
+                                                 int t1, int cx0, int cg0) {
+    const int nx = min(kWgChunk, c.Cin - cx0), ng = min(kWgChunk, c.Cout - cg0);
+    const int ntx = (c.W + kTX - 1) / kTX, nty = (c.H + kTY - 1) / kTY;
+    for (int e = threadIdx.x; e < (t1 - t0) * nx * ng; e += kWgThreads) {
+        const int co = cg0 + e % ng, ci = cx0 + e / ng % nx, t = t0 + e / ng / nx;
+        const int dz = t / 9 - 1, dy = t / 3 % 3 - 1, dx = t % 3 - 1;
+        float sum = 0.f;
+        bool any = false;
+        for (int64_t u = blockIdx.x; u < s.units; u += s.splits) {
+            const int64_t col = u % s.cols_n;
+            const int x0 = (int)(col % ntx) * kTX, y0 = (int)((col / ntx) % nty) * kTY;
+            const bool ex = x0 + kTX > c.W, ey = y0 + kTY > c.H;
+            if (!ex && !ey) continue;
+            const int64_t img = col / ((int64_t)ntx * nty);
+            const int z0 = (int)(u / s.cols_n) * s.seg_len, z1 = min(z0 + s.seg_len, c.D);
+            for (int z = max(z0, -dz); z < min(z1, c.D - dz); ++z)
+                for (int y = max(y0, -dy); y < min(y0 + kTY, c.H - max(dy, 0)); ++y)
+                    for (int xx = max(x0, -dx); xx < min(x0 + kTX, c.W - max(dx, 0)); ++xx) {
+                        if (!(ex && xx + dx == c.W - 1) && !(ey && y + dy == c.H - 1)) continue;
+                        const int64_t v = ((img * c.D + z) * c.H + y) * c.W + xx;
+                        const float f = __bfloat162float(x[(v + ((int64_t)dz * c.H + dy) * c.W + dx) * c.Cin + ci]);
+                        if (isfinite(f)) continue;
+                        sum += f * __bfloat162float(gy[v * c.Cout + co]);
+                        any = true;
+                    }
+        }
+        if (any) atomicAdd(dst + ((int64_t)t * c.Cin + ci) * c.Cout + co, sum);
+    }
+}
+
+// XVEC: x is copied 16 bytes at a time; MX: the M side is x (else gy); NPAD: columns per tap; TAIL: some tiles
+// reach past the volume (the checks for infinite x cost 7 % at 64 channels on both sides).
+template <int NPAD, bool XVEC, bool MX, bool TAIL>
 __global__ void __launch_bounds__(kWgThreads) k_conv3d_wgrad(const __nv_bfloat16* __restrict__ x,
                                                              const __nv_bfloat16* __restrict__ gy,
                                                              float* __restrict__ part, ConvDims c, WgradShape s,
@@ -549,6 +596,7 @@ __global__ void __launch_bounds__(kWgThreads) k_conv3d_wgrad(const __nv_bfloat16
     extern __shared__ __align__(128) unsigned char smraw_[];
     __shared__ __align__(8) uint64_t full[kWgRing], empty[kWgRing], done;
     __shared__ uint32_t tmem_slot;
+    __shared__ int nonfinite;                                // some x was left out (finite8)
     unsigned char* sm = smraw_ + ((128 - (smem_u32(smraw_) & 127)) & 127);
     const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     const int split = blockIdx.x;
@@ -565,6 +613,7 @@ __global__ void __launch_bounds__(kWgThreads) k_conv3d_wgrad(const __nv_bfloat16
             mbar_init(&empty[i], 2);
         }
         mbar_init(&done, 2);
+        nonfinite = 0;
     }
     tc_fence_before();
     __syncthreads();
@@ -634,12 +683,14 @@ __global__ void __launch_bounds__(kWgThreads) k_conv3d_wgrad(const __nv_bfloat16
                 const int64_t corner = (int64_t)y0 * c.W + x0;     // of the tile in its slice
                 const int z0 = (int)(u / s.cols_n) * s.seg_len, nz = min(s.seg_len, c.D - z0);
                 int vx[kPerX], vg[kPerG], dx[kPerX], dg[kPerG];    // row, column in the tile (-1: none); place in the slot
+                constexpr int kEdge = 512;                         // added to vx: last x or y, beside voxels outside
 #pragma unroll
                 for (int k = 0; k < kPerX; ++k) {
                     const int v = lt + k * kWgLoaders, vox = v / nx, pl = v - vox * nx;
                     const int hy = vox / kHX, hx = vox - hy * kHX, yy = y0 - 1 + hy, xx = x0 - 1 + hx;
                     dx[k] = v < kSlice * nx ? (pl * kXPitch + vox) * 16 : -1;
                     vx[k] = dx[k] >= 0 && (unsigned)yy < (unsigned)c.H && (unsigned)xx < (unsigned)c.W ? hy * 16 + hx : -1;
+                    if (TAIL && vx[k] >= 0 && ((xx == c.W - 1 && x0 + kTX > c.W) || (yy == c.H - 1 && y0 + kTY > c.H))) vx[k] |= kEdge;
                 }
 #pragma unroll
                 for (int k = 0; k < kPerG; ++k) {
@@ -660,7 +711,7 @@ __global__ void __launch_bounds__(kWgThreads) k_conv3d_wgrad(const __nv_bfloat16
                         const int ch = cx0 + (dx[k] / (kXPitch * 16)) * 8;
                         bx[k] = make_uint4(0, 0, 0, 0);
                         if (vx[k] >= 0 && (unsigned)zx < (unsigned)c.D)
-                            bx[k] = load8<XVEC>(xs + ((int64_t)(vx[k] >> 4) * c.W + (vx[k] & 15)) * c.Cin, ch, c.Cin, at4(x));
+                            bx[k] = load8<XVEC>(xs + ((int64_t)(vx[k] >> 4 & 31) * c.W + (vx[k] & 15)) * c.Cin, ch, c.Cin, at4(x));
                     }
                     if (i >= 2) {
 #pragma unroll
@@ -675,7 +726,8 @@ __global__ void __launch_bounds__(kWgThreads) k_conv3d_wgrad(const __nv_bfloat16
                     }
 #pragma unroll
                     for (int k = 0; k < kPerX; ++k)
-                        if (dx[k] >= 0) *reinterpret_cast<uint4*>(base + dx[k]) = bx[k];
+                        if (dx[k] >= 0)
+                            *reinterpret_cast<uint4*>(base + dx[k]) = TAIL && vx[k] >= kEdge ? finite8(bx[k], &nonfinite) : bx[k];
                     if (i >= 2) {
 #pragma unroll
                         for (int k = 0; k < kPerG; ++k)
@@ -735,6 +787,8 @@ __global__ void __launch_bounds__(kWgThreads) k_conv3d_wgrad(const __nv_bfloat16
         __syncthreads();                      // accumulators and ring are free for the next run
         tc_fence_after();
     }
+    if (TAIL) __syncthreads();
+    if (TAIL && nonfinite) wgrad_add_nonfinite(x, gy, dst, c, s, t0, t1, cx0, cg0);
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_free(tmem, s.cols);
@@ -871,10 +925,17 @@ WgradShape wgrad_shape(const ConvDims& c, int64_t max_splits) {
 }
 
 using WgradKernel = void (*)(const __nv_bfloat16*, const __nv_bfloat16*, float*, ConvDims, WgradShape, int);
-template <int NPAD>
+template <int NPAD, bool TAIL>
 WgradKernel wgrad_kernel(bool vec, bool mx) {
-    return vec ? (mx ? k_conv3d_wgrad<NPAD, true, true> : k_conv3d_wgrad<NPAD, true, false>)
-               : (mx ? k_conv3d_wgrad<NPAD, false, true> : k_conv3d_wgrad<NPAD, false, false>);
+    return vec ? (mx ? k_conv3d_wgrad<NPAD, true, true, TAIL> : k_conv3d_wgrad<NPAD, true, false, TAIL>)
+               : (mx ? k_conv3d_wgrad<NPAD, false, true, TAIL> : k_conv3d_wgrad<NPAD, false, false, TAIL>);
+}
+template <bool TAIL>
+WgradKernel wgrad_kernel(int npad, bool vec, bool mx) {
+    if (npad == 16) return wgrad_kernel<16, TAIL>(vec, mx);
+    if (npad == 32) return wgrad_kernel<32, TAIL>(vec, mx);
+    if (npad == 48) return wgrad_kernel<48, TAIL>(vec, mx);
+    return wgrad_kernel<64, TAIL>(vec, mx);
 }
 
 int64_t partial_floats(const ConvDims& c) { return 27LL * c.Cin * c.Cout; }
@@ -949,10 +1010,8 @@ extern "C" tr_status tr_conv3d_wgrad(const void* x, const void* gy, float* dw, i
     float* part = (float*)workspace;
     const size_t smem = (size_t)kWgRing * 16 * (s.px * kXPitch + s.pg * kGPitch) + 128;
     const bool vec = c.Cin % 8 == 0 && at16(x);
-    auto fn = wgrad_kernel<16>(vec, s.mx);
-    if (s.npad == 32) fn = wgrad_kernel<32>(vec, s.mx);
-    else if (s.npad == 48) fn = wgrad_kernel<48>(vec, s.mx);
-    else if (s.npad == 64) fn = wgrad_kernel<64>(vec, s.mx);
+    const bool tail = c.W % kTX || c.H % kTY;
+    auto fn = tail ? wgrad_kernel<true>(s.npad, vec, s.mx) : wgrad_kernel<false>(s.npad, vec, s.mx);
     TR_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const dim3 grid((unsigned)s.splits, (unsigned)s.groups, (unsigned)(s.cx * s.cg));
     fn<<<grid, kWgThreads, smem, st>>>(xb, gb, part, c, s, kMbarPollLimit);

@@ -837,7 +837,7 @@ tr_status launch_fwd(const TIn* x, const __nv_bfloat16* w, const float* bias, fl
     const int npad = conv_npad(c.Cout);
     const size_t smem = fwd_smem_bytes(NZ, npad);
     const int nacc = 2 * NZ * npad <= 512 ? 2 : 1;
-    TR_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    TR_TRY(tr::raise_smem_limit((const void*)fn, smem));
     fn<<<(unsigned)std::min<int64_t>(tiles, sm_count()), kFwdThreads, smem, st>>>(
         x, w, bias, y, c, tiles, npad, nacc, tmem_cols(nacc * NZ * npad), at16(y), kMbarPollLimit);
     TR_CHECK_LAUNCH();
@@ -1012,7 +1012,7 @@ extern "C" tr_status tr_conv3d_wgrad(const void* x, const void* gy, float* dw, i
     const bool vec = c.Cin % 8 == 0 && at16(x);
     const bool tail = c.W % kTX || c.H % kTY;
     auto fn = tail ? wgrad_kernel<true>(s.npad, vec, s.mx) : wgrad_kernel<false>(s.npad, vec, s.mx);
-    TR_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    TR_TRY(tr::raise_smem_limit((const void*)fn, smem));
     const dim3 grid((unsigned)s.splits, (unsigned)s.groups, (unsigned)(s.cx * s.cg));
     fn<<<grid, kWgThreads, smem, st>>>(xb, gb, part, c, s, kMbarPollLimit);
     TR_CHECK_LAUNCH();

@@ -242,6 +242,11 @@ namespace tr {
 // cuTensorMapEncodeTiled from the driver, looked up once (no libcuda link); null if it is missing.
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder();
 
+// Lets kernel fn use `bytes` of dynamic shared memory on the current device.  The limit is an attribute of the
+// kernel, shared by all plans and threads, so it is only ever raised: a launch that another thread prepares
+// with more shared memory stays valid.
+tr_status raise_smem_limit(const void* fn, size_t bytes);
+
 tr_status ensure_nufft_buffers(tr_plan* p, size_t ncol);
 tr_status nufft_forward_cols(tr_plan* p, int bin, const float2* images, int64_t img_stride, int n_img,
                              const float2* maps, int C, int mode, float sigma, const float2* y,

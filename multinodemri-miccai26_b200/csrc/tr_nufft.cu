@@ -27,11 +27,13 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <numeric>
 #include <string>
 #include <thread>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "tr_fft.cuh"
@@ -1680,8 +1682,18 @@ static bool factor_radices(int L, int* radix, int* nstages) {
 
 static size_t fft_smem_bytes(int L, int W) { return (size_t)(2 * L * W + L) * sizeof(float2); }
 
-static tr_status set_smem_limit(const void* fn, size_t bytes) {
-    if (bytes > 48 * 1024) TR_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+tr_status raise_smem_limit(const void* fn, size_t bytes) {
+    if (bytes <= 48 * 1024) return TR_OK;             // every kernel's limit to begin with
+    static std::mutex m;
+    static std::map<std::pair<int, const void*>, size_t> limits;      // per device
+    int dev = 0;
+    TR_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(m);
+    size_t& limit = limits[{dev, fn}];
+    if (bytes > limit) {
+        TR_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+        limit = bytes;
+    }
     return TR_OK;
 }
 
@@ -1813,7 +1825,7 @@ static tr_status launch_line(tr_plan* p, int axis, const float2* in, float2* out
         const LineKernels& lk = line_kernels(A.L);
         if (lk.fwd) {
             const void* lfn = inv ? lk.inv : lk.fwd;
-            TR_TRY(set_smem_limit(lfn, lk.smem));
+            TR_TRY(raise_smem_limit(lfn, lk.smem));
             void* args[] = {&la};
             TR_CUDA(cudaLaunchKernel(lfn, dim3((unsigned)((inner + kLineW - 1) / kLineW), (unsigned)outer),
                                      dim3((unsigned)lk.threads), args, lk.smem, st));
@@ -1833,7 +1845,7 @@ static tr_status launch_line(tr_plan* p, int axis, const float2* in, float2* out
     la.vec16 = ((inner % 2) == 0 && (la.W % 2) == 0 && ((uintptr_t)in % 16) == 0) ? 1 : 0;
     const size_t smem = tma ? line_tma_smem_bytes(A.L, la.W) : fft_smem_bytes(A.L, la.W);
     dim3 grid((unsigned)((inner + la.W - 1) / la.W), (unsigned)outer);
-    TR_TRY(set_smem_limit(fn, smem));
+    TR_TRY(raise_smem_limit(fn, smem));
     if (tma) {
         void* args[] = {&la, &tin, &tout};
         TR_CUDA(cudaLaunchKernel(fn, grid, dim3(nt), args, smem, st));
@@ -1916,7 +1928,7 @@ static tr_status stage_fwd_x(tr_plan* p, const float2* images, int64_t img_strid
         }
         if (ok && tfn) {
             const size_t smem = fft_smem_bytes(OSX, wt) + 128;
-            TR_TRY(set_smem_limit(tfn, smem));
+            TR_TRY(raise_smem_limit(tfn, smem));
             dim3 grid((unsigned)(nrows * n_img), 1u, (unsigned)(C / wt));
             void* args[] = {&fa, &timg, &tmap, &tout};
             TR_CUDA(cudaLaunchKernel(tfn, grid, dim3(nt), args, smem, st));
@@ -1927,7 +1939,7 @@ static tr_status stage_fwd_x(tr_plan* p, const float2* images, int64_t img_strid
     if (lk.fwd_x) {
         const int64_t q = (int64_t)Z * Y * C;
         const size_t smem = lk.smem + lp_row_bytes(X, C, n_img);
-        TR_TRY(set_smem_limit(lk.fwd_x, smem));
+        TR_TRY(raise_smem_limit(lk.fwd_x, smem));
         void* args[] = {&fa};
         TR_CUDA(cudaLaunchKernel(lk.fwd_x, dim3((unsigned)((q + kLineW - 1) / kLineW)), dim3((unsigned)lk.threads), args, smem,
                                  st));
@@ -1940,7 +1952,7 @@ static tr_status stage_fwd_x(tr_plan* p, const float2* images, int64_t img_strid
     // the n_img CTAs of one row block are adjacent, so the coil-map rows they share come from L2
     dim3 grid((unsigned)(((Z * Y + fa.rows - 1) / fa.rows) * n_img), 1u, (unsigned)((C + fa.cc - 1) / fa.cc));
     const void* fn = (const void*)k_fwd_x;
-    TR_TRY(set_smem_limit(fn, smem));
+    TR_TRY(raise_smem_limit(fn, smem));
     void* args[] = {&fa};
     TR_CUDA(cudaLaunchKernel(fn, grid, dim3(256), args, smem, st));
     return TR_OK;
@@ -2003,7 +2015,7 @@ static tr_status stage_yz(tr_plan* p, int ncol, bool adj, cudaStream_t st, bool*
         !encode_map_4d(&tgrid, p->bufA, grid_dims, grid_str, grid_box))
         return TR_OK;
     const size_t smem = yz_smem_bytes(OSY, OSZ, ZR);
-    TR_TRY(set_smem_limit(fn, smem));
+    TR_TRY(raise_smem_limit(fn, smem));
     if (CL > 8) TR_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)((int64_t)OSX * (ncol / kYzCW) * CL));
@@ -2137,7 +2149,7 @@ static tr_status launch_spread_t(const SpreadArgs& sa, const CUtensorMap& tgrid,
                                  cudaStream_t st) {
     const size_t smem = (size_t)2 * kSpreadSub * sa.cchunk * sizeof(float2) + 128;
     const void* fn = (const void*)k_spread<CG, TMA>;
-    TR_TRY(set_smem_limit(fn, smem));
+    TR_TRY(raise_smem_limit(fn, smem));
     SpreadArgs args_copy = sa;
     CUtensorMap map_copy = tgrid;
     void* args[] = {&args_copy, &map_copy};
@@ -2300,7 +2312,7 @@ static tr_status stage_adj_x(tr_plan* p, int n_img, const float2* maps, int C, f
         if (tfn && encode_map_3d(&tin, p->bufA, (uint64_t)aa.ncol, (uint64_t)OSX, (uint64_t)Z * Y, (uint32_t)wt,
                                  (uint32_t)(OSX / 2))) {
             const size_t smem = fft_smem_bytes(OSX, wt) + 128;
-            TR_TRY(set_smem_limit(tfn, smem));
+            TR_TRY(raise_smem_limit(tfn, smem));
             dim3 grid((unsigned)((int64_t)Z * Y * n_img));
             void* args[] = {&aa, &tin};
             TR_CUDA(cudaLaunchKernel(tfn, grid, dim3(nt), args, smem, st));
@@ -2310,7 +2322,7 @@ static tr_status stage_adj_x(tr_plan* p, int n_img, const float2* maps, int C, f
     const LineKernels& lk = line_kernels(OSX);
     if (lk.adj_x) {
         const int64_t rows = (int64_t)Z * Y, per = C >= kLineW ? 1 : kLineW / C;
-        TR_TRY(set_smem_limit(lk.adj_x, lk.smem));
+        TR_TRY(raise_smem_limit(lk.adj_x, lk.smem));
         void* args[] = {&aa};
         TR_CUDA(cudaLaunchKernel(lk.adj_x, dim3((unsigned)((rows + per - 1) / per)), dim3((unsigned)lk.threads), args,
                                  lk.smem, st));
@@ -2322,7 +2334,7 @@ static tr_status stage_adj_x(tr_plan* p, int n_img, const float2* maps, int C, f
     const size_t smem = fft_smem_bytes(OSX, W) + (size_t)aa.rows * X * sizeof(float2);
     dim3 grid((unsigned)(((Z * Y + aa.rows - 1) / aa.rows) * n_img));
     const void* fn = (const void*)k_adj_x;
-    TR_TRY(set_smem_limit(fn, smem));
+    TR_TRY(raise_smem_limit(fn, smem));
     void* args[] = {&aa};
     TR_CUDA(cudaLaunchKernel(fn, grid, dim3(256), args, smem, st));
     return TR_OK;

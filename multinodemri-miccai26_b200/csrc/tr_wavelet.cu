@@ -497,7 +497,7 @@ tr_status wavelet_dual(tr_plan* p, const float2* u_bar, float2* p_w2, float sigm
         a.lam = lam;
         a.f = w->f;
         const size_t smem = dwt_yx_smem(si[2]);
-        TR_CUDA(cudaFuncSetAttribute(k_dwt_yx, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(smem, 48 * 1024)));
+        TR_TRY(raise_smem_limit((const void*)k_dwt_yx, smem));
         k_dwt_yx<<<slice_grid((so[1] + kDwtRows - 1) / kDwtRows, (int64_t)nimg * 2 * so[0]), slice_threads(si[2]), smem, st>>>(a);
         TR_CHECK_LAUNCH();
         cur = a.next;
@@ -534,7 +534,7 @@ tr_status wavelet_adjoint(tr_plan* p, const float2* p_w2, float2* out, cudaStrea
         const bool tall = idwt_yx_smem(32, so[2]) <= 100 * 1024;
         const size_t smem = idwt_yx_smem(tall ? 32 : 16, so[2]);
         auto fn = tall ? k_idwt_yx<32> : k_idwt_yx<16>;
-        TR_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(smem, 48 * 1024)));
+        TR_TRY(raise_smem_limit((const void*)fn, smem));
         fn<<<slice_grid((si[1] + (tall ? 31 : 15)) / (tall ? 32 : 16), (int64_t)nimg * 2 * so[0]), slice_threads(2 * so[2]),
              smem, st>>>(a);
         TR_CHECK_LAUNCH();

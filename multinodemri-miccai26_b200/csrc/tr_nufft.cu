@@ -1683,13 +1683,18 @@ static bool factor_radices(int L, int* radix, int* nstages) {
 static size_t fft_smem_bytes(int L, int W) { return (size_t)(2 * L * W + L) * sizeof(float2); }
 
 tr_status raise_smem_limit(const void* fn, size_t bytes) {
-    if (bytes <= 48 * 1024) return TR_OK;             // every kernel's limit to begin with
+    if (bytes <= 32 * 1024) return TR_OK;             // below every kernel's limit to begin with
     static std::mutex m;
     static std::map<std::pair<int, const void*>, size_t> limits;      // per device
     int dev = 0;
     TR_CUDA(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lock(m);
     size_t& limit = limits[{dev, fn}];
+    if (limit == 0) {                                 // to begin with, 48 KB less the kernel's static shared memory
+        cudaFuncAttributes attr;
+        TR_CUDA(cudaFuncGetAttributes(&attr, fn));
+        limit = (size_t)std::max(attr.maxDynamicSharedSizeBytes, 1);
+    }
     if (bytes > limit) {
         TR_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
         limit = bytes;

@@ -15,6 +15,8 @@ namespace tr {
 constexpr int kMinLineLen = 13;      // oversampled length of the smallest image axis (10)
 constexpr int kMaxLineLen = 320;     // longer ones run the runtime-radix kernels
 constexpr int kLineW = 16;           // columns per CTA
+// z lengths whose empty-column skip also takes column counts that are multiples of 8 only (bin_colmask)
+__host__ __device__ constexpr bool lp_mixed_columns(int L) { return L == 240 || L == 320; }
 
 // Arguments of the forward x pass: image * coil map * separable apodisation * scale, centred
 // zero-pad, x FFT, centred shift, into the (Z, Y, OSX, ncol) buffer.
@@ -66,8 +68,9 @@ struct LineArgs {
 // (y / 4, x / 4) holds no busy tile: gridding wrote no tile there (the line is
 // all zeros) and interpolation reads no tap there.  True when every line
 // q0 .. q0 + W - 1 (< inner) of the CTA is unoccupied (the same for all threads).
-// The host passes a mask only when W divides ncol, so a CTA never mixes lines
-// of occupied and unoccupied columns (it would read unwritten tiles).
+// A CTA that mixes lines of occupied and unoccupied columns (W does not divide
+// the column count) must not read the latter's unwritten tiles: k_lp_line
+// takes them as zeros, for the other kernels the host passes no mask then.
 __device__ __forceinline__ bool lines_unoccupied(const LineArgs& a, int64_t q0, int W) {
     if (!a.colmask) return false;
     const int64_t q1 = min(q0 + W, a.inner) - 1;

@@ -149,7 +149,10 @@ __global__ void __launch_bounds__(lp_threads(L), lp_min_ctas(L)) k_lp_line(LineA
     const bool on = q < a.inner;
     const float2* in = a.in + outer * a.Lin * a.inner + q;
     float2* out = a.out + outer * a.Lout * a.inner + q;
-    const int lin = on ? a.Lin : 0, lout = on ? a.Lout : 0;
+    // lines of unoccupied and occupied columns in one CTA: the former's tiles hold no values (compiled only
+    // where it can happen: the check cost the z passes of other lengths 2 %)
+    const bool empty = lp_mixed_columns(L) && on && a.colmask && a.mcol % kLineW && lines_unoccupied(a, q, 1);
+    const int lin = on && !empty ? a.Lin : 0, lout = on ? a.Lout : 0;
     const LineRow<L> from(a.h, a.p_in), to(a.h, a.p_out);
     LpFirst<L> v;
     lp_load<L>(v, [&](int m, int) -> float2 {

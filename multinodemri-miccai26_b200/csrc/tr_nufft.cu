@@ -2062,18 +2062,17 @@ static tr_status stage_fwd_y(tr_plan* p, int ncol, cudaStream_t st) {
 }
 
 // Unoccupied-column mask of a bin for its z passes and its gridding (null: no
-// skipping).  Gridding leaves the tiles of unoccupied columns unwritten only
-// when no z-pass CTA mixes lines of occupied and unoccupied columns (a mixed
-// CTA transforms all its lines): every CTA's W lines lie in one (y, x) column
-// when ncol is a multiple of the z pass's W (16 at the compiled lengths, the
-// runtime-radix width elsewhere).
+// skipping).  Gridding leaves the tiles of unoccupied columns unwritten, so no
+// z-pass CTA may transform lines of such columns together with others: used
+// where the column count is a multiple of the CTA's lines (16; 8 for the
+// TMA kernel of 320 points) and at 240 and 320 points where it is a multiple
+// of 8 (k_lp_line then looks at each of its 16 lines).
 static const uint8_t* bin_colmask(const tr_plan* p, int bin, int ncol) {
-    if (!p->skip_empty_cols || !p->colmask || ncol % kLineW) return nullptr;
+    const int lines = lp_mixed_columns(p->os[0]) ? 8 : kLineW;
+    if (!p->skip_empty_cols || !p->colmask || ncol % lines) return nullptr;
     return p->colmask + (int64_t)bin * p->ntile[1] * p->ntile[2];
 }
 
-// z pass: [1][Z -> OSZ][OSY * OSX * ncol]; the lines of unoccupied columns are
-// not computed (interpolation reads none of them)
 static tr_status stage_fwd_z(tr_plan* p, int bin, int ncol, cudaStream_t st) {
     return launch_line(p, 0, p->bufB, p->bufA, 1, (int64_t)p->os[1] * p->os[2] * ncol, p->n[0], p->os[0],
                        p->ax[0].pad, 0, false, st, bin_colmask(p, bin, ncol), ncol);

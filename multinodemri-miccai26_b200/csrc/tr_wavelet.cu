@@ -323,6 +323,11 @@ __global__ void __launch_bounds__(256) k_dwt_yx(DwtYxArgs a) {
 }
 
 // ------------------------------------------------------------------ synthesis
+// The low filter's large taps come first, the high filter's last: the low products are added from the last
+// tap on, the high ones from the first, so that the large products meet the sum at the end and it rounds
+// less.  Relative error of three levels and time of 36 images of 112 x 160 x 160: 0.97e-7, 978 us; both from
+// the first tap on: 1.29e-7, 950 us; six pairs, half as many operations again: 1.18e-7, 1040 us.
+//
 // Along y, then x, of one slice: 8 bands -> T1 (img, bz, Zo, Yi, Xi).
 struct IdwtYxArgs {
     const float2* approx;     // band aaa: image i at approx + i * approx_stride
@@ -371,9 +376,9 @@ __global__ void __launch_bounds__(256) k_idwt_yx(IdwtYxArgs a) {
             CVec<1> e = cv_zero<1>(), o = cv_zero<1>();
 #pragma unroll
             for (int j = 0; j < kF / 2; ++j) {
-                cv_fma<1>(e, a.f.rec_lo[2 * j], u[(h + 5 - j) % 6]);
+                cv_fma<1>(e, a.f.rec_lo[10 - 2 * j], u[(h + j) % 6]);
                 cv_fma<1>(e, a.f.rec_hi[2 * j], v[(h + 5 - j) % 6]);
-                cv_fma<1>(o, a.f.rec_lo[2 * j + 1], u[(h + 5 - j) % 6]);
+                cv_fma<1>(o, a.f.rec_lo[11 - 2 * j], u[(h + j) % 6]);
                 cv_fma<1>(o, a.f.rec_hi[2 * j + 1], v[(h + 5 - j) % 6]);
             }
             dst[(2 * h) * pitch] = e.v[0];
@@ -391,11 +396,11 @@ __global__ void __launch_bounds__(256) k_idwt_yx(IdwtYxArgs a) {
 #pragma unroll
             for (int j = 0; j < kF / 2; ++j) {
                 CVec<1> u, v;
-                u.v[0] = lo[xp + 5 - j];
+                u.v[0] = lo[xp + j];
                 v.v[0] = hi[xp + 5 - j];
-                cv_fma<1>(e, a.f.rec_lo[2 * j], u);
+                cv_fma<1>(e, a.f.rec_lo[10 - 2 * j], u);
                 cv_fma<1>(e, a.f.rec_hi[2 * j], v);
-                cv_fma<1>(o, a.f.rec_lo[2 * j + 1], u);
+                cv_fma<1>(o, a.f.rec_lo[11 - 2 * j], u);
                 cv_fma<1>(o, a.f.rec_hi[2 * j + 1], v);
             }
             if (a.vec) {
@@ -439,9 +444,9 @@ __global__ void __launch_bounds__(256) k_idwt_z(const float2* __restrict__ in, f
             CVec<V> e = cv_zero<V>(), d = cv_zero<V>();
 #pragma unroll
             for (int j = 0; j < kF / 2; ++j) {
-                cv_fma<V>(e, f.rec_lo[2 * j], u[(h + 5 - j) % 6]);
+                cv_fma<V>(e, f.rec_lo[10 - 2 * j], u[(h + j) % 6]);
                 cv_fma<V>(e, f.rec_hi[2 * j], v[(h + 5 - j) % 6]);
-                cv_fma<V>(d, f.rec_lo[2 * j + 1], u[(h + 5 - j) % 6]);
+                cv_fma<V>(d, f.rec_lo[11 - 2 * j], u[(h + j) % 6]);
                 cv_fma<V>(d, f.rec_hi[2 * j + 1], v[(h + 5 - j) % 6]);
             }
             cv_store<V>(dst + (int64_t)(2 * h) * Q, e);

@@ -77,6 +77,8 @@ typedef struct {
                                     (comparison runs; results agree to float rounding) */
 #define TR_PLAN_NO_COLUMN_SKIP 16 /* transform every z line of the grid, also those of (y, x) tile columns
                                     that no sample's kernel reaches (comparison runs; same results) */
+#define TR_PLAN_SERIAL_BINS 32   /* PDHG iterations run the bins one after another also where small bins would
+                                    run side by side (comparison runs; same results) */
 
 typedef struct {
     int32_t os_shape[3];         /* oversampled grid (ceil(1.25 n) per axis) */

@@ -27,6 +27,7 @@ TR_PLAN_NO_TMA = 2
 TR_PLAN_YZ_FUSION = 4
 TR_PLAN_THREE_PASS_320 = 8
 TR_PLAN_NO_COLUMN_SKIP = 16
+TR_PLAN_SERIAL_BINS = 32
 
 EXPORTED = (
     "tr_plan_create", "tr_plan_destroy", "tr_plan_info", "tr_last_error_string", "tr_plan_set_maps",

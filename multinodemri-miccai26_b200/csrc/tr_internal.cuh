@@ -172,8 +172,8 @@ struct Bin {
     int64_t n_split = 0;       // tiles whose list is split over several work items
 };
 
-struct PdhgGraph;
-struct BinLanes;        // defined in tr_pdhg.cu
+struct PdhgGraph;        // defined in tr_pdhg.cu
+struct BinLanes;         // defined in tr_pdhg.cu
 struct WaveletPlan;      // defined in tr_wavelet.cu
 
 }  // namespace tr
@@ -226,6 +226,7 @@ struct tr_plan {
     bool use_tma = true;
     bool fuse_yz = false;        // TR_PLAN_YZ_FUSION: fused y + z passes where the geometry allows
     bool two_pass_320 = true;    // 320-point TMA FFT passes in two shared-memory passes (not TR_PLAN_THREE_PASS_320)
+    bool serial_bins = false;    // TR_PLAN_SERIAL_BINS: no lanes
     bool autotune = false;       // TR_PLAN_AUTOTUNE: time launch-shape candidates on first use
     std::map<int, int> spread_cols_tuned;   // column count -> chosen spread_cols         // TMA-tiled FFT passes where the geometry allows
     // TVMW

@@ -2887,6 +2887,7 @@ static tr_status plan_create_impl(const tr_plan_desc* d, tr_plan** out) {
     // the fused y + z kernels transform every line: gridding then zero-fills every empty tile
     p->skip_empty_cols = (d->flags & TR_PLAN_NO_COLUMN_SKIP) == 0 && !p->fuse_yz;
     p->autotune = (d->flags & TR_PLAN_AUTOTUNE) != 0;
+    p->serial_bins = (d->flags & TR_PLAN_SERIAL_BINS) != 0;
     p->workspace_bytes = (int64_t)(nks * (sizeof(float4) + sizeof(TapRec) + 2 * sizeof(int32_t)) +
                                    glist.size() * sizeof(int2) + (gwork.size() + gsplits.size()) * sizeof(int4) +
                                    (lstart.size() + torder.size()) * sizeof(int32_t) + cmask.size());

@@ -119,11 +119,13 @@ class B200NufftBackend(NufftBackend):
     TR_PLAN_YZ_FUSION, TR_PLAN_THREE_PASS_320); results agree to float rounding.
     ``column_skip=False`` (TR_PLAN_NO_COLUMN_SKIP) makes the z passes transform
     the grid lines of (y, x) tile columns no sample reaches as well (same bits).
+    ``bin_lanes=False`` (TR_PLAN_SERIAL_BINS) runs the bins of PDHG iterations one
+    after another also where they are small enough to run side by side (same bits).
     """
 
     def __init__(self, img_shape, coordinates, device=0, *, dcf: Iterable | None = None, n_coils: int = 1,
                  n_echoes: int = 1, autotune: bool = False, tma: bool = True, fuse_yz: bool = False,
-                 three_pass_320: bool = False, column_skip: bool = True) -> None:
+                 three_pass_320: bool = False, column_skip: bool = True, bin_lanes: bool = True) -> None:
         super().__init__(img_shape)
         import torch
         self._torch = torch
@@ -166,7 +168,8 @@ class B200NufftBackend(NufftBackend):
         desc.device = self.device_index
         desc.flags = ((_lib.TR_PLAN_AUTOTUNE if autotune else 0) | (0 if tma else _lib.TR_PLAN_NO_TMA)
                       | (_lib.TR_PLAN_YZ_FUSION if fuse_yz else 0) | (_lib.TR_PLAN_THREE_PASS_320 if three_pass_320 else 0)
-                      | (0 if column_skip else _lib.TR_PLAN_NO_COLUMN_SKIP))
+                      | (0 if column_skip else _lib.TR_PLAN_NO_COLUMN_SKIP)
+                      | (0 if bin_lanes else _lib.TR_PLAN_SERIAL_BINS))
         handle = ctypes.c_void_p()
         _lib.check(lib.tr_plan_create(ctypes.byref(desc), ctypes.byref(handle)), "tr_plan_create")
         self._plan = handle

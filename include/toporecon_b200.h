@@ -263,6 +263,9 @@ tr_status tr_profile_nufft(tr_plan* plan, int32_t bin, int32_t reps, double* ms,
  * A kernel whose bounded device wait runs out writes NaN to its outputs. */
 tr_status tr_conv3d_fwd(const void* x, const void* w, const float* bias, float* y, int32_t N, int32_t D,
                         int32_t H, int32_t W, int32_t Cin, int32_t Cout, void* stream);
+/* Polls before a device wait of the convolutions that the calling thread launches gives up (default 1 << 20;
+ * 0: every wait gives up at once).  For tests of the NaN mark. */
+tr_status tr_conv3d_set_wait_limit(int32_t polls);
 tr_status tr_conv3d_packed_size(int32_t Cin, int32_t Cout, size_t* bytes);
 tr_status tr_conv3d_pack(const void* w, int32_t w_f32, int32_t data_grad, void* packed, int32_t Cin, int32_t Cout,
                          void* stream);

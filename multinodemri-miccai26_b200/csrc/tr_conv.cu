@@ -18,9 +18,9 @@
 // per tap.  Forward reads the planes K-major (K = channels), the weight gradient reads the same
 // planes MN-major (K = voxels).
 //
-// Every wait is bounded (kMbarPollLimit polls); a CTA whose wait runs out writes NaN to its
-// outputs (the error mark a caller sees), lets its MMAs drain for a bounded time, frees its TMEM
-// and leaves.
+// Every wait is bounded (kMbarPollLimit polls, or the calling thread's tr_conv3d_set_wait_limit); a CTA
+// whose wait runs out writes NaN to its outputs (the error mark a caller sees), lets its MMAs and copies end
+// (at most kMbarDrainLimit polls, whatever the limit), frees its TMEM and leaves.
 
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -34,6 +34,7 @@
 
 namespace {
 
+using tr::kMbarDrainLimit;
 using tr::kMbarPollLimit;
 using tr::mbar_init;
 using tr::mbar_wait_bounded;
@@ -354,10 +355,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_conv3d_fwd(const TIn* __rest
                 }
                 mma_commit(&afull[as]);
             }
-            if (!ok) {                                       // MMAs in flight end before the TMEM is freed
-                mma_commit(&drained[warp >> 1]);
-                mbar_wait_bounded(&drained[warp >> 1], 0, poll);
-            }
+            // MMAs in flight end before the TMEM is freed, also where only the epilogue's wait ran out
+            mma_commit(&drained[warp >> 1]);
+            mbar_wait_bounded(&drained[warp >> 1], 0, kMbarDrainLimit);
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_conv3d_fwd(const TIn* __rest
                 }
             }
             for (int i = max(0, last - nst); i < last; ++i)  // no copy outlives the CTA
-                mbar_wait_bounded(&wfull[i % nst], (i / nst) & 1, poll);
+                mbar_wait_bounded(&wfull[i % nst], (i / nst) & 1, kMbarDrainLimit);
         }
         __syncwarp();
     } else if (warp >= 8) {
@@ -780,7 +780,7 @@ __global__ void __launch_bounds__(kWgThreads) k_conv3d_wgrad(const __nv_bfloat16
             }
         }
         if (bad) {
-            if (tid == 0) mbar_wait_bounded(&done, run & 1, poll);
+            if (tid == 0) mbar_wait_bounded(&done, run & 1, kMbarDrainLimit);     // MMAs in flight end
             break;
         }
         tc_fence_before();
@@ -807,6 +807,8 @@ __global__ void __launch_bounds__(128) k_wgrad_reduce(const float* __restrict__ 
     const int co = i % Cout, r = i / Cout;
     dw[((int64_t)co * 27 + r / Cin) * Cin + r % Cin] = s;
 }
+
+thread_local int wait_polls = kMbarPollLimit;         // of the convolutions that this thread launches
 
 tr_status check_dims(const ConvDims& c) {
     if (c.N < 1 || c.D < 1 || c.H < 1 || c.W < 1) return tr::fail(TR_ERR_INVALID_ARG, "conv3d: empty volume");
@@ -839,7 +841,7 @@ tr_status launch_fwd(const TIn* x, const __nv_bfloat16* w, const float* bias, fl
     const int nacc = 2 * NZ * npad <= 512 ? 2 : 1;
     TR_TRY(tr::raise_smem_limit((const void*)fn, smem));
     fn<<<(unsigned)std::min<int64_t>(tiles, sm_count()), kFwdThreads, smem, st>>>(
-        x, w, bias, y, c, tiles, npad, nacc, tmem_cols(nacc * NZ * npad), at16(y), kMbarPollLimit);
+        x, w, bias, y, c, tiles, npad, nacc, tmem_cols(nacc * NZ * npad), at16(y), wait_polls);
     TR_CHECK_LAUNCH();
     return TR_OK;
 }
@@ -957,6 +959,12 @@ extern "C" tr_status tr_conv3d_fwd(const void* x, const void* w, const float* bi
     return rc;
 }
 
+extern "C" tr_status tr_conv3d_set_wait_limit(int32_t polls) {
+    if (polls < 0) return tr::fail(TR_ERR_INVALID_ARG, "tr_conv3d_set_wait_limit: polls must be >= 0");
+    wait_polls = polls;
+    return TR_OK;
+}
+
 extern "C" tr_status tr_conv3d_packed_size(int32_t Cin, int32_t Cout, size_t* bytes) {
     if (!bytes) return tr::fail(TR_ERR_INVALID_ARG, "null bytes");
     TR_TRY(check_dims(ConvDims{1, 1, 1, 1, Cin, Cout, 1}));
@@ -1014,7 +1022,7 @@ extern "C" tr_status tr_conv3d_wgrad(const void* x, const void* gy, float* dw, i
     auto fn = tail ? wgrad_kernel<true>(s.npad, vec, s.mx) : wgrad_kernel<false>(s.npad, vec, s.mx);
     TR_TRY(tr::raise_smem_limit((const void*)fn, smem));
     const dim3 grid((unsigned)s.splits, (unsigned)s.groups, (unsigned)(s.cx * s.cg));
-    fn<<<grid, kWgThreads, smem, st>>>(xb, gb, part, c, s, kMbarPollLimit);
+    fn<<<grid, kWgThreads, smem, st>>>(xb, gb, part, c, s, wait_polls);
     TR_CHECK_LAUNCH();
     const int64_t total = partial_floats(c);
     k_wgrad_reduce<<<(unsigned)((total + 127) / 128), 128, 0, st>>>(part, dw, s.splits, Cin, Cout);

@@ -295,15 +295,32 @@ __global__ void __launch_bounds__(256) k_adj_x(AdjXArgs a) {
 //   tr_lines.cuh are faster: z pass at 60, 80, 100, 120 (32 columns) 0.15, 0.18, 0.21, 0.26 against
 //   0.19, 0.22, 0.25, 0.29 ms, y pass at 100, 120, 140 0.13, 0.16, 0.19 against 0.14, 0.16, 0.20 ms,
 //   at 240 (24 columns) 0.30 against 0.42 ms.
-// - x passes with whole groups of 8 or 4 coils (below): forward 0.18, 0.95 and 2.63 ms at 96 x 128 x 128
-//   (32 columns), 112 x 160 x 160 (72) and 128 x 256 x 256 (96) against 0.23, 1.01 and 2.92 ms, adjoint
-//   0.27, 1.11 and 2.94 against 0.27, 1.49 and 4.53 ms.
+// - x passes with whole groups of 8 or 4 coils, by x_tma_fwd and x_tma_adj below.
 // Lengths up to 200 use 16-column tiles, longer ones 8-column tiles (the
 // shared-memory footprint 2 L W x 8 bytes then allows >= 4 CTAs per SM).
 #define TR_LINE_TMA_LENGTHS(X) X(160) X(200) X(320)
 #define TR_CT_WIDE(X) X(60) X(80) X(100) X(120) X(140) X(160) X(200)
 #define TR_CT_NARROW(X) X(240) X(320)
 #define TR_CT_LENGTHS(X) TR_CT_WIDE(X) TR_CT_NARROW(X)
+// Whether the x passes of n_img images and C coils take the TMA kernels (groups of wt = 8 or 4 coils) at a
+// length L of TR_CT_LENGTHS.  The kernels of tr_lines_part.cuh keep a column's map in registers over the
+// images, so that they gain with the images; groups of 4 move 32-byte rows.  Measured on 64 x 128 rows
+// (16 x 32 to 32 x 64 at 320), time of tr_lines_part.cuh / TMA:
+//   forward   8 coils, 1, 2, 4 images: L = 60  1.44 1.07 0.88;  100  1.31 1.04 0.87;  140  1.68 1.35 1.17;
+//             160  1.76 1.43 1.29;  200  1.99 1.64 1.43;  240  1.21 1.00 0.89;  320  1.51 1.35 1.24
+//             4, 12, 20 coils, 1 / 4 images: 80  1.06 / 0.68, 0.89 / 0.53, 0.72 / 0.47;  160  1.41 / 1.13,
+//             1.11 / 0.92, 0.66 / 0.59;  200  1.70 / 1.29, 1.34 / 1.13, 0.81 / 0.70;  240  1.11 / 0.93,
+//             0.87 / 0.77, 0.52 / 0.49;  320  1.32 / 1.26, 1.19 / 0.87, 0.67 / 0.55
+//   adjoint   8 coils, 1, 2, 4 images: 60  0.88 0.64 0.57;  100  0.94 0.74 0.63;  120  1.09 0.84 0.71;
+//             140  1.97 1.42 1.12;  160  1.60 1.20 1.02;  200  1.67 1.37 1.22;  240  1.94 1.46 1.19;
+//             320  2.65 2.04 1.78;   4, 12, 20 coils, 1 / 4 images: 80  0.70 / 0.41, 0.94 / 0.60, 1.01 / 0.71;
+//             120  0.80 / 0.56, 1.21 / 0.80, 1.30 / 0.95;  160  1.20 / 0.80, 1.76 / 1.15, 1.81 / 1.32
+static bool x_tma_fwd(int L, int wt, int C, int n_img) {
+    const bool good = L == 140 || L == 160 || L == 200 || L == 320;
+    if (wt == 8) return good || n_img <= 2;
+    return good ? C <= 12 : C == 4 && n_img <= 2;
+}
+static bool x_tma_adj(int L, int wt, int C, int n_img) { return L >= 140 || (n_img == 1 && (wt == 8 || C > 4)); }
 __host__ __device__ constexpr int ct_width(int L) { return L >= 240 ? 8 : 16; }
 // The TMA x passes take 8 coils per CTA at every length: their rows are contiguous,
 // so narrow tiles cost no DRAM efficiency and buy occupancy (the strided y / z
@@ -1898,7 +1915,7 @@ static tr_status stage_fwd_x(tr_plan* p, const float2* images, int64_t img_strid
     // when OSX % 8 == 0)
     int wt = C % kTmaXWidth == 0 ? kTmaXWidth : (C % 4 == 0 ? 4 : 0);
     if (wt == 4 && ((int64_t)(OSX / 2) * wt * 8) % 128) wt = 0;
-    if (p->use_tma && ct && maps && wt && X % 16 == 0 && X <= 256 && img_stride % 2 == 0 &&
+    if (p->use_tma && ct && maps && wt && x_tma_fwd(OSX, wt, C, n_img) && X % 16 == 0 && X <= 256 && img_stride % 2 == 0 &&
         (int64_t)X * (wt + 1) <= (int64_t)OSX * wt && OSX / 2 <= 256) {
         CUtensorMap timg, tmap, tout;
         const uint64_t nrows = (uint64_t)Z * Y;
@@ -2296,7 +2313,7 @@ static tr_status stage_adj_x(tr_plan* p, int n_img, const float2* maps, int C, f
     // and the second input box, (OSX / 2) 32-byte rows into the tile, is 128-byte aligned)
     int wt = C % kTmaXWidth == 0 ? kTmaXWidth : (C % 4 == 0 ? 4 : 0);
     if (wt == 4 && ((int64_t)(OSX / 2) * wt * 8) % 128) wt = 0;
-    if (p->use_tma && ct && maps && wt && OSX / 2 <= 256 && X <= 256 && X + 4 <= OSX) {
+    if (p->use_tma && ct && maps && wt && x_tma_adj(OSX, wt, C, n_img) && OSX / 2 <= 256 && X <= 256 && X + 4 <= OSX) {
         CUtensorMap tin;
         const void* tfn = nullptr;
         unsigned nt = (unsigned)ct_threads(OSX, wt);

@@ -180,6 +180,7 @@ struct WaveletPlan;      // defined in tr_wavelet.cu
 
 struct tr_plan {
     int device = 0;
+    int sms = 148;               // the device's SMs
     int n[3] = {0, 0, 0};     // Z, Y, X
     int os[3] = {0, 0, 0};
     int C = 1, E = 1, B = 1;

@@ -930,12 +930,14 @@ __global__ void __launch_bounds__(kWideNT, 5) k_adj_x_wide(AdjXArgs a, const __g
 // 16 or more columns over their lanes.
 constexpr int kFewCols = 8;
 // Most samples for which k_interp_rows takes a bin of 1 to 8 columns.  Its sixteen lanes a sample hide
-// latency while samples are few; with many, k_interp reads the same grid lines with fewer instructions
-// (us, rows / k_interp, at 50 000, 100 000 and 213 000 samples: 1 column 12.0 / 15.1, 21.4 / 16.8,
-// 43.2 / 22.9; 2: 12.5 / 21.4, 22.4 / 22.1, 45.2 / 31.2; 4: 15.4 / 21.5, 27.2 / 30.6, 55.2 / 48.6;
-// 6: 23.0 / 28.2, 41.6 / 39.6, 83.6 / 72.3; 7: 32.5 / 26.6, 58.2 / 45.7, 115 / 91; 8: 25.2 / 40.0,
-// 43.8 / 53.6, 84.9 / 82.6).
-constexpr int64_t kFewRowsMax[kFewCols + 1] = {0, 65536, 98304, 65536, 131072, 49152, 81920, 20480, 196608};
+// latency while samples are few; with many, k_interp reads the same grid lines with fewer instructions.
+// With an odd count a lane carries every column, so the line falls with the count.  Measured (us, rows /
+// k_interp, cones on 84 x 100 x 112; 40 000, 110 000 and 250 000 samples): 1 column 12 / 18, 27 / 21, 54 / 29;
+// 3: 16 / 19, 34 / 27, 72 / 54; 5: 21 / 23, 45 / 37, 99 / 86; 7: 29 / 26, 66 / 53, 146 / 123; 2: 12 / 23, 27 / 25,
+// 56 / 42; 4: 15 / 27, 31 / 34, 69 / 64; 6: 20 / 26, 45 / 47, 103 / 105; 8: 24 / 29, 56 / 64, 125 / 121.
+// Over seven grids, cones and random samples, 3 000 to 800 000 of them, the lines cost 0.8 % (cones) and 3 to 5 %
+// (random) against the better kernel each time.
+constexpr int64_t few_rows_max(int ncol) { return ncol % 2 == 0 ? 131072 : 196608 / (ncol < 3 ? 3 : ncol); }
 
 // First tap per axis and the 15 KB weights of every (sorted) sample, computed
 // once at plan creation; interpolation and gridding read them instead of
@@ -2100,7 +2102,7 @@ static tr_status stage_interp(tr_plan* p, int bin, int ncol, int mode, float sig
                               cudaStream_t st, const int32_t* perm = nullptr) {
     const Bin& b = p->bins[bin];
     if (b.count == 0) return TR_OK;
-    if (ncol <= kFewCols && b.count <= kFewRowsMax[ncol]) {
+    if (ncol <= kFewCols && b.count <= few_rows_max(ncol)) {
         const TapRec* taps = reinterpret_cast<const TapRec*>(p->taps) + b.offset;
         const unsigned blocks = (unsigned)((b.count * 16 + 255) / 256);
 #define TR_INTERP_ROWS(NCV)                                                                                       \
@@ -2120,18 +2122,15 @@ static tr_status stage_interp(tr_plan* p, int bin, int ncol, int mode, float sig
     if (ncol > 256) return fail(TR_ERR_UNSUPPORTED, "more than 256 k-space columns per bin are not supported");
     // Even column counts read pairs (bufA is aligned and a row of ncol even columns starts on 16 bytes).
     // While the lanes of one piece each are at most a wave of the chip's threads, one piece a lane is faster
-    // (us at 1 / 2 / 3 pieces a lane, 60 x 70 x 80 grid: 12 columns, 18 000 samples 23 / 29 / 38, 48 000 35 / 49 / 64;
-    // 32 columns, 6 000 samples 21 / 26 / 32, 18 000 35 / 44 / 66); beyond it fewer lanes a sample, so that a warp
-    // holds several samples and a lane several loads in flight (80 x 120 x 120 grid, 80 000 samples, 1 / 2 / 3 / 4:
-    // 12 columns 71 / 66 / 78 / 110, 24: 142 / 90 / 103 / 181, 48: 257 / 155 / 162 / 274; 10: 53 / 63 / 78 / 103;
-    // 8 columns, 960 000 samples on 150^3: 399 / 336 / 353 / 577, 6: 304 / 288 / 259 / 394 but 72 / 73 / 82 / 107 at
-    // 213 000).  Odd ones, single values, turn at four waves (15: 85 / 100 / 83 / 97, 25: 135 / 136 / 112 / 128, at
-    // 48 000 samples 85 / 103 / 85; 9: 48 / 81 / 69 / 84), above 32 columns at once (45, 6 000 samples: 64 / 63 / 50).
+    // (us at 1 / 2 / 3 pieces a lane, cones, 20 000 samples on 40 x 64 x 72: 12 columns 23 / 31 / 60, 32 columns 38 / 44 / 67); beyond
+    // it fewer lanes a sample, so that a warp holds several samples and a lane several loads in flight (130 000
+    // samples on 84 x 100 x 112, 1 / 2 / 3 / 4: 8 columns 80 / 69 / 81 / 134, 10: 101 / 78 / 95 / 137, 24: 220 / 137 / 142 / 223, 48: 406 / 243 / 254 / 387); fewer than four pairs
+    // stay apart.  Odd counts, single values, turn at four waves and 15 pieces (15 columns, 130 000 samples 133 / 130 / 115 / 127,
+    // 50 000 58 / 85 / 69 / 84; 9 columns, 130 000 83 / 100 / 80 / 96), above 32 columns at once (45 columns, 6 000 samples on 40 x 64 x 72, 2 / 3 / 4: 60 / 49 / 62).
     const int V = ncol % 2 == 0 ? 2 : 1, pieces = ncol / V;
-    constexpr int64_t kWave = 148 * 2048;
-    const int64_t lanes = b.count * pieces;
-    const int more = V == 2 ? ((pieces == 4 || pieces >= 6) && lanes > kWave ? 2 : 1)
-                            : (pieces > 32 || (pieces >= 15 && lanes > 4 * kWave) ? 3 : 1);
+    const int64_t lanes = b.count * pieces, wave = (int64_t)p->sms * 2048;
+    const int more = V == 2 ? (pieces >= 4 && lanes > wave ? 2 : 1)
+                            : (pieces > 32 || (pieces >= 15 && lanes > 4 * wave) ? 3 : 1);
     const int cpl = std::max((pieces + 31) / 32, more);
     const int G = (pieces + cpl - 1) / cpl;
     const unsigned blocks = (unsigned)((b.count * G + 255) / 256);
@@ -2154,7 +2153,6 @@ static tr_status stage_interp(tr_plan* p, int bin, int ncol, int mode, float sig
                                                                  p->os[2], mode, sigma, perm, y, out);
                 else TR_INTERP(1, 1);
                 break;
-            case 2: TR_INTERP(1, 2); break;
             case 3: TR_INTERP(1, 3); break;
             case 4: TR_INTERP(1, 4); break;
             default: TR_INTERP(1, 8); break;
@@ -2723,6 +2721,7 @@ static tr_status plan_create_impl(const tr_plan_desc* d, tr_plan** out) {
             if (p) plan_free(p);
         }
     } owner{p};
+    TR_CUDA(cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, d->device));
     auto bad = [&](tr_status code, const std::string& m) { return fail(code, m); };
     for (int i = 0; i < 3; ++i) {
         FftAxis& A = p->ax[i];

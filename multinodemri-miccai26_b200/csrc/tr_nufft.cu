@@ -1504,10 +1504,17 @@ __global__ void __launch_bounds__(32 * kFewWarps) k_spread_few(SpreadArgs a, con
         const int z1 = min((int)zhi * kFewZero, a.n_empty);
         for (int zi = (int)zlo * kFewZero; zi < z1; ++zi) {
             tile_geometry(a, a.tile_order[a.n_busy + zi], t0z, t0y, t0x, Tz, Ty, Tx);
-            if (pz >= Tz || py >= Ty) continue;
-            for (int x = xh; x < min(xh + 2, Tx); ++x)
+            // consecutive lanes along a row's values, two at a time where rows start on 16 bytes (with a lane's own two
+            // points a store reached 8 bytes of each sector; 500 samples, 8 columns on 160^3: 188 us, 54 now)
+            using Zero = std::conditional_t<NC % 2 == 0, float4, float2>;
+            constexpr int per = sizeof(Zero) / sizeof(float2), row_n = 4 * NC / per;
 #pragma unroll
-                for (int j = 0; j < NC; ++j) point(x)[j] = make_float2(0.f, 0.f);
+            for (int i = lane; i < 16 * row_n; i += 32) {
+                const int r = i / row_n, o = (i - r * row_n) * per;
+                if ((r >> 2) < Tz && (r & 3) < Ty && o < Tx * NC)
+                    *reinterpret_cast<Zero*>(a.grid + (((int64_t)(t0z + (r >> 2)) * a.os1 + (t0y + (r & 3))) * a.os2 + t0x) * NC +
+                                             o) = Zero{};
+            }
         }
         return;
     }

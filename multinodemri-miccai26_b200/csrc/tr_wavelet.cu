@@ -184,19 +184,22 @@ __device__ __forceinline__ void cv_fma(CVec<V>& acc, float f, const CVec<V>& x) 
 }
 
 // ------------------------------------------------------------------ analysis
-constexpr int kDwtRun = 12;      // outputs per thread along z: 34 loads instead of the 24 of a whole line
+// Outputs per thread along z: 34 loads for 12 instead of the 24 of a whole line; 4 (18 loads) while runs of 12
+// are less than a wave of blocks.  One image of 48 x 64 x 64, analysis of two levels: 43 us with runs of 12, 36 with 4 (37 with one output a
+// thread before).
+constexpr int kDwtRun = 12, kDwtRunShort = 4;
 constexpr int kDwtRows = 16;     // output rows (of each half) per CTA of the y + x kernel
 
 // Along z: in (P, n, Q) -> out (P, 2, no, Q) (band 0 = low, 1 = high).
-template <int V>
+template <int V, int RUN>
 __global__ void __launch_bounds__(256) k_dwt_z(const float2* __restrict__ in, float2* __restrict__ out, int64_t P, int n,
                                                int64_t Q, int no, Filters f) {
     const int64_t q = ((int64_t)blockIdx.x * 256 + threadIdx.x) * V;
     if (q >= Q) return;
-    const int runs = (no + kDwtRun - 1) / kDwtRun;
+    const int runs = (no + RUN - 1) / RUN;
     for (int64_t pr = blockIdx.y; pr < P * runs; pr += gridDim.y) {
         const int64_t pp = pr / runs;
-        const int o0 = (int)(pr - pp * runs) * kDwtRun;
+        const int o0 = (int)(pr - pp * runs) * RUN;
         const float2* src = in + pp * n * Q + q;
         float2* lo = out + (pp * 2 * no + o0) * Q + q;
         float2* hi = lo + (int64_t)no * Q;
@@ -205,7 +208,7 @@ __global__ void __launch_bounds__(256) k_dwt_z(const float2* __restrict__ in, fl
 #pragma unroll
         for (int t = 0; t < kF - 2; ++t) w[(t + 2) % kF] = get(2 * o0 - (kF - 2) + t);
 #pragma unroll
-        for (int r = 0; r < kDwtRun; ++r) {
+        for (int r = 0; r < RUN; ++r) {
             w[(2 * r) % kF] = get(2 * (o0 + r));
             w[(2 * r + 1) % kF] = get(2 * (o0 + r) + 1);
             CVec<V> a = cv_zero<V>(), b = cv_zero<V>();
@@ -478,11 +481,13 @@ tr_status wavelet_dual(tr_plan* p, const float2* u_bar, float2* p_w2, float sigm
     for (int l = 0; l < w->levels; ++l) {
         const int* si = w->in_shape[l];
         const int* so = w->out_shape[l];
-        const int64_t Q = (int64_t)si[1] * si[2], runs = (int64_t)nimg * ((so[0] + kDwtRun - 1) / kDwtRun);
-        if (two_wide(Q, cur, w->T1))
-            k_dwt_z<2><<<z_grid(Q, 2, runs), 256, 0, st>>>(cur, w->T1, nimg, si[0], Q, so[0], w->f);
-        else
-            k_dwt_z<1><<<z_grid(Q, 1, runs), 256, 0, st>>>(cur, w->T1, nimg, si[0], Q, so[0], w->f);
+        const int64_t Q = (int64_t)si[1] * si[2];
+        const int V = two_wide(Q, cur, w->T1) ? 2 : 1;
+        auto runs = [&](int run) { return (int64_t)nimg * ((so[0] + run - 1) / run); };
+        const bool few = (Q / V + 255) / 256 * runs(kDwtRun) < 2 * p->sms;
+        auto fn = few ? (V == 2 ? k_dwt_z<2, kDwtRunShort> : k_dwt_z<1, kDwtRunShort>)
+                      : (V == 2 ? k_dwt_z<2, kDwtRun> : k_dwt_z<1, kDwtRun>);
+        fn<<<z_grid(Q, V, runs(few ? kDwtRunShort : kDwtRun)), 256, 0, st>>>(cur, w->T1, nimg, si[0], Q, so[0], w->f);
         TR_CHECK_LAUNCH();
         DwtYxArgs a;
         a.in = w->T1;

@@ -271,6 +271,10 @@ tr_status tr_conv3d_pack(const void* w, int32_t w_f32, int32_t data_grad, void* 
                          void* stream);
 tr_status tr_conv3d_fwd_packed(const void* x, int32_t x_f32, const void* packed, const float* bias, float* y, int32_t N,
                                int32_t D, int32_t H, int32_t W, int32_t Cin, int32_t Cout, void* stream);
+/* tr_conv3d_pack into `packed`, then tr_conv3d_fwd_packed with it. */
+tr_status tr_conv3d_fwd_weights(const void* x, int32_t x_f32, const void* w, int32_t w_f32, int32_t data_grad,
+                                void* packed, const float* bias, float* y, int32_t N, int32_t D, int32_t H, int32_t W,
+                                int32_t Cin, int32_t Cout, void* stream);
 tr_status tr_conv3d_wgrad_workspace(int32_t N, int32_t D, int32_t H, int32_t W, int32_t Cin, int32_t Cout,
                                     size_t* bytes);
 tr_status tr_conv3d_wgrad(const void* x, const void* gy, float* dw, int32_t N, int32_t D, int32_t H, int32_t W,

@@ -34,7 +34,7 @@ EXPORTED = (
     "tr_plan_sort_kspace", "tr_plan_unsort_kspace", "tr_nufft_forward", "tr_nufft_adjoint",
     "tr_nufft_forward_bin", "tr_nufft_adjoint_bin", "tr_plan_bin_offset", "tr_pdhg_run",
     "tr_power_iteration", "tr_profile_nufft", "tr_tolerance_sums_noalloc", "tr_conv3d_fwd", "tr_conv3d_packed_size",
-    "tr_conv3d_set_wait_limit",
+    "tr_conv3d_set_wait_limit", "tr_conv3d_fwd_weights",
     "tr_conv3d_pack", "tr_conv3d_fwd_packed",
     "tr_conv3d_wgrad_workspace", "tr_conv3d_wgrad", "tr_pdhg_phase", "tr_plan_set_wait_limit",
     "tr_wavelet_forward", "tr_wavelet_adjoint",
@@ -149,6 +149,7 @@ def load() -> ctypes.CDLL:
             "tr_tolerance_sums_noalloc": ([vp, vp, i64, i32, vp, vp], i32),
             "tr_conv3d_fwd": ([vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp], i32),
             "tr_conv3d_set_wait_limit": ([i32], i32),
+            "tr_conv3d_fwd_weights": ([vp, i32, vp, i32, i32, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp], i32),
             "tr_conv3d_packed_size": ([i32, i32, ctypes.POINTER(ctypes.c_size_t)], i32),
             "tr_conv3d_pack": ([vp, i32, i32, vp, i32, i32, vp], i32),
             "tr_conv3d_fwd_packed": ([vp, i32, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp], i32),

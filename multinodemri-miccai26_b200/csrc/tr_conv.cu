@@ -991,6 +991,13 @@ extern "C" tr_status tr_conv3d_fwd_packed(const void* x, int32_t x_f32, const vo
                  : conv_fwd((const __nv_bfloat16*)x, wp, bias, y, c, (cudaStream_t)stream);
 }
 
+extern "C" tr_status tr_conv3d_fwd_weights(const void* x, int32_t x_f32, const void* w, int32_t w_f32, int32_t data_grad,
+                                           void* packed, const float* bias, float* y, int32_t N, int32_t D, int32_t H,
+                                           int32_t W, int32_t Cin, int32_t Cout, void* stream) {
+    TR_TRY(tr_conv3d_pack(w, w_f32, data_grad, packed, Cin, Cout, stream));
+    return tr_conv3d_fwd_packed(x, x_f32, packed, bias, y, N, D, H, W, Cin, Cout, stream);
+}
+
 // Scratch: one partial per kWgradVox voxels, or per split where the launch wants more of them.
 extern "C" tr_status tr_conv3d_wgrad_workspace(int32_t N, int32_t D, int32_t H, int32_t W, int32_t Cin,
                                                int32_t Cout, size_t* bytes) {

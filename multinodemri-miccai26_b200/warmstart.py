@@ -19,6 +19,7 @@ convolutions on [re | im] channel halves with the weight structure
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 import time
 from dataclasses import asdict, dataclass
@@ -42,17 +43,21 @@ def _stream(t):
     return ctypes.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
 
 
+@functools.lru_cache(maxsize=None)
+def _packed_elems(cin, cout):
+    nbytes = ctypes.c_size_t(0)
+    _lib.check(_lib.load().tr_conv3d_packed_size(cin, cout, ctypes.byref(nbytes)))
+    return nbytes.value // 2
+
+
 def pack_weights(w, cin, cout, data_grad=False):
     """Weights w, bf16 or float32, any strides, in the layout the forward kernel streams, as bf16:
     (cout, 27, cin), or with ``data_grad`` the layer's own (cin, 27, cout) flipped and swapped."""
     import torch
     w = w.contiguous()
-    L = _lib.load()
-    nbytes = ctypes.c_size_t(0)
-    _lib.check(L.tr_conv3d_packed_size(cin, cout, ctypes.byref(nbytes)))
-    packed = torch.empty(nbytes.value // 2, dtype=torch.bfloat16, device=w.device)
-    _lib.check(L.tr_conv3d_pack(_ptr(w), int(w.dtype == torch.float32), int(data_grad), _ptr(packed), cin, cout,
-                                _stream(packed)), "tr_conv3d_pack")
+    packed = torch.empty(_packed_elems(cin, cout), dtype=torch.bfloat16, device=w.device)
+    _lib.check(_lib.load().tr_conv3d_pack(_ptr(w), int(w.dtype == torch.float32), int(data_grad), _ptr(packed), cin, cout,
+                                          _stream(packed)), "tr_conv3d_pack")
     return packed
 
 
@@ -68,9 +73,22 @@ def conv3d_fwd_packed(x, packed, cout, bias=None):
     return y
 
 
+def _conv3d_weights(x, w, cout, bias=None, data_grad=False):
+    """conv3d_fwd_packed with pack_weights(w, ...) in one call of the library (small layers wait for the host)."""
+    import torch
+    w = w.contiguous()
+    N, D, H, W, Cin = x.shape
+    packed = torch.empty(_packed_elems(Cin, cout), dtype=torch.bfloat16, device=w.device)
+    y = torch.empty((N, D, H, W, cout), dtype=torch.float32, device=x.device)
+    _lib.check(_lib.load().tr_conv3d_fwd_weights(
+        _ptr(x), int(x.dtype == torch.float32), _ptr(w), int(w.dtype == torch.float32), int(data_grad), _ptr(packed),
+        _ptr(bias) if bias is not None else None, _ptr(y), N, D, H, W, Cin, cout, _stream(y)), "tr_conv3d_fwd")
+    return y
+
+
 def conv3d_fwd_bf16(x_bf, w_bf, bias=None):
     """x (N, D, H, W, Cin) bf16, w (Cout, 27, Cin) bf16 -> (N, D, H, W, Cout) f32."""
-    return conv3d_fwd_packed(x_bf, pack_weights(w_bf, x_bf.shape[-1], w_bf.shape[0]), w_bf.shape[0], bias)
+    return _conv3d_weights(x_bf, w_bf, w_bf.shape[0], bias)
 
 
 def conv3d_wgrad_bf16(x_bf, gy_bf):
@@ -96,7 +114,7 @@ def conv3d_dgrad_bf16(gy_bf, w_bf):
     if pad:
         import torch
         w_bf = torch.cat([w_bf, w_bf.new_zeros((cout, 27, pad))], dim=2)
-    gx = conv3d_fwd_packed(gy_bf, pack_weights(w_bf, cout, cin + pad, data_grad=True), cin + pad)
+    gx = _conv3d_weights(gy_bf, w_bf, cin + pad, data_grad=True)
     return gx[..., :cin].contiguous() if pad else gx
 
 
@@ -108,7 +126,7 @@ def _make_conv_fn():
         def forward(ctx, x, w, b, grad):
             if not (grad and any(ctx.needs_input_grad)) and x.dtype == w.dtype == torch.float32:
                 # no backward will read bf16 copies of x and w
-                return conv3d_fwd_packed(x.contiguous(), pack_weights(w, x.shape[-1], w.shape[0]), w.shape[0], b)
+                return _conv3d_weights(x.contiguous(), w, w.shape[0], b)
             xb = x.contiguous().to(torch.bfloat16)
             wb = w.contiguous().to(torch.bfloat16)
             ctx.save_for_backward(xb, wb)

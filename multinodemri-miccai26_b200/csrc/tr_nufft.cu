@@ -2228,7 +2228,7 @@ static tr_status stage_spread(tr_plan* p, int bin, const float2* ksp, int ncol, 
         TR_CHECK_LAUNCH();
         if (b.n_split > 0) {
             k_spread_reduce<<<dim3((unsigned)b.n_split, (unsigned)((64 * ncol + 255) / 256)), 256, 0, st>>>(
-            sa, p->splits + b.split_offset);
+                sa, p->splits + b.split_offset);
             TR_CHECK_LAUNCH();
         }
         return TR_OK;
@@ -2992,7 +2992,7 @@ tr_status tr_plan_set_maps(tr_plan* p, const void* mps, void* stream) {
         p->workspace_bytes += N * p->C * (int64_t)sizeof(float2);
     }
     const int64_t tot = N * p->C;
-k_interleave_maps<<<(unsigned)((tot + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+    k_interleave_maps<<<(unsigned)((tot + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
         (const float2*)mps, p->maps, N, p->C, p->n[1], p->n[2], p->ax[0].apod, p->ax[1].apod, p->ax[2].apod, p->fwd_scale);
     TR_CHECK_LAUNCH();
     return TR_OK;

@@ -397,9 +397,11 @@ static PdArgs make_args(tr_plan* p, const tr_pdhg_state* s, const tr_pdhg_params
 // another and of the TV and wavelet duals until the primal update.  Where one bin's workspace is at
 // most kLaneBytes, the bins run on lanes: streams of the plan with a workspace each, forked from the
 // caller's stream by an event and joined to it by events (a captured iteration becomes a graph with
-// parallel branches); the duals run on the caller's stream meanwhile.  Larger bins fill the chip by
-// themselves and keep one workspace.  48 x 64 x 64, 4 coils, 6 bins (22 MB a bin): 554 us per TVM
-// iteration with the bins one after another, 392 us side by side.
+// parallel branches); the duals run on the caller's stream meanwhile.  Larger bins fill the chip nearly
+// by themselves and keep one workspace: side by side gains less than what eight workspaces hold is worth.
+// Measured, an iteration with the bins one after another / side by side, us: 21 MB a bin (48 x 64 x 64, 4
+// coils, 6 bins) 554 / 389; 44 MB 743 / 611; 63 MB (4 bins) 663 / 599; 99 MB 1458 / 1273; 138 MB
+// 2086 / 1876; 258 MB 3154 / 2915; 352 MB (32 columns) 4105 / 3776; 675 MB 6611 / 6255; 1350 MB 5942 / 5785.
 constexpr size_t kLaneBytes = 64u << 20;
 constexpr int kMaxLanes = 8;
 

@@ -260,6 +260,7 @@ tr_status tr_profile_nufft(tr_plan* plan, int32_t bin, int32_t reps, double* ms,
  * weights (Cin, 27, Cout) and packs the data gradient's.  tr_conv3d_fwd_packed is the forward
  * convolution with packed weights; float activations (x_f32) are rounded to bf16 as they are read.
  * tr_conv3d_fwd packs its weights into stream-ordered scratch on each call.
+ * Pointers need the alignment of their element type only (packed weights: 16 bytes).
  * A kernel whose bounded device wait runs out writes NaN to its outputs. */
 tr_status tr_conv3d_fwd(const void* x, const void* w, const float* bias, float* y, int32_t N, int32_t D,
                         int32_t H, int32_t W, int32_t Cin, int32_t Cout, void* stream);

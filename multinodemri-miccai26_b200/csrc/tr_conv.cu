@@ -212,7 +212,7 @@ struct Piece<float, VEC> {
 // operand reads from shared memory (128 bytes a cycle: 4 KB of voxels and 32 bytes per output
 // channel for 128 x Cout x 16 products), so by the tensor cores only from Cout = 128 on.
 // Measured at (1, 128, 256, 256), 64 -> 32 channels, float input (converted by a pass of its own
-// before): 21.5 ms with mma.sync fragments gathered from global memory, 1.38 ms with this kernel (672 TFLOP/s).
+// before): 21.5 ms with mma.sync fragments gathered from global memory, 1.34 to 1.38 ms with this kernel.
 constexpr int kFwdThreads = 512;
 constexpr int kLoaders = 256;                         // warps 8-15
 constexpr int kHaloStages = 4;

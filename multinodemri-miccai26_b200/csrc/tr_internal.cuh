@@ -229,7 +229,7 @@ struct tr_plan {
     bool two_pass_320 = true;    // 320-point TMA FFT passes in two shared-memory passes (not TR_PLAN_THREE_PASS_320)
     bool serial_bins = false;    // TR_PLAN_SERIAL_BINS: no lanes
     bool autotune = false;       // TR_PLAN_AUTOTUNE: time launch-shape candidates on first use
-    std::map<int, int> spread_cols_tuned;   // column count -> chosen spread_cols         // TMA-tiled FFT passes where the geometry allows
+    std::map<int, int> spread_cols_tuned;   // column count -> chosen spread_cols
     // TVMW
     tr::WaveletPlan* wav = nullptr;
     // CUDA graph of one PDHG iteration

@@ -1195,7 +1195,8 @@ __global__ void __launch_bounds__(256) k_interp_rows(const float2* __restrict__ 
 // row) steps through the entries that reach its row, found by a ballot over the row
 // weights.  Bound by instruction issue; with every warp stepping through every entry
 // and three barriers per 32 the gridding of 96 columns (128 x 256 x 256 image) took
-// 3.81 ms and of 72 columns (112 x 160 x 160) 1.33 ms, now 3.22 and 0.96 ms.  The launch runs work items first: a tile's list range
+// 3.81 ms and of 72 columns (112 x 160 x 160) 1.33 ms, now 3.22 and 0.96 ms.
+// The launch runs work items first: a tile's list range
 // (lists longer than kSplitEntries are cut into ranges whose partial tiles go
 // to a scratch buffer, the first range writing the grid), heaviest first; the
 // trailing CTAs write zeros into tiles no sample reaches, kZeroTiles each.
@@ -1504,16 +1505,15 @@ __global__ void __launch_bounds__(32 * kFewWarps) k_spread_few(SpreadArgs a, con
         const int z1 = min((int)zhi * kFewZero, a.n_empty);
         for (int zi = (int)zlo * kFewZero; zi < z1; ++zi) {
             tile_geometry(a, a.tile_order[a.n_busy + zi], t0z, t0y, t0x, Tz, Ty, Tx);
-            // consecutive lanes along a row's values, two at a time where rows start on 16 bytes (with a lane's own two
-            // points a store reached 8 bytes of each sector; 500 samples, 8 columns on 160^3: 188 us, 54 now)
+            // consecutive lanes along a row's values, two at a time where rows start on 16 bytes (with a lane's own
+            // two points a store reached 8 bytes of each sector; 500 samples, 8 columns on 160^3: 188 us, 54 now)
             using Zero = std::conditional_t<NC % 2 == 0, float4, float2>;
             constexpr int per = sizeof(Zero) / sizeof(float2), row_n = 4 * NC / per;
 #pragma unroll
             for (int i = lane; i < 16 * row_n; i += 32) {
                 const int r = i / row_n, o = (i - r * row_n) * per;
-                if ((r >> 2) < Tz && (r & 3) < Ty && o < Tx * NC)
-                    *reinterpret_cast<Zero*>(a.grid + (((int64_t)(t0z + (r >> 2)) * a.os1 + (t0y + (r & 3))) * a.os2 + t0x) * NC +
-                                             o) = Zero{};
+                const int64_t row0 = ((int64_t)(t0z + (r >> 2)) * a.os1 + (t0y + (r & 3))) * a.os2 + t0x;
+                if ((r >> 2) < Tz && (r & 3) < Ty && o < Tx * NC) *reinterpret_cast<Zero*>(a.grid + row0 * NC + o) = Zero{};
             }
         }
         return;
@@ -2129,11 +2129,13 @@ static tr_status stage_interp(tr_plan* p, int bin, int ncol, int mode, float sig
     if (ncol > 256) return fail(TR_ERR_UNSUPPORTED, "more than 256 k-space columns per bin are not supported");
     // Even column counts read pairs (bufA is aligned and a row of ncol even columns starts on 16 bytes).
     // While the lanes of one piece each are at most a wave of the chip's threads, one piece a lane is faster
-    // (us at 1 / 2 / 3 pieces a lane, cones, 20 000 samples on 40 x 64 x 72: 12 columns 23 / 31 / 60, 32 columns 38 / 44 / 67); beyond
-    // it fewer lanes a sample, so that a warp holds several samples and a lane several loads in flight (130 000
-    // samples on 84 x 100 x 112, 1 / 2 / 3 / 4: 8 columns 80 / 69 / 81 / 134, 10: 101 / 78 / 95 / 137, 24: 220 / 137 / 142 / 223, 48: 406 / 243 / 254 / 387); fewer than four pairs
-    // stay apart.  Odd counts, single values, turn at four waves and 15 pieces (15 columns, 130 000 samples 133 / 130 / 115 / 127,
-    // 50 000 58 / 85 / 69 / 84; 9 columns, 130 000 83 / 100 / 80 / 96), above 32 columns at once (45 columns, 6 000 samples on 40 x 64 x 72, 2 / 3 / 4: 60 / 49 / 62).
+    // (us at 1 / 2 / 3 pieces a lane, cones, 20 000 samples on 40 x 64 x 72: 12 columns 23 / 31 / 60, 32 columns
+    // 38 / 44 / 67); beyond it fewer lanes a sample, so that a warp holds several samples and a lane several
+    // loads in flight (130 000 samples on 84 x 100 x 112, 1 / 2 / 3 / 4: 8 columns 80 / 69 / 81 / 134, 10:
+    // 101 / 78 / 95 / 137, 24: 220 / 137 / 142 / 223, 48: 406 / 243 / 254 / 387); fewer than four pairs stay apart.
+    // Odd counts, single values, turn at four waves and 15 pieces (15 columns, 130 000 samples 133 / 130 / 115 / 127,
+    // 50 000 58 / 85 / 69 / 84; 9 columns, 130 000 83 / 100 / 80 / 96), above 32 columns at once (45 columns,
+    // 6 000 samples on 40 x 64 x 72, 2 / 3 / 4: 60 / 49 / 62).
     const int V = ncol % 2 == 0 ? 2 : 1, pieces = ncol / V;
     const int64_t lanes = b.count * pieces, wave = (int64_t)p->sms * 2048;
     const int more = V == 2 ? (pieces >= 4 && lanes > wave ? 2 : 1)

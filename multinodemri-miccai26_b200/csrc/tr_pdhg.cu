@@ -429,8 +429,8 @@ void lanes_destroy(tr_plan* p) {
     p->lanes = nullptr;
 }
 
-// The plan's lanes for ncol columns, or null where the bins run one after another: TR_PLAN_SERIAL_BINS, one bin, a large
-// one, no memory for more workspaces, or lanes not made yet while the caller's stream is being captured.
+// The plan's lanes for ncol columns, or null where the bins run one after another: TR_PLAN_SERIAL_BINS, one
+// bin, a large one, no memory for more workspaces, or lanes not made yet while the caller's stream is being captured.
 static BinLanes* bin_lanes(tr_plan* p, int ncol, cudaStream_t st) {
     const size_t gA = (size_t)p->os[0] * p->os[1] * p->os[2] * ncol * sizeof(float2);
     const size_t gB = (size_t)p->n[0] * p->os[1] * p->os[2] * ncol * sizeof(float2);

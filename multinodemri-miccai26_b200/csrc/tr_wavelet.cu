@@ -185,8 +185,8 @@ __device__ __forceinline__ void cv_fma(CVec<V>& acc, float f, const CVec<V>& x) 
 
 // ------------------------------------------------------------------ analysis
 // Outputs per thread along z: 34 loads for 12 instead of the 24 of a whole line; 4 (18 loads) while runs of 12
-// are less than a wave of blocks.  One image of 48 x 64 x 64, analysis of two levels: 43 us with runs of 12, 36 with 4 (37 with one output a
-// thread before).
+// are fewer than two blocks a multiprocessor.  One image of 48 x 64 x 64, analysis of two levels: 43 us with
+// runs of 12, 36 with 4 (37 with one output a thread before).
 constexpr int kDwtRun = 12, kDwtRunShort = 4;
 constexpr int kDwtRows = 16;     // output rows (of each half) per CTA of the y + x kernel
 

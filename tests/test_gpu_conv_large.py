@@ -39,6 +39,8 @@ def test_forward_of_a_large_slice(dtype):
     # 54 products of multiples of 2^-12 below 4: exact sums
     assert np.array_equal(y[:, :, -13:, -21:].cpu().numpy(), ref.astype(np.float32))
     assert int(torch.count_nonzero(y)) == int(np.count_nonzero(ref))
+    del x, y
+    torch.cuda.empty_cache()
 
 
 def test_weight_gradient_of_a_large_slice():
@@ -53,3 +55,5 @@ def test_weight_gradient_of_a_large_slice():
     gy[:, :, -12:, -20:] = torch.from_numpy(gt).cuda().bfloat16()
     dw = ws.conv3d_wgrad_bf16(x, gy).cpu().numpy()
     assert np.array_equal(dw, oconv.conv3d_wgrad(xt, gt).astype(np.float32))
+    del x, gy
+    torch.cuda.empty_cache()

@@ -96,6 +96,7 @@ struct AdjXArgs {
     int ncol;
     const float2* maps;     // (Z, Y, X, C) or null
     int C, cc, rows;
+    int cta_rows, tiles;    // k_lp_adj_x_one: image rows and 16-column tiles per CTA
     int n_img;
     int Z, Y, X, OSX, h, pad;
     const float* apz;
@@ -116,6 +117,7 @@ struct LineKernels {
     const void* inv = nullptr;
     const void* fwd_x = nullptr;     // (FwdXArgs)
     const void* adj_x = nullptr;     // (AdjXArgs)
+    const void* adj_x_one = nullptr; // the same for one image; null where adj_x is the faster one
     int threads = 0;
     int smem = 0;                    // dynamic shared memory, bytes
 };

@@ -301,6 +301,57 @@ __global__ void __launch_bounds__(lp_threads(L), lp_x_min_ctas(L)) k_lp_adj_x(Ad
     }
 }
 
+// Adjoint of one image at long lengths, where a map held in registers spills (336 to 448 bytes a thread at 240 and
+// 320): the map is read where it is used, and a CTA takes a.cta_rows rows in a.tiles tiles of 16 columns, so that
+// the coils of several rows fill whole tiles; a row whose coils began in an earlier tile is added to.
+// 64 x 192 x 192: 5 coils 171 -> 124 us, 6 coils 214 -> 152, 10 coils 375 -> 230; 32 x 256 x 256: 6 coils 230 -> 153,
+// 10 coils 407 -> 236.  At 125 and 200 points the kernel above is a quarter faster.
+constexpr int kOneImageLen = 240;
+template <int L>
+__global__ void __launch_bounds__(lp_threads(L), lp_x_min_ctas(L)) k_lp_adj_x_one(AdjXArgs a) {
+    extern __shared__ float2 sm[];
+    constexpr int NT = lp_threads(L), kPitch = kLineW + 1;
+    float2* tw = sm + L * kLineW;
+    for (int i = threadIdx.x; i < L; i += NT) tw[i] = a.tw[i];
+    const int w = threadIdx.x & (kLineW - 1);
+    const int64_t rows = (int64_t)a.Z * a.Y, row0 = (int64_t)blockIdx.x * a.cta_rows;
+    const LineRow<L> to(a.h, a.pad);
+    for (int t0 = 0; t0 < a.tiles * kLineW; t0 += kLineW) {
+        const int rl = (t0 + w) / a.C, c = t0 + w - rl * a.C;
+        const int64_t row = row0 + rl;
+        const bool on = rl < a.cta_rows && row < rows;
+        const float2* in = a.in + (on ? row * a.OSX * a.ncol + c : 0);
+        LpFirst<L> v;
+        lp_load<L>(v, [&](int m, int) -> float2 {
+            int j = m + a.h;
+            if (j >= L) j -= L;
+            return on ? in[j * a.ncol] : make_float2(0.f, 0.f);
+        });
+        const int z = on ? (int)(row / a.Y) : 0, y = on ? (int)(row - (int64_t)z * a.Y) : 0;
+        const float sc = a.apz[z] * a.apy[y] * a.scale;
+        const float2* mp = a.maps ? a.maps + (on ? row * a.X * a.C + c : 0) : nullptr;
+        lp_pass<L, true, 0, 1, true>(v, sm, tw, [&](int k, float2 r, int) {
+            const int x = to(k);
+            if ((unsigned)x >= (unsigned)a.X) return;
+            const float2 m = mp ? (on ? mp[x * a.C] : make_float2(0.f, 0.f)) : make_float2(on ? sc * a.apx[x] : 0.f, 0.f);
+            sm[x * kPitch + w] = cmulc(r, m);
+        });
+        __syncthreads();
+        const int r0 = t0 / a.C, n = min(a.cta_rows, (t0 + kLineW - 1) / a.C + 1) - r0;      // rows in this tile
+        for (int i = threadIdx.x; i < n * a.X; i += NT) {
+            const int r = r0 + (n == 1 ? 0 : i / a.X), x = i - (r - r0) * a.X;
+            if (row0 + r >= rows) break;
+            const int k0 = max(r * a.C - t0, 0), k1 = min((r + 1) * a.C - t0, kLineW);
+            const float2* p = sm + x * kPitch;
+            float2 t = p[k0];
+            for (int k = k0 + 1; k < k1; ++k) t = cadd(t, p[k]);
+            float2* dst = a.img + (row0 + r) * a.X + x;
+            *dst = r * a.C < t0 ? cadd(*dst, t) : t;
+        }
+        __syncthreads();
+    }
+}
+
 // ------------------------------------------------------------------ table
 template <int L>
 LineKernels lp_entry() {
@@ -310,6 +361,7 @@ LineKernels lp_entry() {
         k.inv = (const void*)k_lp_line<L, true>;
         k.fwd_x = (const void*)k_lp_fwd_x<L>;
         k.adj_x = (const void*)k_lp_adj_x<L>;
+        if constexpr (L >= kOneImageLen) k.adj_x_one = (const void*)k_lp_adj_x_one<L>;
         k.threads = lp_threads(L);
         k.smem = lp_smem(L);
     }

@@ -2349,11 +2349,23 @@ static tr_status stage_adj_x(tr_plan* p, int n_img, const float2* maps, int C, f
     }
     const LineKernels& lk = line_kernels(OSX);
     if (lk.adj_x) {
-        const int64_t rows = (int64_t)Z * Y, per = C >= kLineW ? 1 : kLineW / C;
-        TR_TRY(raise_smem_limit(lk.adj_x, lk.smem));
+        const int64_t rows = (int64_t)Z * Y;
+        aa.cta_rows = C >= kLineW ? 1 : kLineW / C;
+        aa.tiles = (C + kLineW - 1) / kLineW;
+        const bool one = n_img == 1 && lk.adj_x_one;
+        // a fifth or more of the columns idle: as many rows as fill whole tiles, while that leaves four CTAs a
+        // multiprocessor (64 x 192 x 192, one tile / filled: 6 coils 160 / 147 us, 9 coils 269 / 210, 11 273 / 251;
+        // with fewer CTAs it is the slower one: 3072 rows of 64, 9 coils 21 / 33)
+        const int fill = kLineW / std::gcd(C, kLineW);
+        if (one && aa.cta_rows * C * 5 <= kLineW * 4 && rows >= (int64_t)fill * p->sms * 4) {
+            aa.cta_rows = fill;
+            aa.tiles = fill * C / kLineW;
+        }
+        const void* afn = one ? lk.adj_x_one : lk.adj_x;
+        TR_TRY(raise_smem_limit(afn, lk.smem));
         void* args[] = {&aa};
-        TR_CUDA(cudaLaunchKernel(lk.adj_x, dim3((unsigned)((rows + per - 1) / per)), dim3((unsigned)lk.threads), args,
-                                 lk.smem, st));
+        TR_CUDA(cudaLaunchKernel(afn, dim3((unsigned)((rows + aa.cta_rows - 1) / aa.cta_rows)),
+                                 dim3((unsigned)lk.threads), args, lk.smem, st));
         return TR_OK;
     }
     aa.cc = coils_per_cta(C);

@@ -116,6 +116,7 @@ struct LineKernels {
     const void* fwd = nullptr;       // line pass, (LineArgs)
     const void* inv = nullptr;
     const void* fwd_x = nullptr;     // (FwdXArgs)
+    const void* fwd_x_images = nullptr;   // several images of one coil with maps; null where fwd_x is used
     const void* adj_x = nullptr;     // (AdjXArgs)
     const void* adj_x_one = nullptr; // the same for one image; null where adj_x is the faster one
     int threads = 0;

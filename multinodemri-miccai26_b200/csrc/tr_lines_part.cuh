@@ -234,6 +234,48 @@ __global__ void __launch_bounds__(lp_threads(L), lp_x_min_ctas(L)) k_lp_fwd_x(Fw
     }
 }
 
+// Forward, several images of one coil at long lengths: 16 consecutive (row, image) columns, so that a row's images are
+// stored beside one another, each column's image row in shared memory.  (The kernel above stores 8 bytes a row apart, and
+// its two buffers of 16 rows leave two CTAs a multiprocessor; one coil, 6 images: 64 x 192 x 192 217 us, 105 now,
+// 32 x 256 x 256 199 us, 112 now.)
+constexpr int kLongLen = 240;
+template <int L>
+__global__ void __launch_bounds__(lp_threads(L), lp_x_min_ctas(L)) k_lp_fwd_x_images(FwdXArgs a) {
+    extern __shared__ float2 sm[];
+    constexpr int NT = lp_threads(L);
+    float2* tw = sm + L * kLineW;
+    float2* rowbuf = tw + L;                              // [16][pitch]
+    const int pitch = lp_row_pitch(a.X);
+    for (int i = threadIdx.x; i < L; i += NT) tw[i] = a.tw[i];
+    const int64_t q0 = (int64_t)blockIdx.x * kLineW, total = (int64_t)a.Z * a.Y * a.n_img;
+    for (int r = threadIdx.x >> 5; r < kLineW; r += NT / 32) {
+        if (q0 + r >= total) break;
+        const int64_t row = (q0 + r) / a.n_img;
+        const float2* src = a.img + (q0 + r - row * a.n_img) * a.img_stride + row * a.X;
+        for (int x = threadIdx.x & 31; x < a.X; x += 32) cp_async8(rowbuf + r * pitch + x, src + x, 8);
+    }
+    const int w = threadIdx.x & (kLineW - 1);
+    const bool on = q0 + w < total;
+    const int64_t row = on ? (q0 + w) / a.n_img : 0;
+    const int e = on ? (int)(q0 + w - row * a.n_img) : 0;
+    const LineRow<L> from(a.h, a.pad);
+    const float2* mp = a.maps + row * a.X;
+    cp_async_wait_all();
+    __syncthreads();
+    const float2* u = rowbuf + w * pitch;
+    LpFirst<L> v;
+    lp_load<L>(v, [&](int m, int) -> float2 {
+        const int x = from(m);
+        return (unsigned)x < (unsigned)a.X ? cmul(u[x], mp[x]) : make_float2(0.f, 0.f);
+    });
+    float2* out = a.out + row * a.OSX * a.ncol + e;
+    lp_pass<L, false, 0, 1, false>(v, sm, tw, [&](int k, float2 r, int) {
+        int g = k + a.h;
+        if (g >= L) g -= L;
+        if (on) out[g * a.ncol] = r;
+    });
+}
+
 // Adjoint: whole rows of at most 16 coils (several rows where they fit), or 16 coils of a row at a
 // time; the products go back into the tile with 17 columns, where the threads along x sum a row's coils
 // in order and write the image row (coils past the first 16 are added to it).  The next image's inputs
@@ -306,7 +348,6 @@ __global__ void __launch_bounds__(lp_threads(L), lp_x_min_ctas(L)) k_lp_adj_x(Ad
 // the coils of several rows fill whole tiles; a row whose coils began in an earlier tile is added to.
 // 64 x 192 x 192: 5 coils 171 -> 124 us, 6 coils 214 -> 152, 10 coils 375 -> 230; 32 x 256 x 256: 6 coils 230 -> 153,
 // 10 coils 407 -> 236.  At 125 and 200 points the kernel above is a quarter faster.
-constexpr int kOneImageLen = 240;
 template <int L>
 __global__ void __launch_bounds__(lp_threads(L), lp_x_min_ctas(L)) k_lp_adj_x_one(AdjXArgs a) {
     extern __shared__ float2 sm[];
@@ -361,7 +402,10 @@ LineKernels lp_entry() {
         k.inv = (const void*)k_lp_line<L, true>;
         k.fwd_x = (const void*)k_lp_fwd_x<L>;
         k.adj_x = (const void*)k_lp_adj_x<L>;
-        if constexpr (L >= kOneImageLen) k.adj_x_one = (const void*)k_lp_adj_x_one<L>;
+        if constexpr (L >= kLongLen) {
+            k.fwd_x_images = (const void*)k_lp_fwd_x_images<L>;
+            k.adj_x_one = (const void*)k_lp_adj_x_one<L>;
+        }
         k.threads = lp_threads(L);
         k.smem = lp_smem(L);
     }

@@ -1968,11 +1968,13 @@ static tr_status stage_fwd_x(tr_plan* p, const float2* images, int64_t img_strid
     }
     const LineKernels& lk = line_kernels(OSX);
     if (lk.fwd_x) {
-        const int64_t q = (int64_t)Z * Y * C;
-        const size_t smem = lk.smem + lp_row_bytes(X, C, n_img);
-        TR_TRY(raise_smem_limit(lk.fwd_x, smem));
+        const bool images = C == 1 && n_img > 1 && maps && lk.fwd_x_images;
+        const void* xfn = images ? lk.fwd_x_images : lk.fwd_x;
+        const int64_t q = (int64_t)Z * Y * (images ? n_img : C);
+        const size_t smem = lk.smem + lp_row_bytes(X, C, images ? 1 : n_img);
+        TR_TRY(raise_smem_limit(xfn, smem));
         void* args[] = {&fa};
-        TR_CUDA(cudaLaunchKernel(lk.fwd_x, dim3((unsigned)((q + kLineW - 1) / kLineW)), dim3((unsigned)lk.threads), args, smem,
+        TR_CUDA(cudaLaunchKernel(xfn, dim3((unsigned)((q + kLineW - 1) / kLineW)), dim3((unsigned)lk.threads), args, smem,
                                  st));
         return TR_OK;
     }
